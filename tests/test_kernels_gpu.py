@@ -51,6 +51,24 @@ def test_gemm_simt_rows_do_not_depend_on_the_batch():
     assert torch.equal(full[33:34], one)                 # bit for bit
 
 
+# the 16 x 32, 64 x 32, 64 x 64 and 128 x 64 tiles, whole and with remainders in every direction
+@pytest.mark.parametrize("M,N,K", [(16, 70, 100), (17, 70, 100), (64, 96, 33), (130, 9000, 35), (300, 5000, 66), (700, 9001, 70)])
+@pytest.mark.parametrize("pitch", [0, 1])
+def test_gemm_simt_tiles_add_in_one_order(M, N, K, pitch):
+    """Every tile gives a row what the one-token product gives it, bit for bit, and stays within the bound of a chain of K
+    32-bit FMAs; a row pitch of no multiple of four elements takes the scalar loads."""
+    g = torch.Generator(device="cpu").manual_seed(M + N)
+    a = torch.randn(M, K + pitch, generator=g).to(DEV)[:, :K]
+    w = torch.randn(N, K + pitch, generator=g).bfloat16().to(DEV)[:, :K]
+    out, one = torch.empty(M, N, device=DEV), torch.empty(1, N, device=DEV)
+    ops().gemm_simt(a, w, out)
+    for m in sorted({0, 15, M // 2, M - 1}):
+        ops().gemm_simt(a[m:m + 1], w, one)
+        assert torch.equal(one[0], out[m]), m
+    want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    assert bool(((out.double() - want).abs() <= K * 2.0 ** -24 * size).all())
+
+
 TC_SHAPES = [(1, 128, 64), (3, 96, 320), (8, 256, 2112), (40, 4096, 4096), (128, 4096, 4096), (96, 12288, 4096), (72, 1000, 328), (130, 4096, 16384), (100, 520, 8200),
              (250, 12288, 4096), (16, 4096, 1024), (17, 1000, 96), (33, 200, 136), (64, 512, 4096),
              (65, 384, 256), (128, 128, 64), (200, 1000, 328), (300, 520, 1032), (2048, 768, 512),
@@ -424,6 +442,26 @@ def test_attention_simt(n_heads, n_kv, d, dtype, window):
     out = torch.zeros(case.N, n_heads * d, dtype=dtype, device=DEV)
     ops().attention_simt(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, n_heads, scale, window or 0)
     assert rel_err(out, case.want(scale, window)) <= (1e-5 if dtype == torch.float32 else 1e-2)
+
+
+@pytest.mark.parametrize("n_heads,n_kv,d", [(32, 32, 20), (20, 5, 64), (17, 17, 100), (16, 2, 128), (16, 16, 144)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("options", [{}, {"sink": 0.5, "bias": True}, {"window": 37, "keep_first": 5}])
+def test_attention_simt_portions_and_rows_agree(n_heads, n_kv, d, dtype, options):
+    """Portions in tiles (edges inside a tile, several requests in one, rows alone beside them), row by row, and with one
+    warp a row (a head size without the staged kernels): the same bits where two of them take a call, and the plain result."""
+    case = PagedCase([(0, 33), (17, 1), (40, 2), (100, 64), (3, 1), (130, 1), (0, 1), (61, 5)], n_heads, n_kv, d, dtype, seed=d)
+    kw = dict(options)
+    if kw.pop("bias", False):
+        g = torch.Generator().manual_seed(1)
+        kw["bias"] = (torch.rand(n_heads, generator=g).to(DEV), torch.rand(n_heads, generator=g).to(DEV))
+    scale = 1.0 / math.sqrt(d)
+    outs = [torch.zeros(case.N, n_heads * d, dtype=dtype, device=DEV) for _ in range(2)]
+    for out, portions in zip(outs, (True, False)):
+        ops().attention_simt(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, n_heads, scale, portions=portions, **kw)
+    assert torch.equal(outs[0], outs[1])
+    if not options:
+        assert rel_err(outs[0], case.want(scale, None)) <= (1e-5 if dtype == torch.float32 else 1e-2)
 
 
 @pytest.mark.parametrize("n_heads,n_kv,d", ATT_SHAPES)

@@ -293,8 +293,9 @@ def _score_options(keep_first, bias, sink, n_heads, window):
 
 
 def attention_simt(q, cache, block_tables, token_request, positions, out, n_heads, scale, window=0, chunk=0, keep_first=0,
-                   bias=None, sink=None):
-    """q: [N, n_heads * head_dim] view; out likewise; cache as in kv_append."""
+                   bias=None, sink=None, portions=True):
+    """q: [N, n_heads * head_dim] view; out likewise; cache as in kv_append.  portions: False says that every request has
+    one row, which saves the kernel that takes a portion's rows together (results are the same bit for bit)."""
     lib = _lib("attention_simt", cache, q, out)
     _need(cache, "cache", _FLOATS, 5)
     N, width, q_stride = _rows_2d(q, "q")
@@ -309,7 +310,7 @@ def attention_simt(q, cache, block_tables, token_request, positions, out, n_head
                                   _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(N),
                                   c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask_rule(window, chunk)),
                                   c_float(scale), *_score_options(keep_first, bias, sink, n_heads, window),
-                                  c_int(_is_h16(cache)), _stream()), "attention_simt")
+                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), _stream()), "attention_simt")
 
 
 def sample(logits, out, temperature=None, top_k=None, top_p=None, seeds=None, counters=None, suppress_id=-1,
@@ -818,7 +819,7 @@ def attention(ctx, group, q, cache, out, n_heads, scale, window=0, new_kv=None, 
     if new_kv is not None:
         kv_append(new_kv[0], new_kv[1], new_kv[2], cache, ctx.page_size)
     attention_simt(q, cache, ctx.block_tables[group], ctx.token_request, ctx.positions, out, n_heads, scale,
-                   window, chunk, keep_first, bias, sink)
+                   window, chunk, keep_first, bias, sink, portions=not ctx.decode_only)
 
 
 # ---------------------------------------------------------------------------------------------
