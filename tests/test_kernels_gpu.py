@@ -546,6 +546,41 @@ def test_attention_decode_with_a_key_value_heads_query_heads_in_one_block(n_head
         assert torch.equal(case.cache[written], full[written])
 
 
+@pytest.mark.parametrize("n_heads,n_kv,d", [(3, 1, 64), (8, 1, 80), (9, 1, 96), (16, 1, 112), (17, 1, 128), (40, 2, 128), (3, 3, 128), (5, 5, 80)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("window", [None, 50])
+@pytest.mark.parametrize("n_splits,warps", [(1, 4), (1, 8), (3, 4), (8, 8), (None, None)])
+def test_attention_decode_grouped_keeps_the_probabilities(n_heads, n_kv, d, dtype, window, n_splits, warps):
+    """Head tiles of 8 and 16 whole and with remainders, every head size, one to eight splits (more than there are pages of
+    some rows), a token at the start and the end of a page.  The result is the 64-bit one rounded once: the probabilities
+    are held to 2^-20 and the sums to 32 bits, which 2^-12 of the largest value covers."""
+    lens = [(0, 1), (15, 1), (16, 1), (255, 1), (700, 1), (63, 1)]
+    case = PagedCase(lens, n_heads, n_kv, d, dtype, seed=d + n_heads, plant=False)
+    scale = 0.8 / math.sqrt(d)
+    out = torch.zeros(case.N, n_heads * d, dtype=dtype, device=DEV)
+    ops().attention_decode(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, n_heads, scale, window or 0,
+                           max_kv_len=701, n_splits=n_splits, warps=warps, grouped=True)
+    rep, outs = n_heads // n_kv, []
+    for (c, _), q, k, v in zip(lens, case.q, case.k, case.v):
+        lo = max(0, c + 1 - window) if window else 0
+        k, v = (x[lo:].double().transpose(0, 1).repeat_interleave(rep, dim=0) for x in (k, v))
+        p = torch.softmax((k @ q[0].double()[:, :, None])[..., 0] * scale, -1)
+        outs.append((p[:, None] @ v).reshape(-1))
+    want = torch.stack(outs).to(DEV)
+    step = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)                 # half a unit in the last place, relative
+    assert bool(((out.double() - want).abs() <= step * want.abs() + 2.0 ** -12 * step * want.abs().max() + 2.0 ** -24).all())
+
+
+def test_attention_decode_grouped_keeps_an_infinite_value():
+    """An infinite value makes its dim infinite, not undefined, whatever its key's probability is split into."""
+    case = PagedCase([(40, 1), (3, 1)], 8, 2, 128, torch.float16, seed=4, plant=False)
+    case.cache[case.bt[0, 1].long(), 1, 1, 3, 5] = float("inf")            # position 19 of the first request, head group 1
+    out = torch.zeros(2, 8 * 128, dtype=torch.float16, device=DEV)
+    ops().attention_decode(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, 8, 0.09, max_kv_len=41, grouped=True)
+    o = out.view(2, 8, 128)
+    assert bool((o[0, 4:, 5] == float("inf")).all()) and int(torch.isfinite(o).logical_not().sum()) == 4
+
+
 def test_attention_decode_row_list():
     """Only the rows named are computed (a mixed batch: the others belong to the prefill kernel)."""
     lens = [(5, 1), (0, 40), (99, 1), (10, 3), (33, 1)]

@@ -41,6 +41,7 @@ SOURCES: Dict[str, str] = {
     "gemm_tc": "gemm_tc.cu",
     "gemv": "gemv.cu",
     "attention_decode": "attention_decode.cu",
+    "attention_decode_grouped": "attention_decode_grouped.cu",
     "attention_prefill": "attention_prefill.cu",
     "attention_prefill_tc": "attention_prefill_tc.cu",
     "rmsnorm": "rmsnorm.cu",

@@ -638,15 +638,63 @@ def decode_attention_plan(pairs: int, sms: int, head_dim: int, max_pages: int):
     return (4, 1) if t4 < t8 else (8, 1)
 
 
+def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms: int, max_pages: int) -> bool:
+    """Whether decode attention runs the tensor-core kernel (csrc/attention_decode_grouped.cu) where that takes the sizes.
+
+    With shared key/value heads always, but for the shortest steps (16 heads on one, 100 tokens: 4.6 us with a block a head,
+    6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1).  Without, where the other kernel's lanes idle (head sizes that
+    are no power of two: 80 dims, 8 rows of 32 heads over up to 1,400 tokens 34 and 26 us, 64 rows 164 and 135), with
+    few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 13.8 and 10.7 us; 8 rows 35 and 31) and with
+    many long ones (64 rows 172 and 166); between those a block a head is as fast or faster (16 rows 53 and 56 us; heads of
+    64, 8 rows over 1,000 tokens 16 and 21)."""
+    blocks = rows * n_heads
+    if max_pages <= 12 and blocks <= sms:
+        return False
+    if n_heads != n_kv:
+        return True
+    if head_dim == 64:
+        return False
+    if max_pages < 32:
+        return max_pages > 12 and 2 * blocks <= sms
+    return head_dim != 128 or blocks <= 2 * sms or blocks > 4 * sms
+
+
+def grouped_decode_plan(blocks: int, sms: int, heads_per_block: int, max_pages: int):
+    """(warps a block, splits of the context) for `blocks` (row, head tile) blocks of the grouped decode attention.
+
+    An SM holds twelve of its warps with up to eight query heads a block (one block of twelve or three of four), eight with
+    sixteen.  Splits are a cluster's blocks, and clusters leave places empty: those of up to four blocks fill nine places in
+    ten, wider ones seven (16 blocks in eight splits each, 128 places of 148, ran in two rounds: 21 against 14 us with six)."""
+    big = 12 if heads_per_block == 8 else 8
+    if blocks > sms:
+        # More blocks than SMs: short contexts in blocks of four warps (512 blocks of 8 pages: 15 us, of twelve warps 22),
+        # and so many blocks that ragged contexts leave the big ones' last rounds uneven (1,024 of up to 88 pages: 70
+        # against 80 us, equal ones of 128 pages 187 against 177).  Else whichever leaves the fewer places of its
+        # last round empty (256 blocks of 128 pages: 53 us with twelve warps, 57 with four; 512: 102 and 121, 384 ragged
+        # ones 62 and 58).
+        if max_pages < 2 * big or blocks > 4 * sms:
+            return 4, 1
+        fill = lambda per: blocks / (-(-blocks // (per * sms)) * per * sms)
+        return (4, 1) if fill(big // 4) >= fill(1) else (big, 1)
+    # Fewer: big blocks, split while the SMs last; few pages (under four a warp of a big block) in splits of four warps
+    # (one row of 32 heads on 8 over 400 tokens: 5.4 us in eight splits of four warps, 6.4 of twelve).
+    short = max_pages < 4 * big
+    warps, places = (4, sms * big // 4) if short else (big, sms)
+    most = max(1, max_pages // (3 if short else 8))
+    splits = min(most, (9 * places) // (10 * blocks))
+    if splits > 4:
+        splits = min(most, 8, max(4, (7 * places) // (10 * blocks)))
+    return warps, max(1, splits)
+
+
 def attention_decode(q, cache, block_tables, token_request, positions, out, n_heads, scale, window=0, rows=None,
                      n_rows=None, max_kv_len=None, n_splits=None, new_kv=None, warps=None, grouped=None, chunk=0, keep_first=0, bias=None, sink=None):
     """One query token per row over the paged 16-bit cache.  `rows` (int32) names the rows of q
     that are decode tokens (None: all); max_kv_len bounds their contexts (for the split plan).
     new_kv = (k, v), [rows of q, kv_heads * head_dim] bfloat16: the keys and values of the rows' own
     tokens, which the kernel then writes into their pages itself (no kv_append before it).
-    n_splits (with warps, 4 or 8 a block) forces a plan: a test hook.  grouped: with 2 or 4 query heads a key/value
-    head a block can take all query heads of a key/value head and read the head's pages once (None: where that pays;
-    True / False: a test hook)."""
+    n_splits (with warps, 4 or 8 a block) forces a plan: a test hook.  grouped: with several query heads a key/value
+    head a block takes up to 16 of them and reads the head's pages once (True / False: a test hook)."""
     lib = _lib("attention_decode", cache, q, out)
     _need(cache, "cache", _H16, 5)
     N, width, q_stride = _rows_2d(q, "q")
@@ -664,43 +712,31 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
     max_pages = max(1, -(-(int(max_kv_len) if max_kv_len is not None else block_tables.shape[1] * ps) // ps))
     if window or chunk:                                    # the kernel walks the pages that hold visible keys only
         max_pages = min(max_pages, (int(window or chunk) - 1) // ps + 2 + -(-int(keep_first or 0) // ps))
-    forced_warps, warps = warps, 4
-    # with grouped key/value heads (2 or 4 query heads each) a block takes all query heads of a key/value head
-    # Measured (32 query heads of 128 on 8 key/value heads, contexts of 2,048): the grouped form wins from 64 rows on
-    # (a layer's step 1.58 against 1.77 ms at 64 rows, 2.44 against 2.78 at 128) and loses below (1.34 against 1.18 at 32:
-    # its blocks are a quarter as many, one an SM), so it runs once the (row, key/value head) pairs are three an SM.
-    heads_per_block = lib.tnx_attention_decode_heads_per_block(c_int(n_heads), c_int(n_kv), c_int(d))
-    # Measured again with 8 query heads a key/value head (the two maps of differential attention; 64 heads on 8, contexts
-    # of 2,048): between two thirds of a block and three blocks an SM the grouped form wins as well when its blocks are
-    # four warps and the context is split so that about two blocks an SM run (8 rows: 75 us with two splits against 93
-    # with a block a head; 16 rows: 123 against 153; the plan drawn for one head a block gave 107 and 206 there).
-    few_grouped = False
-    if heads_per_block > 1 and grouped is None:
-        blocks = R * n_heads // heads_per_block
-        if blocks < 3 * st["sms"]:
-            few_grouped = 3 * blocks >= 2 * st["sms"] and n_splits is None
-            if not few_grouped:
-                heads_per_block = 1
-    elif grouped is False:
-        heads_per_block = 1
-    if few_grouped:
-        warps = 4
-        n_splits = max(1, min(max_pages // 8, (2 * st["sms"] + blocks // 2) // blocks))
+    # The kernel that takes up to 8 or 16 query heads of a key/value head a block and reads a page once for all of them;
+    # a forced plan is the other kernel's unless `grouped` asks for this one.
+    heads_per_block = 0
+    if grouped or (grouped is None and n_splits is None and grouped_decode_takes(R, n_heads, n_kv, d, st["sms"], max_pages)):
+        group_lib = _lib("attention_decode_grouped", cache, q, out)
+        heads_per_block = group_lib.tnx_attention_decode_grouped_heads(c_int(n_heads), c_int(n_kv), c_int(d))
+    if heads_per_block:
+        tiles = n_kv * -(-(n_heads // n_kv) // heads_per_block)
+        if n_splits is None:
+            warps, n_splits = grouped_decode_plan(R * tiles, st["sms"], heads_per_block, max_pages)
+        most_warps = 12 if heads_per_block == 8 else 8     # a forced plan's warps: 4, or all that an SM holds
+        warps = 4 if warps in (None, 4) else most_warps
+        n_splits = max(1, min(int(n_splits), max_pages, 8))
         pps = -(-max_pages // n_splits)
-        pps = -(-pps // warps) * warps
     elif n_splits is None:
-        warps, n_splits = decode_attention_plan(R * n_heads // heads_per_block, st["sms"], d, max_pages)
-        if heads_per_block > 1 and warps == 16:
-            warps = 8                                           # their accumulators leave no registers for sixteen warps
+        warps, n_splits = decode_attention_plan(R * n_heads, st["sms"], d, max_pages)
         pps = -(-max_pages // n_splits)
         pps = -(-pps // warps) * warps
     else:                                                  # a test's own plan (warps: 4, 8 or 16 a block)
-        warps = int(forced_warps or 4)
+        warps = int(warps or 4)
         n_splits = max(1, min(int(n_splits), max_pages))
         pps = -(-max_pages // n_splits)
     n_splits = -(-max_pages // pps)
     scratch = None
-    if n_splits > 1:
+    if n_splits > 1 and not heads_per_block:
         need = R * n_heads * n_splits * (d + 2)
         scratch = _grow(st, "att_scratch", need, torch.float32, q.device, 1 << 20)
         _grow(st, "att_counters", R * n_heads, torch.int32, q.device, 8192, zero=True)
@@ -715,12 +751,20 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
         kv_stride = k_new.stride(0)
         if v_new.stride(0) != kv_stride:
             raise KernelError("new k and v must have the same row pitch")
+    if heads_per_block:
+        _check(group_lib.tnx_attention_decode_grouped(
+            _p(q), c_int(q_stride), _p(cache), _p(block_tables), c_int(block_tables.stride(0)),
+            _p(rows), _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(R),
+            c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask_rule(window, chunk)), c_float(scale),
+            c_int(n_splits), c_int(pps), _p(k_new), _p(v_new), c_int(kv_stride), c_int(warps),
+            *_score_options(keep_first, bias, sink, n_heads, window), _stream()), "attention_decode")
+        return
     _check(lib.tnx_attention_decode_append(
         _p(q), c_int(q_stride), _p(cache), _p(block_tables), c_int(block_tables.stride(0)),
         _p(rows), _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(R),
         c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask_rule(window, chunk)), c_float(scale),
         c_int(n_splits), c_int(pps), _p(scratch), _p(st.get("att_counters")), _p(k_new), _p(v_new), c_int(kv_stride),
-        c_int(warps), c_int(heads_per_block), *_score_options(keep_first, bias, sink, n_heads, window), _stream()), "attention_decode")
+        c_int(warps), *_score_options(keep_first, bias, sink, n_heads, window), _stream()), "attention_decode")
 
 
 ATTN_PREFILL_TILE = 128      # query rows of one work item of the prefill attention kernel

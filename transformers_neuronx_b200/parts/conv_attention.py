@@ -39,7 +39,7 @@ class ConvAttention(FusableMixer):
     @property
     def extra_libraries(self):
         prefill = "attention_prefill_tc" if self.pad_dim in (64, 80, 96, 112, 128) else "attention_prefill"
-        return ("conv_qkv", "rotary_qkv", "kv_cache", "attention_simt", prefill, "attention_decode")
+        return ("conv_qkv", "rotary_qkv", "kv_cache", "attention_simt", prefill, "attention_decode", "attention_decode_grouped")
 
     def __init__(self, spec: ConvAttentionSpec):
         s = self.spec = spec

@@ -36,7 +36,7 @@ class DiffAttention(FusableMixer):
     @property
     def extra_libraries(self):
         prefill = "attention_prefill_tc" if self.pad_dim in (64, 80, 96, 112, 128) else "attention_prefill"
-        return ("diff_attention", "kv_cache", "attention_simt", prefill, "attention_decode")
+        return ("diff_attention", "kv_cache", "attention_simt", prefill, "attention_decode", "attention_decode_grouped")
 
     def __init__(self, spec: DiffAttentionSpec):
         s = self.spec = spec

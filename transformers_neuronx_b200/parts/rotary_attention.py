@@ -44,7 +44,7 @@ class RotaryAttention(FusableMixer):
     def extra_libraries(self):
         # the prefill kernel of this head size only: tcgen05 for 64 .. 128, mma.sync for the others
         prefill = "attention_prefill_tc" if self.pad_dim in (64, 80, 96, 112, 128) else "attention_prefill"
-        return ("rotary_qkv", "kv_cache", "attention_simt", prefill, "attention_decode")
+        return ("rotary_qkv", "kv_cache", "attention_simt", prefill, "attention_decode", "attention_decode_grouped")
 
     def __init__(self, spec: RotaryAttentionSpec):
         s = self.spec = spec
