@@ -128,6 +128,45 @@ def test_retention_scan_carries_its_state_across_cuts_and_requests(H, dk, dv):
     assert float((state[1] - 7.0).abs().max()) == 0.0 and float(state[3].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("H, Hq, dk, dv", [(2, 2, 128, 128), (4, 2, 128, 64), (3, 3, 64, 64), (2, 1, 64, 128)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("gates", [False, True])
+def test_retention_in_chunks_equals_the_recurrence(H, Hq, dk, dv, dtype, gates):
+    """Chunks whole and with remainders of 1, 16, 17 and 63 tokens, several requests (one of them padding) with states of their
+    own, fixed and per-token decays (one zero, two negative, strong ones beside weak ones) and key scales.  A product keeps
+    22 bits and more (2^-22 left out, 2^-23 a cut sum), so a result of up to 128 + 64 + 64 of them stays within 2^-20 of the
+    size of its terms, which is at most 16 times the results' root mean square (256 terms of random sign)."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(H + dk)
+    lens, slots = [64, 1, 0, 145, 127, 16], [3, 0, 1, -1, 2, 5]
+    N = sum(lens)
+    q, k = torch.randn(N, Hq * dk, generator=g), torch.randn(N, Hq * dk, generator=g) * dk ** -0.5
+    v = torch.randn(N, H * dv, generator=g).to(dtype)
+    decay = torch.tensor([0.97, 0.9995, 0.9, 1.0][:H])
+    dec, ks = decay.expand(N, H).clone(), torch.ones(N, H)
+    if gates:
+        dec, ks = torch.exp(-3.0 * torch.rand(N, H, generator=g) ** 6), torch.rand(N, H, generator=g)
+        dec[3, 0], dec[230, 1], dec[231, 1] = 0.0, -0.5, -0.9
+    state0 = torch.randn(6, H, dv, dk, generator=g)
+    want, states, at = torch.zeros(N, H * dv, dtype=torch.float64), state0.double().clone(), 0
+    for n, slot in zip(lens, slots):
+        if slot >= 0:
+            S = states[slot]
+            for t in range(at, at + n):
+                kt, qt = (x[t].double().view(Hq, dk).repeat_interleave(H // Hq, 0) for x in (k, q))
+                S = dec[t].double()[:, None, None] * S + ks[t].double()[:, None, None] * v[t].double().view(H, dv, 1) * kt[:, None, :]
+                want[t] = (S @ qt[:, :, None])[..., 0].reshape(-1)
+            states[slot] = S
+        at += n
+    state, out = state0.to(DEV), torch.zeros(N, H * dv, device=DEV)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    ops.retention_scan(q.to(DEV), k.to(DEV), v.to(DEV), None if gates else decay.to(DEV), state, _i32(starts), _i32(lens), _i32(slots), out,
+                       H, dk, dv, decay_tok=dec.to(DEV) if gates else None, kscale_tok=ks.to(DEV) if gates else None, qk_heads=Hq, chunked=None)
+    for got, ref in ((out.cpu().double(), want), (state.cpu().double(), states)):
+        assert float((got - ref).abs().max()) <= 2.0 ** -20 * 16 * float(ref.pow(2).mean().sqrt())
+    assert torch.equal(state[1].cpu(), state0[1]) and torch.equal(state[4].cpu(), state0[4])      # a request without rows; nobody's slot
+
+
 @pytest.mark.parametrize("H, dk, dv, rot", [(3, 20, 24, 12), (2, 128, 64, 128), (1, 256, 16, 0), (2, 8, 40, 8)])
 def test_retention_for_single_tokens_in_one_kernel(H, dk, dv, rot):
     """Rotation, state update, output, head-wise norm, gate and scale of a step of single tokens, against the

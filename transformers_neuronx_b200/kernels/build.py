@@ -47,6 +47,7 @@ SOURCES: Dict[str, str] = {
     "rmsnorm": "rmsnorm.cu",
     "rotary_qkv": "rotary_qkv.cu",
     "retention": "retention.cu",
+    "retention_chunked": "retention_chunked.cu",
     "mingru": "mingru.cu",
     "gated_act": "gated_act.cu",
     "conv_qkv": "conv_qkv.cu",

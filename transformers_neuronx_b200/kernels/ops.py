@@ -1302,15 +1302,28 @@ def retention_prep(proj, q_off, k_off, token_request, positions, inv_freq, rot_d
                                   c_int(n_values), c_int(_is_h16(proj)), _stream()), "retention_prep")
 
 
+RETENTION_CHUNKED_BYTES = 1 << 28     # the most scratch memory of a scan in chunks (a state a head and 64 tokens)
+
+
+def retention_chunked_takes(tokens: int, requests: int, n_heads: int, k_dim: int, v_dim: int) -> bool:
+    """Whether a scan that may run in chunks of 64 tokens does: where the requests are several chunks long (one request of
+    128 / 256 / 512 tokens, 16 heads of 128 x 128: 27 us token by token and 34 in chunks, 47 and 38, 88 and 41; 8 requests
+    of 64: 53 and 48, 16 of 16: 29 and 52), and the chunks' states (1 MB each there) stay bounded."""
+    scratch = (tokens // 64 + requests) * n_heads * k_dim * v_dim * 4
+    return tokens >= 192 and tokens >= 64 * requests and scratch <= RETENTION_CHUNKED_BYTES
+
+
 def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_heads, k_dim, v_dim, most_tokens=None,
-                   decay_tok=None, kscale_tok=None, qk_heads=None):
+                   decay_tok=None, kscale_tok=None, qk_heads=None, chunked=False):
     """S <- decay S + k v^T, o = S^T q, token by token for every request of the step (q_start, q_len: its rows;
     q_len 0 or slot < 0: skipped).  q, k: 32-bit [N, n_heads * k_dim]; v: [N, n_heads * v_dim] view in the
     activation type or 32-bit; state: 32-bit [slots, n_heads, v_dim, k_dim]; out: 32-bit [N, n_heads * v_dim].
     most_tokens: an upper bound of any request's rows (default: N); a step of single tokens says 1 and gets
     small stages.  decay_tok, kscale_tok (32-bit [N, n_heads]): S <- decay_tok S + kscale_tok k v^T with numbers of the
     token (absent: decay[h], 1); qk_heads: q and k are [N, qk_heads * k_dim] and head h reads those of
-    h // (n_heads // qk_heads)."""
+    h // (n_heads // qk_heads).  chunked: portions of prompts may run 64 tokens at a time on the tensor cores
+    (csrc/retention_chunked.cu: 32-bit results to a rounding, but where a prompt was cut then shows in the last bits);
+    None: they do wherever the kernels take the sizes (a test hook)."""
     lib = _lib("retention", v)
     N = q.shape[0]
     qk_heads = n_heads if qk_heads is None else int(qk_heads)
@@ -1343,6 +1356,18 @@ def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_he
     R = q_len.shape[0]
     if q_start.shape[0] < R or state_slots.shape[0] < R:
         raise KernelError("q_start and state_slots must cover every request of q_len")
+    if (chunked is not False and k_dim in (64, 128) and v_dim in (64, 128) and v_ld % 4 == 0 and v.data_ptr() % (4 * v.element_size()) == 0
+            and not any(t.data_ptr() % 16 for t in (q, k, state, out))
+            and (chunked is None or retention_chunked_takes(N, R, n_heads, k_dim, v_dim))):
+        chunk_lib = _lib("retention_chunked", v)
+        chunks = chunk_lib.tnx_retention_chunks(c_int(N), c_int(R))
+        adds = torch.empty(chunks * n_heads * v_dim * k_dim, dtype=torch.float32, device=q.device)
+        spans = torch.empty(chunks * n_heads, dtype=torch.float32, device=q.device)
+        _check(chunk_lib.tnx_retention_chunked(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
+                                               _p(state_slots), _p(out), c_int(N), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
+                                               c_int(_is_h16(v)), _p(decay_tok), _p(kscale_tok), c_int(qk_heads), _p(adds), _p(spans),
+                                               _stream()), "retention_scan")
+        return
     _check(lib.tnx_retention_scan(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                   _p(state_slots), _p(out), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
                                   c_int(max(1, int(most_tokens if most_tokens is not None else N))), c_int(_is_h16(v)),

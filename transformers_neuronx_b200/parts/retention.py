@@ -11,7 +11,8 @@ The state S (heads x k_dim x v_dim numbers per request) is state of fixed size i
 request's slot, starts at zero when a request takes the slot, and is carried from step to step.  What enters
 the recurrence is 32-bit: activation and rotation are applied in 32-bit to the projection's output and not rounded again.
 A step's tokens of one request are walked in order by one kernel, portions of prompts and single decoded
-tokens alike, so the state after a token does not depend on how the prompt was cut.
+tokens alike, so the state after a token does not depend on how the prompt was cut; in a 16-bit engine, whose products' kernels
+depend on it anyway, portions may run in chunks of 64 tokens on the tensor cores, to a 32-bit rounding the same.
 """
 from __future__ import annotations
 
@@ -30,7 +31,10 @@ from .spec import RetentionSpec
 
 
 class Retention(FusableMixer):
-    extra_libraries = ("retention",)
+    extra_libraries = ("retention", "retention_chunked")
+    # Chunks lose a little to the token-by-token scan where a state forgets quickly (1.8e-7 and 1.3e-7 at a decay of 0.97) and
+    # gain where it does not (equal at 0.99, 2.7e-7 and 3.6e-7 at 0.999): they run where at least half of the heads gain.
+    CHUNKS_FROM_DECAY = 0.99
 
     def __init__(self, spec: RetentionSpec):
         s = self.spec = spec
@@ -38,6 +42,7 @@ class Retention(FusableMixer):
             raise ValueError(f"{len(s.decay)} decays for {s.n_heads} heads")
         if s.k_dim > 256:
             raise ValueError(f"key size {s.k_dim} is not supported: the scan keeps up to 256 rows of a column in a warp")
+        self.slow = sorted(float(d) for d in s.decay)[s.n_heads // 2] >= self.CHUNKS_FROM_DECAY
         if s.rotary is not None and (s.rotary.dims > s.k_dim or s.rotary.dims % 2):
             raise ValueError(f"{s.rotary.dims} rotated dims do not fit heads of {s.k_dim}")
         activation_code(s.activation)
@@ -95,7 +100,8 @@ class Retention(FusableMixer):
             if not s.joint_norm:
                 o = ctx.scratch(N, H * dv, torch.float32)
             ops.retention_scan(qr, kr, v if vr is None else vr, self.decay, ctx.cache(sub), ctx.q_start, ctx.q_len,
-                               ctx.state_slots, o, H, dk, dv, most_tokens=1 if ctx.decode_only else N)
+                               ctx.state_slots, o, H, dk, dv, most_tokens=1 if ctx.decode_only else N,
+                               chunked=self.slow and ctx.act_dtype != torch.float32)
         if s.joint_norm:
             ops.gated_rms_norm(o, gate, ctx.token_request, self.norm_weight, s.norm_eps, out_scale, inner_out,
                                gate_activation=s.gate_activation)
