@@ -293,6 +293,37 @@ def test_the_recurrence_across_cuts_and_slots(H, G, dk, dv):
     _close(got[2], want[2].reshape(T, -1), 2e-5)
 
 
+@pytest.mark.parametrize("H, G, dk, dv", [(2, 1, 16, 64), (2, 2, 28, 18), (4, 2, 64, 64), (1, 1, 72, 30), (2, 1, 128, 33), (1, 1, 256, 8), (2, 1, 18, 7)])
+def test_the_scan_ahead_over_stage_edges(H, G, dk, dv):
+    """Requests of one token, of whole stages (16, 8 and 4 tokens) and of one more and one less, up to four stages and through
+    all three buffers, in one call; columns that end inside a lane's pair and a warp's.  An output is a sum of at most 256
+    rounded products whose terms' errors are carried on by a state that forgets: 2^-24 x 64 of the largest value."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(dk + dv)
+    lens = [1, 4, 5, 8, 15, 16, 17, 33, 64, 3]
+    N, R = sum(lens), len(lens)
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k = unit(torch.randn(N, G, dk, generator=g)) * dk ** -0.5, unit(torch.randn(N, G, dk, generator=g))
+    v, beta = torch.randn(N, H, dv, generator=g), torch.rand(N, H, generator=g)
+    decay = torch.exp(-torch.rand(N, H, dk, generator=g) ** 2)
+    state0 = torch.randn(R, H, dv, dk, generator=g)
+    want, states, t = torch.zeros(N, H, dv, dtype=torch.float64), state0.double().clone(), 0
+    for r, n in enumerate(lens):
+        S = states[r]
+        for t in range(t, t + n):
+            kt, qt = (x[t].double().repeat_interleave(H // G, 0) for x in (k, q))
+            S = S * decay[t].double()[:, None, :]
+            S = S + (beta[t].double()[:, None] * (v[t].double() - (S @ kt[:, :, None])[..., 0]))[:, :, None] * kt[:, None, :]
+            want[t] = (S @ qt[:, :, None])[..., 0]
+        states[r], t = S, t + 1
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    state, out = state0.to(DEV), torch.zeros(N, H * dv, device=DEV)
+    ops.delta_scan(*(x.reshape(N, -1).to(DEV) for x in (q, k, v, beta, decay)), state, i32([sum(lens[:r]) for r in range(R)]), i32(lens),
+                   i32(list(range(R))), out, H, G, dk, dv)
+    for got, ref in ((out.view(N, H, dv).cpu().double(), want), (state.cpu().double(), states)):
+        assert float((got - ref).abs().max()) <= 2.0 ** -24 * 64 * float(ref.abs().max())
+
+
 def test_a_value_written_long_ago_is_read_back_exactly():
     """No decay, full write strength, orthonormal keys: a value is read back many tokens and steps later bit for bit
     (sums of exact zeros) until its key is written again; a rewritten key returns its latest value, v_old + (v_new -

@@ -17,7 +17,7 @@
 //   library's state kernel afterwards.
 // tnx_delta_scan: a thread block owns C columns (value dims) of one head of one request and walks the request's tokens
 //   of this step in order, the state's columns in registers: a column's k_dim rows are spread over R adjacent lanes,
-//   which add their partial sums of S^T k, S^T q and q.k with shuffles (one round for all three: o = (gS)^T q + (q.k) u).
+//   which add their partial sums of S^T k, S^T q and q.k with shuffles (o = (gS)^T q + (q.k) u).
 //   The tokens' inputs reach shared memory by asynchronous copies, a stage ahead of the walk.
 //   The state is stored [slot, head, v_dim, k_dim] (a column's rows side by side).
 #include "common.cuh"
@@ -192,11 +192,11 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool ta
                  "r"(take ? 16u : 0u) : "memory");
 }
 
-// KPT: rows of a column one thread keeps; R: lanes a column's rows are spread over (KPT * R >= k_dim); a block of 128
-// threads owns 128 / R columns.  The tokens' inputs come in stages through two buffers: while one stage is walked, the
-// next one's copies are in flight, so the walk waits for memory once, at the first stage.  VEC: k_dim is a multiple
-// of 4 and the rows are 16-byte aligned (16-byte copies).
-template <int KPT, int R, bool VEC>
+// Key sizes that are no multiple of 4, and rows off 16-byte boundaries.  KPT: rows of a column one thread keeps; R: lanes
+// a column's rows are spread over (KPT * R >= k_dim); a block of 128 threads owns 128 / R columns.  The tokens' inputs come in
+// stages through two buffers: while one stage is walked, the next one's copies are in flight, so the walk waits for memory
+// once, at the first stage.
+template <int KPT, int R>
 __global__ void __launch_bounds__(128)
 delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ state,
@@ -219,24 +219,13 @@ delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
 
     auto fetch = [&](int t0, int buf) {               // the inputs of tokens t0 .. t0 + ST - 1 of this request's rows
         const int nt = min(ST, len - t0);
-        if (VEC) {
-            for (int e = threadIdx.x; e < nt * (DKP / 4); e += 128) {
-                const int tt = e / (DKP / 4), i = (e % (DKP / 4)) * 4;
-                const size_t t = (size_t)(t_first + t0 + tt);
-                const bool in = i < dk;
-                cp_async16(&qs[buf][tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
-                cp_async16(&ks[buf][tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
-                cp_async16(&gs[buf][tt][i], in ? g + (t * H + h) * dk + i : g, in);
-            }
-        } else {
-            for (int e = threadIdx.x; e < nt * DKP; e += 128) {
-                const int tt = e / DKP, i = e % DKP;
-                const size_t t = (size_t)(t_first + t0 + tt);
-                const bool in = i < dk;
-                cp_async4(&qs[buf][tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
-                cp_async4(&ks[buf][tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
-                cp_async4(&gs[buf][tt][i], in ? g + (t * H + h) * dk + i : g, in);
-            }
+        for (int e = threadIdx.x; e < nt * DKP; e += 128) {
+            const int tt = e / DKP, i = e % DKP;
+            const size_t t = (size_t)(t_first + t0 + tt);
+            const bool in = i < dk;
+            cp_async4(&qs[buf][tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
+            cp_async4(&ks[buf][tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
+            cp_async4(&gs[buf][tt][i], in ? g + (t * H + h) * dk + i : g, in);
         }
         for (int e = threadIdx.x; e < nt * C; e += 128) {
             const int tt = e / C, c = blockIdx.x * C + e % C;
@@ -295,6 +284,188 @@ delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     }
 }
 
+// Two 32-bit numbers at once: an ordinary multiplication, or multiply-add, of each in one instruction.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*(const unsigned long long*)&a), "l"(*(const unsigned long long*)&b));
+    return *(float2*)&d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d)
+        : "l"(*(const unsigned long long*)&a), "l"(*(const unsigned long long*)&b), "l"(*(const unsigned long long*)&c));
+    return *(float2*)&d;
+}
+__device__ __forceinline__ float2 low(const float4& x) { return make_float2(x.x, x.y); }
+__device__ __forceinline__ float2 high(const float4& x) { return make_float2(x.z, x.w); }
+
+// Everything else.  A thread keeps KPT rows, in runs of four neighbours, of two neighbouring columns (what it reads from
+// shared memory feeds both), and multiplies them in pairs; R lanes share the columns.
+// A token's write waits for the sum u = beta (v - S^T k), and that sum over R lanes is most of a token's chain.  So the walk
+// forms it a token ahead, from the state before the write that comes between, and corrects it by one number:
+//     S_t^T k_(t+1) after its decay  =  (g_t S_(t-1))^T (g_(t+1) k_(t+1))  +  (k_t . g_(t+1) k_(t+1)) u_t
+// One chain of a sum and a write then serves two tokens.  The four sums of a lane (the next token's S^T k and this one's
+// S^T q, two columns) are added over the lanes by halving what a lane keeps in the first two rounds; the two numbers that
+// the columns share (q.k and k.gk) likewise.  The lanes whose top bit is clear end up with S^T k and k.gk and form u, the
+// others with S^T q and q.k and form the output.
+// Measured, 16 heads of 128 x 128 on 4 key heads, against a column a lane and the sum inside the token's chain: three
+// requests of 512 tokens 360 -> 198 us, one of 2,048 650 -> 406 (32 heads 969 -> 557), one of 64 26 -> 19; four columns a
+// lane without the sum ahead 251, 799 (799); two 209, 527 (650); eight lanes a column 228, 656.  Errors against 64-bit are equal.
+// What bounds it: one warp a scheduler, about 150 instructions a token and the chain of two tokens in turn.
+// Inputs come in stages through three buffers: one is walked, the next one has landed (the token ahead may be its first), the
+// third one's copies are in flight.
+constexpr int WIDE_THREADS = 128;
+template <int KPT, int R>
+__global__ void __launch_bounds__(WIDE_THREADS)
+delta_scan_ahead_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                        const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ state,
+                        const int* __restrict__ q_start, const int* __restrict__ q_len, const int* __restrict__ state_slots,
+                        float* __restrict__ out, int H, int G, int dk, int dv) {
+    constexpr int DKP = KPT * R, C = WIDE_THREADS / R * 2, ST = scan_stage(DKP), RUNS = KPT / 4;
+    __shared__ __align__(16) float qs[3 * ST][DKP], ks[3 * ST][DKP], gs[3 * ST][DKP];
+    __shared__ __align__(16) float vs[3 * ST][C], bs[3 * ST];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int req = blockIdx.z, h = blockIdx.y;
+    const int len = q_len[req];
+    if (len <= 0) return;                             // a padded request of a captured batch
+    const int slot = state_slots[req];
+    if (slot < 0) return;
+    const int t_first = q_start[req], kvh = h / (H / G);
+    const int jl = threadIdx.x / R * 2, r = threadIdx.x % R;     // the thread's first column in the block, its place among the R lanes
+    const int j0 = blockIdx.x * C + jl;
+
+    auto fetch = [&](int t0, int at) {                // the inputs of tokens t0 .. t0 + ST - 1 of this request into rows `at` on
+        const int nt = min(ST, len - t0);
+        for (int e = threadIdx.x; e < nt * (DKP / 4); e += WIDE_THREADS) {
+            const int tt = e / (DKP / 4), i = (e % (DKP / 4)) * 4;
+            const size_t t = (size_t)(t_first + t0 + tt);
+            const bool in = i < dk;
+            cp_async16(&qs[at + tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
+            cp_async16(&ks[at + tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
+            cp_async16(&gs[at + tt][i], in ? g + (t * H + h) * dk + i : g, in);
+        }
+        for (int e = threadIdx.x; e < nt * C; e += WIDE_THREADS) {
+            const int tt = e / C, c = blockIdx.x * C + e % C;
+            cp_async4(&vs[at + tt][e % C], c < dv ? v + ((size_t)(t_first + t0 + tt) * H + h) * dv + c : v, c < dv);
+        }
+        for (int e = threadIdx.x; e < nt; e += WIDE_THREADS) cp_async4(&bs[at + e], beta + (size_t)(t_first + t0 + e) * H + h, true);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    fetch(ST, ST);                                    // an empty group where the request has one stage
+
+    float2 S[2][KPT / 2];                             // rows 4 (r + R m) .. + 3 of the two columns, in pairs
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const float* st = state + (((size_t)slot * H + h) * dv + min(j0 + c, dv - 1)) * dk;
+#pragma unroll
+        for (int m = 0; m < RUNS; ++m) {
+            const int i = 4 * (r + R * m);
+            const float4 x = j0 + c < dv && i < dk ? *(const float4*)(st + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            S[c][2 * m] = low(x); S[c][2 * m + 1] = high(x);
+        }
+    }
+    const unsigned FULL = 0xffffffffu;
+    const bool top = r & (R / 2);
+    const int mine = r / (R / 4) & 1;                 // the column whose sum the lane ends up with
+    float* o = out + ((size_t)t_first * H + h) * dv + j0 + mine;
+    const bool stores = top && r % (R / 4) == 0 && j0 + mine < dv;
+    // The sums a[0], a[1] (to the lanes with the top bit clear) and b[0], b[1] (to the others) over the R lanes.
+    auto sum_columns = [&](float2 (&a)[2], float2 (&b)[2]) {
+        const float a0 = a[0].x + a[0].y, a1 = a[1].x + a[1].y, b0 = b[0].x + b[0].y, b1 = b[1].x + b[1].y;
+        const float w0 = (top ? b0 : a0) + __shfl_xor_sync(FULL, top ? a0 : b0, R / 2);
+        const float w1 = (top ? b1 : a1) + __shfl_xor_sync(FULL, top ? a1 : b1, R / 2);
+        float w = (mine ? w1 : w0) + __shfl_xor_sync(FULL, mine ? w0 : w1, R / 4);
+#pragma unroll
+        for (int x = R / 8; x > 0; x >>= 1) w += __shfl_xor_sync(FULL, w, x);
+        return w;
+    };
+    auto sum_shared = [&](float a, float b) {
+        float w = (top ? b : a) + __shfl_xor_sync(FULL, top ? a : b, R / 2);
+#pragma unroll
+        for (int x = R / 4; x > 0; x >>= 1) w += __shfl_xor_sync(FULL, w, x);
+        return w;
+    };
+
+    float4 k4[RUNS], q4[RUNS], g4[RUNS];              // of the token that is walked
+    float ahead = 0.f, shared = 0.f, u_before = 0.f;  // its S^T k but for the write before it; (k.gk | q.k); that write's u
+    int at = 0;
+    for (int t0 = 0; t0 < len; t0 += ST) {
+        const int nt = min(ST, len - t0);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                              // this stage and the next one are there; the one before is no longer read
+        if (t0 + 2 * ST < len) fetch(t0 + 2 * ST, at >= ST ? at - ST : 2 * ST);
+        if (t0 == 0) {                                // the first token's sum has no write before it
+            float2 sk[2], none[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+            for (int m = 0; m < RUNS; ++m) {
+                const int i = 4 * (r + R * m);
+                k4[m] = *(const float4*)&ks[0][i]; q4[m] = *(const float4*)&qs[0][i]; g4[m] = *(const float4*)&gs[0][i];
+                const float2 kl = mul2(low(k4[m]), low(g4[m])), kh = mul2(high(k4[m]), high(g4[m]));
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    sk[c] = m ? fma2(kl, S[c][2 * m], sk[c]) : mul2(kl, S[c][2 * m]);
+                    sk[c] = fma2(kh, S[c][2 * m + 1], sk[c]);
+                }
+            }
+            ahead = sum_columns(sk, none);
+        }
+#pragma unroll 2
+        for (int tt = 0; tt < nt; ++tt) {
+            const int row = at + tt, next = t0 + tt + 1 < len ? (row + 1 < 3 * ST ? row + 1 : 0) : row;
+            const float vb = vs[row][jl + mine], b = bs[row];
+            float4 kn[RUNS], gn[RUNS], qn[RUNS];
+            float2 sk[2], sq[2], qk, kgk;
+#pragma unroll
+            for (int m = 0; m < RUNS; ++m) {
+                const int i = 4 * (r + R * m);
+                kn[m] = *(const float4*)&ks[next][i]; gn[m] = *(const float4*)&gs[next][i]; qn[m] = *(const float4*)&qs[next][i];
+            }
+            // u of this token: the sum formed a token ago and the write since
+            const float u_mine = b * (vb - fmaf(shared, u_before, ahead));       // in the lanes whose top bit is clear
+            const float u0 = __shfl_sync(FULL, u_mine, 0, R), u1 = __shfl_sync(FULL, u_mine, R / 4, R);
+#pragma unroll
+            for (int m = 0; m < KPT / 2; ++m) {
+                const float2 kp = m & 1 ? high(k4[m / 2]) : low(k4[m / 2]), qp = m & 1 ? high(q4[m / 2]) : low(q4[m / 2]);
+                const float2 gp = m & 1 ? high(g4[m / 2]) : low(g4[m / 2]);
+                const float2 kg = m & 1 ? mul2(high(kn[m / 2]), high(gn[m / 2])) : mul2(low(kn[m / 2]), low(gn[m / 2]));
+                qk = m ? fma2(qp, kp, qk) : mul2(qp, kp);
+                kgk = m ? fma2(kp, kg, kgk) : mul2(kp, kg);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    S[c][m] = mul2(S[c][m], gp);
+                    sk[c] = m ? fma2(kg, S[c][m], sk[c]) : mul2(kg, S[c][m]);
+                    sq[c] = m ? fma2(qp, S[c][m], sq[c]) : mul2(qp, S[c][m]);
+                }
+            }
+            const float both = sum_shared(kgk.x + kgk.y, qk.x + qk.y);
+            const float sums = sum_columns(sk, sq);
+#pragma unroll
+            for (int m = 0; m < KPT / 2; ++m) {
+                const float2 kp = m & 1 ? high(k4[m / 2]) : low(k4[m / 2]);
+                S[0][m] = fma2(kp, make_float2(u0, u0), S[0][m]);
+                S[1][m] = fma2(kp, make_float2(u1, u1), S[1][m]);
+            }
+            if (stores) *o = fmaf(both, mine ? u1 : u0, sums);
+            o += (size_t)H * dv;
+            ahead = sums; shared = both; u_before = u_mine;
+#pragma unroll
+            for (int m = 0; m < RUNS; ++m) { k4[m] = kn[m]; g4[m] = gn[m]; q4[m] = qn[m]; }
+        }
+        at = at + ST < 3 * ST ? at + ST : 0;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        float* st = state + (((size_t)slot * H + h) * dv + j0 + c) * dk;
+#pragma unroll
+        for (int m = 0; m < RUNS; ++m) {
+            const int i = 4 * (r + R * m);
+            if (j0 + c < dv && i < dk) *(float4*)(st + i) = make_float4(S[c][2 * m].x, S[c][2 * m].y, S[c][2 * m + 1].x, S[c][2 * m + 1].y);
+        }
+    }
+}
+
 }  // namespace
 
 TNX_EXPORT int tnx_delta_prep(const void* proj, int ld, int col0, int b_off, const float* a, int a_ld, const float* conv_w,
@@ -334,17 +505,17 @@ TNX_EXPORT int tnx_delta_scan(const float* q, const float* k, const float* v, co
                               int n_requests, int H, int G, int dk, int dv, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0) return TNX_ERR_BAD_ARG;
+    const bool vec = dk % 4 == 0 && !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)g | (uintptr_t)state) & 15);
 #define DSCAN(KPT, R)                                                                                                   \
     do {                                                                                                                \
-        const int C = 128 / (R);                                                                                        \
+        const int C = (vec ? 2 : 1) * (WIDE_THREADS / (R));                                                             \
         const dim3 grid((dv + C - 1) / C, H, n_requests);                                                               \
         if (vec)                                                                                                        \
-            return tnx_launch_in_order(delta_scan_kernel<KPT, R, true>, grid, dim3(128), 0, stream, q, k, v, beta, g,   \
-                                       state, q_start, q_len, state_slots, out, H, G, dk, dv);                          \
-        return tnx_launch_in_order(delta_scan_kernel<KPT, R, false>, grid, dim3(128), 0, stream, q, k, v, beta, g,      \
+            return tnx_launch_in_order(delta_scan_ahead_kernel<KPT, R>, grid, dim3(WIDE_THREADS), 0, stream, q, k, v,   \
+                                       beta, g, state, q_start, q_len, state_slots, out, H, G, dk, dv);                 \
+        return tnx_launch_in_order(delta_scan_kernel<KPT, R>, grid, dim3(128), 0, stream, q, k, v, beta, g,             \
                                    state, q_start, q_len, state_slots, out, H, G, dk, dv);                              \
     } while (0)
-    const bool vec = dk % 4 == 0 && !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)g) & 15);
     if (dk <= 16) DSCAN(4, 4);
     if (dk <= 32) DSCAN(4, 8);
     if (dk <= 64) DSCAN(8, 8);
