@@ -340,6 +340,25 @@ def test_gemm_tc_refuses_unaligned_sizes():
         o.gemm_tc(a, w, out)
 
 
+@pytest.mark.parametrize("H", [4, 508, 512, 516, 514, 2560])
+@pytest.mark.parametrize("table,act", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float32), (torch.float32, torch.float32)])
+def test_embed_in_pieces_of_four(H, table, act):
+    """Rows in one, two and several blocks of 512 columns, a remainder of one piece, a width that is no multiple of four, and a
+    table off a piece's boundary: one rounding of the product and one of the sum, as the plain expression."""
+    g = torch.Generator().manual_seed(H)
+    for off in (0, 1):
+        tok = torch.randn(50 * H + off, generator=g).to(table).to(DEV)[off:].view(50, H)
+        pos_t = torch.randn(20, H, generator=g).to(table).to(DEV)
+        ids, pos = torch.tensor([3, 49, 0], dtype=torch.int32, device=DEV), torch.tensor([0, 17, 5], dtype=torch.int32, device=DEV)
+        out, out_act = torch.empty(3, H, device=DEV), torch.empty(3, H, dtype=act, device=DEV)
+        ops().embed(tok, None, ids, pos_t, pos, 2, out, out_act, tok_scale=1.0)
+        want = tok.float()[ids.long()] + pos_t.float()[pos.long() + 2]
+        assert torch.equal(out, want) and torch.equal(out_act, want.to(act))
+        pre = torch.randn(3, H, generator=g).to(DEV)
+        ops().embed(None, pre, ids, pos_t, pos, 2, out, None)
+        assert torch.equal(out, pre + pos_t.float()[pos.long() + 2])
+
+
 # ---- attention over the paged cache ----------------------------------------------------------------
 def plain_attention(q, k, v, n_heads, n_kv, scale, first_pos, window):
     """q [Tq, n_heads, d] at positions first_pos.., k/v [Tk, n_kv, d] -> [Tq, n_heads, d], by the
