@@ -598,7 +598,8 @@ def decode_attention_plan(pairs: int, sms: int, head_dim: int, max_pages: int):
     against the one chosen here), the fastest plan keeps all blocks on the GPU at once where it can and
     gives the SMs equal numbers of them:
       * few pairs: blocks of eight warps, as many splits as fill two blocks per SM (1 / 2 rows of 32
-        heads: 13 / 18 us);
+        heads: 13 / 18 us); none below 24 pages, where merging two splits through scratch memory costs more than the
+        pages (one row of 12 heads of 64 over 190 tokens: 4.6 us, with two splits 6.6);
       * about one pair per SM (0.75 to 1): one block of sixteen warps each and no split (4 rows: 28 us,
         eight warps and two splits 30);
       * up to a third of four blocks per SM: four warps and three splits (6 rows: 39 us; eight warps and
@@ -615,6 +616,8 @@ def decode_attention_plan(pairs: int, sms: int, head_dim: int, max_pages: int):
     most = max(1, max_pages // 8)
     wide = 16 if head_dim <= 128 else 8
     if pairs * 4 <= sms * 3:
+        if most <= 2:
+            return 8, 1
         if most <= 4 and pairs * 4 >= sms:
             return wide, 1
         return 8, max(1, min(most, 32, (2 * sms) // max(1, pairs)))
@@ -644,18 +647,16 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
     With shared key/value heads always, but for the shortest steps (16 heads on one, 100 tokens: 4.6 us with a block a head,
     6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1).  Without, where the other kernel's lanes idle (head sizes that
     are no power of two: 80 dims, 8 rows of 32 heads over up to 1,400 tokens 34 and 26 us, 64 rows 164 and 135), with
-    few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 13.8 and 10.7 us; 8 rows 35 and 31) and with
-    many long ones (64 rows 172 and 166); between those a block a head is as fast or faster (16 rows 53 and 56 us; heads of
-    64, 8 rows over 1,000 tokens 16 and 21)."""
+    few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 13.8 and 10.7 us, of 12 heads of 64 over 400 7.0
+    and 5.0; 8 rows of 32 heads of 128 35 and 31) and with many long ones (64 rows 172 and 166); between those a block a
+    head is as fast or faster (16 rows 53 and 56 us; heads of 64, 8 rows over 1,000 tokens 16 and 21)."""
     blocks = rows * n_heads
     if max_pages <= 12 and blocks <= sms:
         return False
     if n_heads != n_kv:
         return True
-    if head_dim == 64:
-        return False
-    if max_pages < 32:
-        return max_pages > 12 and 2 * blocks <= sms
+    if head_dim == 64 or max_pages < 32:
+        return max_pages > (16 if head_dim == 64 else 12) and 2 * blocks <= sms
     return head_dim != 128 or blocks <= 2 * sms or blocks > 4 * sms
 
 
