@@ -128,6 +128,55 @@ def test_retention_scan_carries_its_state_across_cuts_and_requests(H, dk, dv):
     assert float((state[1] - 7.0).abs().max()) == 0.0 and float(state[3].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("dv, H, N", [(64, 3, 171), (128, 5, 103), (256, 2, 257)])
+@pytest.mark.parametrize("dtype, step", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
+@pytest.mark.parametrize("activation", [None, "silu", "sigmoid", "gelu_new"])
+def test_many_heads_are_normalised_in_pieces_of_eight(dv, H, N, dtype, step, activation):
+    """The form from 512 (token, head) pairs on: pair counts that fill neither a warp's rounds nor a block, a padded row, gates in
+    a wider buffer; one rounding of a 32-bit result."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(dv)
+    o, w = torch.randn(N, H * dv, generator=g), torch.rand(dv, generator=g) + 0.5
+    wide = torch.randn(N, 16 + H * dv, generator=g).to(dtype)
+    rows = [0] * N
+    rows[7] = -1
+    out = torch.full((N, H * dv), 9.0, dtype=dtype, device=DEV)
+    ops.headwise_gated_rms_norm(o.to(DEV), wide.to(DEV)[:, 16:] if activation else None, _i32(rows), w.to(DEV), 1e-5, 0.7, out, H, dv,
+                                gate_activation=activation or "silu")
+    x = o.double().view(N, H, dv)
+    y = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()
+    if activation:
+        z = wide[:, 16:].double().view(N, H, dv)
+        y = y * {"silu": lambda t: t * torch.sigmoid(t), "sigmoid": torch.sigmoid,
+                 "gelu_new": lambda t: torch.nn.functional.gelu(t, approximate="tanh")}[activation](z)
+    y, got = (0.7 * y).reshape(N, -1), out.cpu().double()
+    keep = torch.arange(N) != 7
+    assert bool(((got - y).abs()[keep] <= step * y.abs()[keep] + 1e-6).all()) and float((got[7] - 9.0).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("H, dk, rot", [(16, 128, 128), (3, 20, 8), (2, 64, 32), (1, 12, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_queries_and_keys_turn_in_pieces_of_four(H, dk, rot, dtype):
+    """Whole and partly rotated heads, more and fewer pieces than threads; the angle is a 32-bit number, and a turned number has
+    two rounded products and a rounded sum: 2^-22 of the pair's size covers them and the sine's own error."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(dk)
+    N, W = 5, H * dk
+    proj = torch.randn(N, 8 + 2 * W, generator=g).to(dtype)
+    freq = torch.rand(rot // 2, generator=g)
+    pos, rows = [0, 3, 1000, 7, 2047], [0, 0, 1, -1, 2]
+    q, k = torch.full((N, W), 9.0, device=DEV), torch.full((N, W), 9.0, device=DEV)
+    ops.retention_prep(proj.to(DEV), 8, 8 + W, _i32(rows), _i32(pos), freq.to(DEV), rot, 0.3, q, k, H, dk)
+    angle = (torch.tensor(pos).float()[:, None] * freq).double()[:, None, :]
+    for got, off, scale in ((q, 8, 1.0), (k, 8 + W, 0.3)):
+        x = proj[:, off:off + W].double().view(N, H, dk)
+        u, v = x[..., :rot // 2], x[..., rot // 2:rot]
+        want = torch.cat([u * angle.cos() - v * angle.sin(), v * angle.cos() + u * angle.sin(), x[..., rot:]], -1) * scale
+        err = (got.cpu().double().view(N, H, dk) - want).abs()
+        size = torch.cat([torch.sqrt(u * u + v * v)] * 2 + [x[..., rot:].abs()], -1) * scale
+        assert bool((err <= 2.0 ** -22 * size + 1e-12)[[0, 1, 2, 4]].all()) and float((got[3] - 9.0).abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("H, Hq, dk, dv", [(2, 2, 128, 128), (4, 2, 128, 64), (3, 3, 64, 64), (2, 1, 64, 128)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("gates", [False, True])

@@ -93,7 +93,10 @@ delta_prep_kernel(const T* __restrict__ proj, int ld, int col0, int b_off, const
 
 // The same with eight channels a thread (16-byte loads of the projections and the state, the taps' loads independent of
 // one another): sizes and addresses in multiples of eight channels.
-template <typename T>
+// TAPS: the number of taps where it is the usual four (a thread then has all its rows' loads in flight; one after the other a
+// token's three rounds of four loads are what its block waits for), 0: any.  1,536 tokens, 16 heads
+// of 128 on 4: 34.2 -> 29.0 us; about half of that is exponentials, logarithms and divisions in full 32-bit precision.
+template <typename T, int TAPS>
 __global__ void __launch_bounds__(256)
 delta_prep_vec_kernel(const T* __restrict__ proj, int ld, int col0, int b_off, const float* __restrict__ a, int a_ld,
                   const float* __restrict__ conv_w, int taps, T* state, const int* __restrict__ token_request,
@@ -116,15 +119,13 @@ delta_prep_vec_kernel(const T* __restrict__ proj, int ld, int col0, int b_off, c
     auto conv8 = [&](int c, float (&s)[8]) {          // channels c .. c + 7: convolution, state shift, activation
 #pragma unroll
         for (int i = 0; i < 8; ++i) s[i] = 0.f;
-        for (int b = keep; b >= 0; --b) {             // oldest first, as the one-channel form adds them
-            const T* src = row + c;                   // the value b positions back: this step's rows, the state, or zero
-            if (b > 0) {
-                if (pos - b < 0) src = nullptr;
-                else if (idx - b >= 0) src = row + c - (ptrdiff_t)b * ld;
-                else src = st ? st + (size_t)(keep + idx - b) * C + c : nullptr;
-            }
-            Vec8<T> x;
-            if (src) x.load(src); else x.zero();
+        auto source = [&](int b) -> const T* {        // the value b positions back: this step's rows, the state, or zero
+            if (b == 0) return row + c;
+            if (pos - b < 0) return nullptr;
+            if (idx - b >= 0) return row + c - (ptrdiff_t)b * ld;
+            return st ? st + (size_t)(keep + idx - b) * C + c : nullptr;
+        };
+        auto tap = [&](int b, const Vec8<T>& x) {
             const float* w = conv_w + (size_t)(keep - b) * C + c;
             const float4 w0 = *(const float4*)w, w1 = *(const float4*)(w + 4);
             float xv[8];
@@ -132,9 +133,34 @@ delta_prep_vec_kernel(const T* __restrict__ proj, int ld, int col0, int b_off, c
             s[0] = fmaf(w0.x, xv[0], s[0]); s[1] = fmaf(w0.y, xv[1], s[1]); s[2] = fmaf(w0.z, xv[2], s[2]);
             s[3] = fmaf(w0.w, xv[3], s[3]); s[4] = fmaf(w1.x, xv[4], s[4]); s[5] = fmaf(w1.y, xv[5], s[5]);
             s[6] = fmaf(w1.z, xv[6], s[6]); s[7] = fmaf(w1.w, xv[7], s[7]);
-            // a request's single row moves its past on: what is b back now is b + 1 back for the next token (the slot
-            // written here was read one round ago)
-            if (alone && st && b < keep) x.store(st + (size_t)(keep - 1 - b) * C + c);
+        };
+        // oldest first, as the one-channel form adds them; a request's single row moves its past on: what is b back now is
+        // b + 1 back for the next token
+        if constexpr (TAPS > 0) {
+            Vec8<T> x[TAPS];
+#pragma unroll
+            for (int b = TAPS - 1; b >= 0; --b) {
+                const T* src = source(b);
+                if (src) x[b].load(src); else x[b].zero();
+            }
+#pragma unroll
+            for (int b = TAPS - 1; b >= 0; --b) {
+                tap(b, x[b]);
+                if (alone && st && b < TAPS - 1) x[b].store(st + (size_t)(TAPS - 2 - b) * C + c);
+            }
+        } else {
+            for (int b = keep; b >= 0; --b) {         // the slot written here was read one round ago
+                const T* src = source(b);
+                Vec8<T> x;
+                if (src) x.load(src); else x.zero();
+                tap(b, x);
+                if (alone && st && b < keep) x.store(st + (size_t)(keep - 1 - b) * C + c);
+            }
+        }
+        if (act == TNX_ACT_SILU) {                    // inline: the usual one
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[i] = s[i] / (1.f + expf(-s[i]));
+            return;
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) s[i] = apply_activation(s[i], act);
@@ -488,7 +514,7 @@ TNX_EXPORT int tnx_delta_prep(const void* proj, int ld, int col0, int b_off, con
                         (uintptr_t)q_out | (uintptr_t)k_out | (uintptr_t)v_out | (uintptr_t)g_out) & 15);
 #define DPREP(T)                                                                                                        \
     do {                                                                                                                \
-        auto kernel = vec ? delta_prep_vec_kernel<T> : delta_prep_kernel<T>;                                            \
+        auto kernel = !vec ? delta_prep_kernel<T> : taps == 4 ? delta_prep_vec_kernel<T, 4> : delta_prep_vec_kernel<T, 0>;                                            \
         if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
         return tnx_launch_in_order(kernel, dim3(n_tokens, parts), dim3(256), smem, stream, (const T*)proj, ld, col0,    \
                                    b_off, a, a_ld, conv_w, taps, (T*)state, token_request, positions, q_start, q_len,   \
