@@ -446,6 +446,37 @@ def test_the_entry_point_class_and_the_command_line(tmp_path):
     assert r.returncode == 0 and "generated_sequence=" in r.stdout, r.stderr
 
 
+@pytest.mark.parametrize("counts, N, K", [((1, 0, 32, 33), 256, 64), ((255, 256, 257), 264, 72), ((31, 513, 0, 0, 64), 520, 200),
+                                          ((0, 0), 128, 64), ((700, 1), 1032, 1096), ((40,) * 90, 1600, 136)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_grouped_product_in_pairs(counts, N, K, out_dtype):
+    """Every tile's rows against its group's matrix: groups without rows, tiles of one granule, whole tiles and what is left
+    over, widths and depths that fill no tile, more tiles than pairs of CTAs, tiles without a group; rows of no tile stay."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(7)
+    groups, spans, granule, used = [], [], 0, []
+    for e, n in enumerate(counts):
+        for j in range(0, n, 256):
+            take = -(-min(256, n - j) // 32)
+            groups.append(e); spans.append(granule * 8 + take - 1); used.append((granule * 32, take * 32, e))
+            granule += take
+    groups += [-1] * 3
+    spans += [0] * 3
+    M = granule * 32 + 64
+    a = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    w = torch.randn(len(counts), N, K, generator=g).to(torch.bfloat16)
+    out = torch.full((M, N), 7.0, dtype=out_dtype, device=DEV)
+    ops.gemm_tc_grouped(a.to(DEV), w.to(DEV), out, _i32(groups), 256, 0, _i32(spans))
+    ops.raise_on_device_error()
+    out = out.cpu().double()
+    for row, n, e in used:
+        x, m = a[row:row + n].double(), w[e].double()
+        # K sums in 32 bits, each off by at most an ulp (the tensor cores cut off), and the result's own rounding
+        bound = K * 2.0 ** -23 * (x.abs() @ m.abs().T) + (2.0 ** -8 * (x @ m.T).abs() if out_dtype == torch.bfloat16 else 0)
+        assert bool(((out[row:row + n] - x @ m.T).abs() <= bound).all())
+    assert bool((out[M - 64:] == 7.0).all())
+
+
 @pytest.mark.parametrize("N, W, E, top, F, on_input", [(300, 256, 8, 2, 128, True), (129, 320, 3, 3, 72, True),
                                                       (1000, 64, 40, 1, 200, False), (64, 128, 5, 4, 64, True),
                                                       (2, 2048, 8, 2, 2816, True), (9, 256, 8, 2, 136, True),      # tiles of 16

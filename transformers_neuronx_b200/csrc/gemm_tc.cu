@@ -60,7 +60,8 @@ struct Params {
                                  // through distributed shared memory instead of scratch memory
     int sk_tiles;                // paired kernel: the last sk_tiles output tiles are shared out by K blocks
     int sk_pairs;                // ... over the first sk_pairs pairs
-    const int* group_of_tile;    // grouped product: the group of every tile of tokens (128 of them, or BN in the swapped form), -1: none;
+    const int* span_of_tile;     // grouped product in CTA pairs: a tile's rows, (first row / 32) * 8 + rows / 32 - 1
+    const int* group_of_tile;    // grouped product: the group of every tile of tokens (up to 256 of them in CTA pairs, or BN), -1: none;
     int group_rows;              //   W holds group_rows rows per group, a tile of group g reads W's rows from g * group_rows on
     int batch_w_step;            // batched product (not swapped, K not split): blockIdx.z = b multiplies the columns of A from
     int batch_a_step;            //   b * batch_a_step on with W's rows from b * batch_w_step on and writes the columns of C from
@@ -381,13 +382,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     // A grouped product: every tile of tokens belongs to one group (an expert) and multiplies that group's rows of W.
     // Which group is written by the kernel before this one, so it is read behind the dependency wait; a tile without
     // a group has nothing to do (nothing has been set up yet, so the whole CTA may leave).
-    // (In the swapped form the tokens are the Q operand; the CTAs of a cluster share their tile of tokens, so they leave together.)
+    // (The tokens are the Q operand; the CTAs of a cluster share their tile of tokens, so they leave together.)
     int q_row0 = tile_q * BN, p_row0 = tile_p * TILE_P;
-    if (p.group_of_tile != nullptr) {
+    if (SWAP && p.group_of_tile != nullptr) {
         pdl_wait();
-        const int g = p.group_of_tile[SWAP ? tile_q : tile_p];
+        const int g = p.group_of_tile[tile_q];
         if (g < 0) return;
-        if (SWAP) p_row0 += g * p.group_rows; else q_row0 += g * p.group_rows;
+        p_row0 += g * p.group_rows;
     }
     q_row0 += batch * p.batch_w_step;
     // Split K summed in a cluster, swapped form, 2, 4 or 8 splits: every CTA sends the bands of its partial tile
@@ -1083,6 +1084,15 @@ __host__ __device__ constexpr uint32_t instr_desc_pair(int n) {      // M = 256 
     return (1u << 4) | IDESC_H16_AB | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 
+//
+// GROUPED: a grouped product, with the operands' places exchanged.  The weights' 256 rows fill the 256-row operand and a tile of
+// tokens is the other one, only as wide as the tile has tokens (p.span_of_tile: a multiple of 32 up to 256, and rows begin at any
+// multiple of 32): the last tile of a group is rarely full, and the multiplications are what a tile costs.  tiles_m tiles of
+// tokens, the first ones of which have a group (p.group_of_tile, which an earlier kernel wrote: nothing can be asked for before
+// that has finished), whole tiles only.  16 experts of 2048 x 4096 and 4096 x 2048 with 512 rows each and all that
+// lies around them take 517 us (614 in 128 x 256 tiles of one CTA each, whose last tiles were 128 rows whatever they held); with
+// 128 rows each 223 (295), with 64 206 (209); 128 experts of 1536 x 2048 and 2048 x 768 with 128 rows each 454 (608).
+template <bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                     const __grid_constant__ CUtensorMap map_res, const __grid_constant__ CUtensorMap map_out,
@@ -1101,6 +1111,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
     const int num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
+    if constexpr (GROUPED) {
+        pdl_launch_dependents();
+        pdl_wait();
+        int used = 0;
+        for (int i = 0; i < tiles_m; i += 32)
+            used += __popc(__ballot_sync(0xffffffffu, i + lane < tiles_m && p.group_of_tile[i + lane] >= 0));
+        tiles_m = used;
+    }
     const int n_tiles = tiles_m * tiles_n;                    // 256 x 256 tiles
     // Work of pair g of G.  Tiles [0, dp_tiles) are computed whole, tile g + t * G by pair g.  The
     // last sk_tiles tiles (fewer than G: they would leave pairs idle in a last wave) are laid end to
@@ -1129,6 +1147,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             tile = g + (i - n_seg) * G; kb0 = 0; kb1 = num_kb;
         }
     };
+    // GROUPED: a tile's first token, and the columns its tokens take of the accumulator; each CTA of the pair brings half of them
+    auto row_of = [&](int tm) { return (p.span_of_tile[tm] >> 3) * 32; };
+    auto columns_of = [&](int tm) { return ((p.span_of_tile[tm] & 7) + 1) * 32; };
     // A walk over the K blocks this pair loads, item after item, without a division per step: the
     // loading thread has a few hundred cycles for each.
     struct Cursor { int item, kb, kb1, x_row, w_row, stage; };
@@ -1137,6 +1158,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         int tile; item_of(c.item, tile, c.kb, c.kb1);
         c.x_row = (tile % tiles_m) * 256 + (int)rank * 128;
         c.w_row = (tile / tiles_m) * 256 + (int)rank * 128;
+        if constexpr (GROUPED) {                              // map_p: the weights, map_q: the tokens
+            const int tm = tile % tiles_m;
+            c.x_row = p.group_of_tile[tm] * p.group_rows + (tile / tiles_m) * 256 + (int)rank * 128;
+            c.w_row = row_of(tm) + (int)rank * (columns_of(tm) / 2);
+        }
     };
     auto cursor_next = [&](Cursor& c) {
         c.stage = c.stage + 1 == CSTAGES ? 0 : c.stage + 1;
@@ -1152,7 +1178,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         tma_load_2d_pair(smem + (size_t)c.stage * STAGE_BYTES, &map_p, full0(c.stage), c.kb * BLOCK_K, c.x_row);
     };
 
-    pdl_launch_dependents();
+    if constexpr (!GROUPED) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < CSTAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }   // 4 warps x 2 CTAs
@@ -1176,7 +1202,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         cursor_set(cw);
         for (; issued < total && issued < CSTAGES; ++issued) { load_weights(cw); cursor_next(cw); }   // weights: before the dependency wait
     }
-    pdl_wait();
+    if constexpr (!GROUPED) pdl_wait();
     const uint32_t tmem_base = tmem_base_smem;
     bool ok = true;
 
@@ -1197,13 +1223,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         }
     } else if (warp == 1) {
         if (leader && lane == 0) {
-            constexpr uint32_t idesc = instr_desc_pair(256);
             int mma_stage = 0;
             uint32_t mma_phase = 0;
             for (int t = 0; t < n_items && ok; ++t) {
                 const int acc = t & 1;
                 const uint32_t acc_ph = (uint32_t)((t >> 1) & 1);
                 int tile, kb0, kb1; item_of(t, tile, kb0, kb1);
+                uint32_t idesc = instr_desc_pair(256);
+                if constexpr (GROUPED) idesc = instr_desc_pair(columns_of(tile % tiles_m));
                 ok = mbar_wait(&acc_empty[acc], acc_ph ^ 1, p.err, 22);      // both CTAs drained this accumulator
                 if (!ok) break;
                 tc_fence_after();
@@ -1240,6 +1267,34 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 const int et = threadIdx.x - 64;
                 for (int j = et; j < 256; j += 128) bias_tile[acc][j] = (tn * 256 + j < p.rows_q) ? p.bias[tn * 256 + j] : 0.f;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
+            }
+            if constexpr (GROUPED) {
+                // a lane is a feature, a column a token: two columns at a time, neighbouring lanes exchange halves, so
+                // that a lane stores two neighbouring features of one token
+                const int f = tn * 256 + (int)rank * 128 + quad * 32 + (lane & ~1), columns = columns_of(tm), row0 = row_of(tm);
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], acc_ph, p.err, 24));
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int c = 0; c < columns; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256 + c), r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const uint32_t other = __shfl_xor_sync(0xffffffffu, lane & 1 ? r[j] : r[j + 1], 1);
+                        const float a = __uint_as_float(lane & 1 ? other : r[j]), b = __uint_as_float(lane & 1 ? r[j + 1] : other);
+                        const size_t at = (size_t)(row0 + c + j + (lane & 1)) * p.ldc + f;
+                        if (f < p.rows_q) {
+                            if (p.c_is_h16) *(h16x2*)((h16*)p.C + at) = floats_to_h16x2(a, b);
+                            else *(float2*)((float*)p.C + at) = make_float2(a, b);
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[acc]), 0));
+                continue;
             }
             const int row0 = tm * 256 + (int)rank * 128 + quad * 32;
             if (whole && tma_epilogue && lane == 0) epilogue_tma_begin(epi, row0, tn * 256);
@@ -1479,6 +1534,20 @@ TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int n_sms, int* splits, lon
     return 0;
 }
 
+template <bool GROUPED>
+static int launch_pair(int ctas, cudaStream_t stream, const CUtensorMap& mp, const CUtensorMap& mq, const CUtensorMap& mres,
+                       const CUtensorMap& mout, const Params& p, int tiles_m, int tiles_n, int tma_epilogue) {
+    constexpr size_t smem = (size_t)CSTAGES * (TILE_P * BLOCK_K * 2 + 128 * BLOCK_K * 2) + PAIR_EPI_BYTES + 1024;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return tnx_launch_ex(1, gemm_tc_pair_kernel<GROUPED>, dim3(ctas), dim3(NUM_THREADS), smem, stream, mp, mq, mres, mout, p,
+                         tiles_m, tiles_n, tma_epilogue);
+}
+
 TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, const float* residual, void* C,
                            int M, int N, int K, int lda, int ldw, int ldc, int act, int c_h16,
                            int splits, float* scratch, int* counters, int* err_word, cudaStream_t stream) {
@@ -1525,20 +1594,12 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
             }
             p.sk_tiles = mt.sk_tiles; p.sk_pairs = mt.sk_pairs;
             if (!make_map(&mq, W, N, K, ldw, 128)) return TNX_ERR_UNSUPPORTED;
-            constexpr size_t psmem = (size_t)CSTAGES * (TILE_P * BLOCK_K * 2 + 128 * BLOCK_K * 2) + PAIR_EPI_BYTES + 1024;
             // A 32-bit residual goes through TMA boxes when the row pitch and the addresses allow it.
             CUtensorMap mres = mp, mout = mp;
             int tma_epilogue = 0;
             if (residual && !c_h16 && ldc % 4 == 0 && !(((uintptr_t)residual | (uintptr_t)C) & 15))
                 tma_epilogue = make_map_f32(&mres, residual, M, N, ldc, 32) && make_map_f32(&mout, C, M, N, ldc, 32);
-            static bool pconfigured = false;
-            if (!pconfigured) {
-                cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
-                if (e != cudaSuccess) return (int)e;
-                pconfigured = true;
-            }
-            return tnx_launch_ex(1, gemm_tc_pair_kernel, dim3(2 * mt.pairs), dim3(NUM_THREADS), psmem, stream, mp, mq, mres, mout, p,
-                                 ptiles_m, ptiles_n, tma_epilogue);
+            return launch_pair<false>(2 * mt.pairs, stream, mp, mq, mres, mout, p, ptiles_m, ptiles_n, tma_epilogue);
         }
         if (!make_map(&mq, W, N, K, ldw, PBN)) return TNX_ERR_UNSUPPORTED;
         constexpr size_t smem = (size_t)PSTAGES * (TILE_P * BLOCK_K * 2 + PBN * BLOCK_K * 2) + 1024;
@@ -1570,33 +1631,30 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
     return launch<128, 3, true>(mp, mq, p, grid, stream);
 }
 
-// A grouped product: C[m, :] = A[m, :] W_g^T for the rows m of every 128-row tile, g = group_of_tile[m / 128] (a device
-// array written by an earlier kernel; -1: the tile is skipped).  W holds the groups' matrices one after the other,
-// [groups * N, K]; A is [M, K] with M a multiple of 128; C is [M, ldc] in the 16-bit type or 32-bit.  No bias, no
-// activation: what follows a group's product is the caller's own kernel.
-TNX_EXPORT int tnx_gemm_tc_grouped(const void* A, const void* W, void* C, int M, int N, int K, int groups, int lda, int ldw,
-                                   int ldc, int c_h16, const int* group_of_tile, int* err_word, cudaStream_t stream) {
-    if (M <= 0 || N <= 0 || groups <= 0) return 0;
-    if (M % TILE_P || K <= 0 || K % 8 || lda % 8 || ldw % 8 || lda < K || ldw < K || ldc < N) return TNX_ERR_UNSUPPORTED;
-    if ((((uintptr_t)A | (uintptr_t)W) & 15) || (long long)groups * N >= (1ll << 31)) return TNX_ERR_UNSUPPORTED;
-    if (!err_word || !group_of_tile) return TNX_ERR_BAD_ARG;
+// A grouped product in CTA pairs: C[m, :] = A[m, :] W_g^T for the rows m of every tile of tokens, g = group_of_tile[tile] (a
+// device array written by an earlier kernel; -1: this tile has no group, nor has one after it).  A tile has up to 256 rows, given
+// by span_of_tile (first row / 32 * 8 + rows / 32 - 1; tiles do not overlap and end by row M, a multiple of 32).  W holds the
+// groups' matrices one after the other, [groups * N, K]; C is [M, ldc] in the 16-bit type or 32-bit.  No bias, no activation:
+// what follows a group's product is the caller's own kernel.
+TNX_EXPORT int tnx_gemm_tc_grouped(const void* A, const void* W, void* C, int M, int N, int K, int groups, int tiles, int lda,
+                                   int ldw, int ldc, int c_h16, const int* group_of_tile, const int* span_of_tile,
+                                   int* err_word, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || groups <= 0 || tiles <= 0) return 0;
+    if (M % 32 || K <= 0 || K % 8 || lda % 8 || ldw % 8 || lda < K || ldw < K || ldc < N || N % 2 || ldc % 2) return TNX_ERR_UNSUPPORTED;
+    if ((((uintptr_t)A | (uintptr_t)W) & 15) || ((uintptr_t)C & 7) || (long long)groups * N >= (1ll << 31)) return TNX_ERR_UNSUPPORTED;
+    if (!err_word || !group_of_tile || !span_of_tile) return TNX_ERR_BAD_ARG;
     Params p{};
     p.K = K; p.ldc = ldc; p.act = TNX_ACT_NONE; p.c_is_h16 = c_h16; p.C = C; p.err = err_word;
     p.rows_p = M; p.rows_q = N; p.splits = 1; p.kb_per_split = (K + BLOCK_K - 1) / BLOCK_K;
-    p.group_of_tile = group_of_tile; p.group_rows = N;
-    CUtensorMap mp, mq;
-    if (!make_map(&mp, A, M, K, lda, TILE_P)) return TNX_ERR_UNSUPPORTED;
-    // tiles of 128 x 256 where a group is wide enough: half as many activation bytes per FLOP into shared memory
-    // (measured on 8 experts of 11008 x 4096 and 4096 x 5504, 4,096 rows: 2.42 against 3.28 ms for four layers' products).
-    // Two stages, so that two CTAs fit on an SM and one's products run while the other stores its tile: 16 experts of
-    // 2048 x 2048 and 2048 x 1024 with about 410 rows each take 100 and 77 us, against 131 and 106 with one CTA of four stages;
-    // 8 of 11008 x 4096 and 4096 x 5504 with about 1,024 rows 763 and 371 against 907 and 449.
-    if (N >= 256) {
-        if (!make_map(&mq, W, groups * N, K, ldw, 256)) return TNX_ERR_UNSUPPORTED;
-        return launch<256, 2, false>(mp, mq, p, dim3(M / TILE_P, (N + 255) / 256, 1), stream);
-    }
-    if (!make_map(&mq, W, groups * N, K, ldw, 128)) return TNX_ERR_UNSUPPORTED;
-    return launch<128, 6, false>(mp, mq, p, dim3(M / TILE_P, (N + 127) / 128, 1), stream);
+    p.group_of_tile = group_of_tile; p.span_of_tile = span_of_tile; p.group_rows = N;
+    CUtensorMap mw, mx;
+    if (!make_map(&mw, W, groups * N, K, ldw, 128) || !make_map(&mx, A, M, K, lda, 128)) return TNX_ERR_UNSUPPORTED;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return TNX_ERR_UNSUPPORTED;
+    const int tiles_n = (N + 255) / 256;
+    const long long most = (long long)tiles * tiles_n;
+    return launch_pair<true>(2 * (int)(most < sms / 2 ? most : sms / 2), stream, mw, mx, mw, mw, p, tiles, tiles_n, 0);
 }
 
 // A batched product: C[m, b * c_step + n] = sum_k A[m, b * a_step + k] W[b * N + n, k] for b < batches, n < N, k < K, in one

@@ -1,11 +1,11 @@
 // Routed experts on the tensor cores: the (token, chosen expert) pairs are sorted by expert into a layout in which every
-// expert's rows begin at a multiple of the tile (128 rows where experts get many rows; 16, 32 or 64 where they get few),
-// so that each tile belongs to one expert and the two products of an expert run as grouped tensor-core products
+// expert's rows begin at a multiple of the granule, and each tile belongs to one expert: 16, 32, 64 or 128 rows, which are the
+// granule too, where experts get few rows; up to 256 rows, of granules of 32, where they get many. The two products of an expert run as grouped tensor-core products
 // (gemm_tc.cu: tnx_gemm_tc_grouped, tnx_gemm_tc_grouped_few).  The kernels of this file are what lies around those products:
 //
 //   moe_plan_kernel      one block: counts per expert, every expert's first row, the expert of every tile (-1 beyond
-//                        the last used tile), and the row of every pair.  Which row of its expert's segment a pair
-//                        gets depends on the order in which threads arrive; a row's result does not depend on where it sits
+//                        the last used tile), how many of a granule's rows are pairs, and the row of every pair.
+//                        Which row of its expert's segment a pair gets depends on the order in which threads arrive; a row's result does not depend on where it sits
 //   moe_gather_kernel    x[row(pair)] = weight * h[token]  (or h[token] when the weight multiplies the output), 16-bit
 //   moe_act_kernel       y = g * sigmoid(alpha g) * (u + up_shift), g and u clamped, from the gate/up product's output
 //                        (moe_act_relu2_kernel: y = relu(u)^2 for experts without a gate)
@@ -13,17 +13,19 @@
 //                        (a pair whose expert is the token itself takes no row: weight * h[token])
 //
 // Nothing is read on the host: the sizes of the buffers follow from the numbers of tokens and experts alone (at most
-// pairs / tile + experts tiles), so a step can be captured in a CUDA graph.
+// pairs / tile + experts tiles, and as many granules), so a step can be captured in a CUDA graph.
 #include "common.cuh"
 
 namespace {
 constexpr int MAX_EXPERTS = 1024;
 constexpr int IDENTITY = -2;      // of a pair's expert, and then of its row: the token itself (-1: a padded row)
 
+// span_of_tile (may be null): where a tile's rows begin and how many granules they take, (first granule) * 8 + granules - 1.
 __global__ void __launch_bounds__(1024)
-moe_plan_kernel(const int* __restrict__ ids, int n_pairs, int n_experts, int max_tiles, int TILE, int* __restrict__ group_of_tile,
+moe_plan_kernel(const int* __restrict__ ids, int n_pairs, int n_experts, int max_tiles, int max_granules, int TILE, int GRANULE,
+                int* __restrict__ group_of_tile, int* __restrict__ span_of_tile, int* __restrict__ rows_of_granule,
                 int* __restrict__ row_of_pair) {
-    __shared__ int count[MAX_EXPERTS], first[MAX_EXPERTS], cursor[MAX_EXPERTS], used_tiles;
+    __shared__ int count[MAX_EXPERTS], first[MAX_EXPERTS], cursor[MAX_EXPERTS], first_tile[MAX_EXPERTS], used_tiles, used_granules;
     pdl_launch_dependents();
     pdl_wait();
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
@@ -36,24 +38,38 @@ moe_plan_kernel(const int* __restrict__ ids, int n_pairs, int n_experts, int max
         if (e >= 0 && lane == __ffs(same) - 1) atomicAdd(&count[e], __popc(same));
     }
     __syncthreads();
-    if (threadIdx.x < 32) {                            // every expert's first tile: a running sum, 32 experts at a time
-        int before = 0;
+    if (threadIdx.x < 32) {                            // every expert's first tile and first granule: running sums, 32 experts at a time
+        int tiles = 0, granules = 0;
         for (int e0 = 0; e0 < n_experts; e0 += 32) {
-            const int e = e0 + lane, t = e < n_experts ? (count[e] + TILE - 1) / TILE : 0;
-            int upto = t;
+            const int e = e0 + lane, n = e < n_experts ? count[e] : 0;
+            const int t = (n + TILE - 1) / TILE, u = (n + GRANULE - 1) / GRANULE;
+            int t_upto = t, u_upto = u;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += v; }
-            if (e < n_experts) first[e] = (before + upto - t) * TILE;
-            before += __shfl_sync(0xffffffffu, upto, 31);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int tv = __shfl_up_sync(0xffffffffu, t_upto, o), uv = __shfl_up_sync(0xffffffffu, u_upto, o);
+                if (lane >= o) { t_upto += tv; u_upto += uv; }
+            }
+            if (e < n_experts) { first_tile[e] = tiles + t_upto - t; first[e] = (granules + u_upto - u) * GRANULE; }
+            tiles += __shfl_sync(0xffffffffu, t_upto, 31);
+            granules += __shfl_sync(0xffffffffu, u_upto, 31);
         }
-        if (lane == 0) used_tiles = before;
+        if (lane == 0) { used_tiles = tiles; used_granules = granules; }
     }
     __syncthreads();
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x) {
-        const int tile = first[e] / TILE, t = (count[e] + TILE - 1) / TILE;
-        for (int j = 0; j < t && tile + j < max_tiles; ++j) group_of_tile[tile + j] = e;
+        const int tile = first_tile[e], t = (count[e] + TILE - 1) / TILE, granule = first[e] / GRANULE;
+        for (int j = 0; j < t && tile + j < max_tiles; ++j) {
+            group_of_tile[tile + j] = e;
+            if (span_of_tile) {
+                const int rows = min(TILE, count[e] - j * TILE);
+                span_of_tile[tile + j] = (granule + j * (TILE / GRANULE)) * 8 + (rows + GRANULE - 1) / GRANULE - 1;
+            }
+        }
+        for (int j = 0; j * GRANULE < count[e] && granule + j < max_granules; ++j)
+            rows_of_granule[granule + j] = min(GRANULE, count[e] - j * GRANULE);
     }
     for (int tile = used_tiles + threadIdx.x; tile < max_tiles; tile += blockDim.x) group_of_tile[tile] = -1;
+    for (int i = used_granules + threadIdx.x; i < max_granules; i += blockDim.x) rows_of_granule[i] = 0;
     for (int i0 = 0; i0 < n_pairs; i0 += blockDim.x) {
         const int i = i0 + threadIdx.x, e = i < n_pairs ? ids[i] : -1;
         const unsigned same = __match_any_sync(0xffffffffu, e);
@@ -92,12 +108,12 @@ moe_gather_kernel(const h16* __restrict__ h, int ld, const float* __restrict__ w
 }
 
 __global__ void __launch_bounds__(256)
-moe_act_kernel(const h16* __restrict__ gu, h16* __restrict__ y, const int* __restrict__ group_of_tile, int TILE, int F,
+moe_act_kernel(const h16* __restrict__ gu, h16* __restrict__ y, const int* __restrict__ rows_of_granule, int GRANULE, int F,
                float gate_max, float up_min, float up_max, float alpha, float up_shift) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x;
-    if (group_of_tile[row / TILE] < 0) return;
+    if (row % GRANULE >= rows_of_granule[row / GRANULE]) return;
     const h16* g = gu + (size_t)row * 2 * F;
     const h16* u = g + F;
     if (F % 8 == 0 && !(((uintptr_t)gu | (uintptr_t)y) & 15)) {
@@ -135,11 +151,11 @@ moe_act_kernel(const h16* __restrict__ gu, h16* __restrict__ y, const int* __res
 
 // Experts without a gate: y = relu(u)^2 from the up product's output [rows, F].
 __global__ void __launch_bounds__(256)
-moe_act_relu2_kernel(const h16* __restrict__ u, h16* __restrict__ y, const int* __restrict__ group_of_tile, int TILE, int F) {
+moe_act_relu2_kernel(const h16* __restrict__ u, h16* __restrict__ y, const int* __restrict__ rows_of_granule, int GRANULE, int F) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x;
-    if (group_of_tile[row / TILE] < 0) return;
+    if (row % GRANULE >= rows_of_granule[row / GRANULE]) return;
     const h16* src = u + (size_t)row * F;
     h16* dst = y + (size_t)row * F;
     if (F % 2 == 0) {
@@ -216,13 +232,16 @@ TNX_EXPORT int tnx_moe_grouped_max_tiles(int n_pairs, int n_experts, int tile) {
     return n_pairs / tile + (n_pairs < n_experts ? n_pairs : n_experts);
 }
 
-TNX_EXPORT int tnx_moe_plan(const int* ids, int n_pairs, int n_experts, int max_tiles, int tile, int* group_of_tile,
-                            int* row_of_pair, cudaStream_t stream) {
+// tile 256: granules of 32 rows and span_of_tile is written; other tiles are their own granules.
+TNX_EXPORT int tnx_moe_plan(const int* ids, int n_pairs, int n_experts, int max_tiles, int max_granules, int tile, int* group_of_tile,
+                            int* span_of_tile, int* rows_of_granule, int* row_of_pair, cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
-    if (n_experts <= 0 || n_experts > MAX_EXPERTS || tile <= 0 || max_tiles < tnx_moe_grouped_max_tiles(n_pairs, n_experts, tile))
+    const int granule = tile == 256 ? 32 : tile;
+    if (n_experts <= 0 || n_experts > MAX_EXPERTS || tile <= 0 || max_tiles < tnx_moe_grouped_max_tiles(n_pairs, n_experts, tile) ||
+        max_granules < tnx_moe_grouped_max_tiles(n_pairs, n_experts, granule) || (tile == 256) != (span_of_tile != nullptr))
         return TNX_ERR_BAD_ARG;
-    return tnx_launch_in_order(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, ids, n_pairs, n_experts, max_tiles, tile,
-                               group_of_tile, row_of_pair);
+    return tnx_launch_in_order(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, ids, n_pairs, n_experts, max_tiles, max_granules, tile,
+                               granule, group_of_tile, span_of_tile, rows_of_granule, row_of_pair);
 }
 
 TNX_EXPORT int tnx_moe_gather(const void* h, int ld, const float* weights, const int* row_of_pair, void* x, int n_pairs, int W,
@@ -232,14 +251,14 @@ TNX_EXPORT int tnx_moe_gather(const void* h, int ld, const float* weights, const
                                (h16*)x, W, top, weight_on_input);
 }
 
-TNX_EXPORT int tnx_moe_act(const void* gu, void* y, const int* group_of_tile, int tile, int rows, int F, float gate_max,
+TNX_EXPORT int tnx_moe_act(const void* gu, void* y, const int* rows_of_granule, int granule, int rows, int F, float gate_max,
                            float up_min, float up_max, float alpha, float up_shift, int form, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (form == 1)
         return tnx_launch_in_order(moe_act_relu2_kernel, dim3(rows), dim3(F >= 512 ? 256 : 128), 0, stream, (const h16*)gu,
-                                   (h16*)y, group_of_tile, tile, F);
+                                   (h16*)y, rows_of_granule, granule, F);
     return tnx_launch_in_order(moe_act_kernel, dim3(rows), dim3(F >= 512 ? 256 : 128), 0, stream, (const h16*)gu, (h16*)y,
-                               group_of_tile, tile, F, gate_max, up_min, up_max, alpha, up_shift);
+                               rows_of_granule, granule, F, gate_max, up_min, up_max, alpha, up_shift);
 }
 
 TNX_EXPORT int tnx_moe_combine(const float* rows, const void* h, int ld, const int* row_of_pair, const float* weights, float* out, int N, int W, int top,
