@@ -648,8 +648,10 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
     6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1).  Without, where the other kernel's lanes idle (head sizes that
     are no power of two: 80 dims, 8 rows of 32 heads over up to 1,400 tokens 34 and 26 us, 64 rows 164 and 135), with
     few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 13.8 and 10.7 us, of 12 heads of 64 over 400 7.0
-    and 5.0; 8 rows of 32 heads of 128 35 and 31) and with many long ones (64 rows 172 and 166); between those a block a
-    head is as fast or faster (16 rows 53 and 56 us; heads of 64, 8 rows over 1,000 tokens 16 and 21)."""
+    and 5.0; 8 rows of 32 heads of 128 35 and 31) and with many long ones (64 rows 172 and 166) if its three blocks an SM leave no
+    more places of the last round empty than the other's four (32 rows of 40 heads up to 700 tokens 38 and 41; of 32
+    heads 49 and 51, with 18 of the rows in use 27 and 30); between those a block a head is as fast or faster (16 rows 53
+    and 56 us; heads of 64, 8 rows over 1,000 tokens 16 and 21)."""
     blocks = rows * n_heads
     if max_pages <= 12 and blocks <= sms:
         return False
@@ -657,7 +659,8 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
         return True
     if head_dim == 64 or max_pages < 32:
         return max_pages > (16 if head_dim == 64 else 12) and 2 * blocks <= sms
-    return head_dim != 128 or blocks <= 2 * sms or blocks > 4 * sms
+    rounds = lambda per: -(-blocks // (per * sms)) * per
+    return head_dim != 128 or blocks <= 2 * sms or (blocks > 4 * sms and rounds(3) <= rounds(4))
 
 
 def grouped_decode_plan(blocks: int, sms: int, heads_per_block: int, max_pages: int):
