@@ -1328,9 +1328,11 @@ RETENTION_CHUNKED_BYTES = 1 << 28     # the most scratch memory of a scan in chu
 def retention_chunked_takes(tokens: int, requests: int, n_heads: int, k_dim: int, v_dim: int) -> bool:
     """Whether a scan that may run in chunks of 64 tokens does: where the requests are several chunks long (one request of
     128 / 256 / 512 tokens, 16 heads of 128 x 128: 27 us token by token and 34 in chunks, 47 and 38, 88 and 41; 8 requests
-    of 64: 53 and 48, 16 of 16: 29 and 52), and the chunks' states (1 MB each there) stay bounded."""
+    of 64: 53 and 48, 16 of 16: 29 and 52), the chunks' states (1 MB each there) stay bounded, and the step is long enough
+    that the device is what it waits for: the two more launches are the host's time before (a layer over 439 tokens of
+    two requests 139 us token by token and 160 in chunks, over 800 of four 180 and 166, over 768 of one 218 and 145)."""
     scratch = (tokens // 64 + requests) * n_heads * k_dim * v_dim * 4
-    return tokens >= 192 and tokens >= 64 * requests and scratch <= RETENTION_CHUNKED_BYTES
+    return tokens >= (512 if requests == 1 else 768) and tokens >= 64 * requests and scratch <= RETENTION_CHUNKED_BYTES
 
 
 def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_heads, k_dim, v_dim, most_tokens=None,
@@ -1380,13 +1382,12 @@ def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_he
             and not any(t.data_ptr() % 16 for t in (q, k, state, out))
             and (chunked is None or retention_chunked_takes(N, R, n_heads, k_dim, v_dim))):
         chunk_lib = _lib("retention_chunked", v)
-        chunks = chunk_lib.tnx_retention_chunks(c_int(N), c_int(R))
-        adds = torch.empty(chunks * n_heads * v_dim * k_dim, dtype=torch.float32, device=q.device)
-        spans = torch.empty(chunks * n_heads, dtype=torch.float32, device=q.device)
+        states = (N // 64 + R) * n_heads * v_dim * k_dim     # one of every chunk and head, and behind them its decays
+        adds = torch.empty(states + states // (v_dim * k_dim), dtype=torch.float32, device=q.device)
         _check(chunk_lib.tnx_retention_chunked(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                                _p(state_slots), _p(out), c_int(N), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
-                                               c_int(_is_h16(v)), _p(decay_tok), _p(kscale_tok), c_int(qk_heads), _p(adds), _p(spans),
-                                               _stream()), "retention_scan")
+                                               c_int(_is_h16(v)), _p(decay_tok), _p(kscale_tok), c_int(qk_heads), _p(adds),
+                                               c_void_p(adds.data_ptr() + 4 * states), _stream()), "retention_scan")
         return
     _check(lib.tnx_retention_scan(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                   _p(state_slots), _p(out), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
