@@ -463,24 +463,43 @@ def test_attention_simt(n_heads, n_kv, d, dtype, window):
     assert rel_err(out, case.want(scale, window)) <= (1e-5 if dtype == torch.float32 else 1e-2)
 
 
-@pytest.mark.parametrize("n_heads,n_kv,d", [(32, 32, 20), (20, 5, 64), (17, 17, 100), (16, 2, 128), (16, 16, 144)])
+def exact_attention(q, k, v, scale, first_pos, window=0, keep_first=0, bias=None, sink=None):
+    """q [Tq, n_heads, d] at positions first_pos.., k/v [Tk, n_kv, d] -> [Tq, n_heads, d] in 64-bit, with a window, first keys kept
+    beside it, a distance bias and a sink."""
+    rep = q.shape[1] // k.shape[1]
+    q, k, v = (x.double().transpose(0, 1) for x in (q, k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1)))
+    i, j = torch.arange(q.shape[1])[:, None] + first_pos, torch.arange(k.shape[1])[None, :]
+    s = (q @ k.transpose(1, 2)) * scale
+    if bias is not None:
+        s = s - bias[0].cpu().double()[:, None, None] * torch.log1p(bias[1].cpu().double()[:, None, None] * (i - j).clamp(min=0))
+    seen = (j <= i) & ((j > i - window) | (j < keep_first) if window else True)
+    s = s.masked_fill(~seen, float("-inf"))
+    if sink is not None:
+        s = torch.cat([torch.full_like(s[..., :1], sink), s], -1)
+    p = torch.softmax(s, -1)
+    return (p[..., p.shape[-1] - v.shape[1]:] @ v).transpose(0, 1)
+
+
+@pytest.mark.parametrize("n_heads,n_kv,d", [(32, 32, 20), (20, 5, 64), (20, 20, 100), (24, 3, 128), (16, 16, 144)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("options", [{}, {"sink": 0.5, "bias": True}, {"window": 37, "keep_first": 5}])
+@pytest.mark.parametrize("options", [{}, {"sink": 0.5, "bias": True}, {"window": 37, "keep_first": 5}, {"window": 37, "sink": -0.3, "bias": True}])
 def test_attention_simt_portions_and_rows_agree(n_heads, n_kv, d, dtype, options):
-    """Portions in tiles (edges inside a tile, several requests in one, rows alone beside them), row by row, and with one
-    warp a row (a head size without the staged kernels): the same bits where two of them take a call, and the plain result."""
+    """Portions in tiles (edges inside a tile, several requests in one, rows alone beside them; not behind a window), row by row,
+    and with one warp a row (a cache off the staged kernels' boundary): the same bits, and the 64-bit result."""
     case = PagedCase([(0, 33), (17, 1), (40, 2), (100, 64), (3, 1), (130, 1), (0, 1), (61, 5)], n_heads, n_kv, d, dtype, seed=d)
+    assert d > 128 or case.N * n_heads >= 2048           # from there on portions go in tiles
     kw = dict(options)
     if kw.pop("bias", False):
         g = torch.Generator().manual_seed(1)
         kw["bias"] = (torch.rand(n_heads, generator=g).to(DEV), torch.rand(n_heads, generator=g).to(DEV))
     scale = 1.0 / math.sqrt(d)
-    outs = [torch.zeros(case.N, n_heads * d, dtype=dtype, device=DEV) for _ in range(2)]
-    for out, portions in zip(outs, (True, False)):
-        ops().attention_simt(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, n_heads, scale, portions=portions, **kw)
-    assert torch.equal(outs[0], outs[1])
-    if not options:
-        assert rel_err(outs[0], case.want(scale, None)) <= (1e-5 if dtype == torch.float32 else 1e-2)
+    odd = torch.empty(case.cache.numel() + 1, dtype=dtype, device=DEV)[1:].view(case.cache.shape).copy_(case.cache)
+    outs = [torch.zeros(case.N, n_heads * d, dtype=dtype, device=DEV) for _ in range(3)]
+    for out, cache, portions in zip(outs, (case.cache, case.cache, odd), (True, False, True)):
+        ops().attention_simt(case.q_flat, cache, case.bt, case.tok_req, case.positions, out, n_heads, scale, portions=portions, **kw)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    want = torch.cat([exact_attention(q, k, v, scale, c, **kw).reshape(len(q), -1) for (c, _), q, k, v in zip(case.lens, case.q, case.k, case.v)])
+    assert rel_err(outs[0], want.to(DEV)) <= (1e-5 if dtype == torch.float32 else 1e-2)
 
 
 @pytest.mark.parametrize("n_heads,n_kv,d", ATT_SHAPES)
