@@ -609,14 +609,52 @@ def test_attention_decode_grouped_keeps_the_probabilities(n_heads, n_kv, d, dtyp
     assert bool(((out.double() - want).abs() <= step * want.abs() + 2.0 ** -12 * step * want.abs().max() + 2.0 ** -24).all())
 
 
-def test_attention_decode_grouped_keeps_an_infinite_value():
-    """An infinite value makes its dim infinite, not undefined, whatever its key's probability is split into."""
-    case = PagedCase([(40, 1), (3, 1)], 8, 2, 128, torch.float16, seed=4, plant=False)
-    case.cache[case.bt[0, 1].long(), 1, 1, 3, 5] = float("inf")            # position 19 of the first request, head group 1
-    out = torch.zeros(2, 8 * 128, dtype=torch.float16, device=DEV)
-    ops().attention_decode(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, 8, 0.09, max_kv_len=41, grouped=True)
-    o = out.view(2, 8, 128)
-    assert bool((o[0, 4:, 5] == float("inf")).all()) and int(torch.isfinite(o).logical_not().sum()) == 4
+def _dominated(dtype, peak, n_heads=8, n_kv=2, d=128, ctx=700, seed=4):
+    """One request whose first key is `peak` above the rest in score for every query head and has the value zero; the others'
+    are large, so that float16 has steps enough for what is left of them."""
+    case = PagedCase([(ctx - 1, 1)], n_heads, n_kv, d, dtype, seed=seed, plant=False)
+    case.q[0][:] = case.q[0].view(1, n_kv, -1, d)[:, :, :1].expand(1, n_kv, n_heads // n_kv, d).reshape(1, n_heads, d)
+    case.k[0].mul_(0.02)
+    q = case.q[0].float().view(n_kv, -1, d)[:, 0]
+    case.k[0][0] = (q * (peak / (0.09 * (q * q).sum(-1, keepdim=True)))).to(dtype)
+    case.v[0].mul_(1024.0)
+    case.v[0][0] = 0
+    case.cache[case.bt[0, 0].long(), 0, :, 0] = case.k[0][0].to(DEV)
+    case.cache[case.bt[0, 0].long(), 1, :, 0] = 0
+    for t in range(1, ctx):
+        case.cache[case.bt[0, t // 16].long(), 0, :, t % 16] = case.k[0][t].to(DEV)
+        case.cache[case.bt[0, t // 16].long(), 1, :, t % 16] = case.v[0][t].to(DEV)
+    return case, case.q[0].reshape(1, -1).to(DEV)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("peak", [4.0, 8.0, 12.0, 16.0])
+@pytest.mark.parametrize("n_splits,warps", [(1, 12), (3, 4), (None, None)])
+def test_attention_decode_grouped_keeps_small_probabilities(dtype, peak, n_splits, warps):
+    """A first key that takes nearly all of the sum and has the value zero: the output is made of the others' probabilities, which
+    stay exact to their own size (up to 2^-23 here): the 64-bit result rounded once, and 2^-18 of the
+    largest for the exponentials, whose arguments of up to 16 are rounded to 2^-20."""
+    case, q = _dominated(dtype, peak)
+    out = torch.zeros_like(q)
+    ops().attention_decode(q, case.cache, case.bt, case.tok_req, case.positions, out, 8, 0.09, max_kv_len=700, n_splits=n_splits,
+                           warps=warps, grouped=True)
+    want = exact_attention(case.q[0], case.k[0], case.v[0], 0.09, 699).reshape(1, -1).to(DEV)
+    step = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)                 # half a unit in the last place, relative
+    assert bool(((out.double() - want).abs() <= step * want.abs() + 2.0 ** -25 + 2.0 ** -18 * want.abs().max()).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("peak", [0.0, 6.0, 11.0, 12.5, 17.0, 40.0])
+@pytest.mark.parametrize("at", [3, 19, 600])
+def test_attention_decode_grouped_keeps_an_infinite_value(dtype, peak, at):
+    """An infinite value makes its dim infinite, not undefined, whatever its key's probability is split into: beside the largest
+    key and pages away from it, from 1/700 to 2^-57 of the sum."""
+    case, q = _dominated(dtype, peak)
+    case.cache[case.bt[0, at // 16].long(), 1, 1, at % 16, 5] = float("inf")
+    out = torch.zeros_like(q)
+    ops().attention_decode(q, case.cache, case.bt, case.tok_req, case.positions, out, 8, 0.09, max_kv_len=700, grouped=True)
+    o = out.view(8, 128)
+    assert bool((o[4:, 5] == float("inf")).all()) and int(torch.isfinite(o).logical_not().sum()) == 4
 
 
 def test_attention_decode_row_list():

@@ -13,12 +13,19 @@
 //   softmax  a lane holds two keys of two heads; the maximum runs over eight lanes
 //   values   O^T [16 dims x 8 heads] += V^T P^T: a lane's 16-byte pieces of four value rows, two rows' halves merged by a
 //            byte permutation, are the 16-row operand; P is turned by movmatrix.
-// A probability enters the products as a sum of 16-bit numbers, two in float16 and three in bfloat16 to within 2^-20 and 2^-21
-// of itself (the exponential's own error), with 32-bit sums; the denominator sums it in 32-bit.  The leading terms
-// are cut below p so that the last one stays positive: an infinite value stays infinite (infinity x 0 has no value).
-// Measured, pages beyond the second-level cache, us a call (at the copy rate; one block a head): 48 rows of 32 heads on 8 over
-// 950 to 1,900 tokens 58 (45; 174), 64 rows over 2,048 102 (82; 294), 8 rows 19 (10; 47), one row 8.8 (1.3; 11.7); 64 rows
-// of 16 heads on one 26 (10; 145).  With as many key/value heads as heads: 80 dims, 8 rows of 32 heads 26 (13; 34).
+// A page's probabilities are formed against the page's own largest score, and its products, which start from zero, are added
+// to the running sums times exp(page's maximum - running maximum) by ordinary 32-bit multiply-adds: the tensor cores cut the
+// sums they form where those round, a bias that adds up along a chain of pages.  (The scores likewise, two 16-dim steps at a
+// time.)  A probability enters the products as a sum of 16-bit numbers cut towards zero and a rounded last one: three in bfloat16,
+// to within 2^-22 of itself, and two in float16, to within 2^-21 of itself down to 2^-18 of its page's largest and to 2^-39 of
+// the page's largest below (in multiples of 2^-15, which takes float16's smallest number to 2^-39); the denominator sums it in
+// 32-bit.  No term is zero or less: an infinite value stays infinite (infinity x 0 has no value).  Results rounded otherwise
+// than the 64-bit ones are, of float16 results, 48 rows of 32 heads on 8: 1.3 in 1,000 (a block a head: 1.8; with sums chained
+// through the accumulators and unscaled terms 4.6).
+// Measured, pages beyond the second-level cache, us a call in float16 / bfloat16 (with one block a head): 48 rows of 32 heads on
+// 8 over 950 to 1,900 tokens 60 / 63 (165 / 171; 45 would be the copy rate), 64 rows over 1,024 to 2,048 77 / 80 (215 / 227), 8
+// rows of 32 heads on 2 over 950 to 1,900 14.5 / 16.5 (39 / 41); 64 rows of 16 heads on one over 500 to 1,000 18.6 / 19.4 (65 / 68).
+// With as many key/value heads as heads: 80 dims, 8 rows of 32 heads over 700 to 1,400 29 / 31 (33 / 35).
 //
 // Grid (key/value heads x head tiles, rows, splits), 4, 8 or 12 warps; a warp takes every WARPS-th page of the split's range,
 // its next keys and values in flight while it works.  Warps are merged in shared memory.  The splits of a (row, head tile)
@@ -52,32 +59,46 @@ struct GroupedParams {
     h16* cache_w;
 };
 
-__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
 #ifdef TNX_F16
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+#define MMA_KIND "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
 #else
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+#define MMA_KIND "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
 #endif
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm(MMA_KIND "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma_from_zero(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm(MMA_KIND "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+#undef MMA_KIND
 // An 8 x 8 matrix of 16-bit numbers turned: lane (g, c) gives row g, columns 2c and 2c + 1, and receives those of the transpose.
 __device__ __forceinline__ uint32_t turned(uint32_t v) {
     uint32_t r;
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
     return r;
 }
-__device__ __forceinline__ uint32_t pack(float a, float b) {
-    const h16x2 v = floats_to_h16x2(a, b);
-    return *(const uint32_t*)&v;
+
+// Two numbers cut to 16 bits: towards zero, so that what is left has no other sign.
+__device__ __forceinline__ h16x2 cut(float a, float b) {
+    uint32_t v;
+#ifdef TNX_F16
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(b), "f"(a));
+#else
+    asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(b), "f"(a));
+#endif
+    return *(const h16x2*)&v;
 }
 
 #ifdef TNX_F16
 constexpr int TERMS = 2;
-constexpr float BELOW = 1.f - 0x1p-10f;      // times this, rounding to 16 bits stays below the number itself
+constexpr float SCALE = 0x1p15f;             // of the probabilities in the products: float16 has no small numbers to spare
+constexpr float LEAST = 0x1p-24f;            // the smallest positive number of the 16-bit type
 #else
 constexpr int TERMS = 3;
-constexpr float BELOW = 1.f - 0x1p-7f;
+constexpr float SCALE = 1.f;
+constexpr float LEAST = 0x1p-133f;
 #endif
 
 __device__ __forceinline__ uint32_t shared_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -116,8 +137,9 @@ attention_decode_grouped_kernel(const GroupedParams p) {
     const int pos = p.positions[row];
     const int* bt = p.block_tables + (size_t)req * p.bt_stride;
 
-    // the queries as the 8-column operand: lane (g, c) holds head g's dims in the order its key pieces come in
-    uint32_t q[NT][STEPS][2];
+    // the queries as the 8-column operand: lane (g, c) holds head g's dims in the order its key pieces come in, kept where the
+    // warp's results go in the end (in registers they spilled others: 88 us for the first measurement above)
+    uint2* const qs = (uint2*)(sm_o + (size_t)warp * HEADS * PITCH) + lane;
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
         const bool has = t * 8 + g < n_mine;
@@ -125,11 +147,11 @@ attention_decode_grouped_kernel(const GroupedParams p) {
 #pragma unroll
         for (int i = 0; i < N32; ++i) {
             const uint4 v = has ? *(const uint4*)(src + 32 * i + 8 * c) : make_uint4(0, 0, 0, 0);
-            q[t][2 * i][0] = v.x; q[t][2 * i][1] = v.y; q[t][2 * i + 1][0] = v.z; q[t][2 * i + 1][1] = v.w;
+            qs[(t * STEPS + 2 * i) * 32] = make_uint2(v.x, v.y); qs[(t * STEPS + 2 * i + 1) * 32] = make_uint2(v.z, v.w);
         }
         if constexpr (D % 32 != 0) {
             const uint2 v = has ? *(const uint2*)(src + 32 * N32 + 4 * c) : make_uint2(0, 0);
-            q[t][STEPS - 1][0] = v.x; q[t][STEPS - 1][1] = v.y;
+            qs[(t * STEPS + STEPS - 1) * 32] = v;
         }
     }
 
@@ -230,17 +252,22 @@ attention_decode_grouped_kernel(const GroupedParams p) {
         float s[NT][4];                                  // [0], [1]: key g of heads 2c, 2c + 1;  [2], [3]: key g + 8
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
+            float x[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
+            for (int k = 0; k < STEPS; ++k) {
+                const uint2 q = qs[(n * STEPS + k) * 32];
+                if (k % 2 == 0) mma_from_zero(x, kr[0][2 * k], kr[1][2 * k], kr[0][2 * k + 1], kr[1][2 * k + 1], q.x, q.y);
+                else mma(x, kr[0][2 * k], kr[1][2 * k], kr[0][2 * k + 1], kr[1][2 * k + 1], q.x, q.y);
+                if (k % 2 == 0 && k + 1 < STEPS) continue;
 #pragma unroll
-            for (int k = 0; k < STEPS; ++k)
-                mma(s[n], kr[0][2 * k], kr[1][2 * k], kr[0][2 * k + 1], kr[1][2 * k + 1], q[n][k][0], q[n][k][1]);
+                for (int i = 0; i < 4; ++i) s[n][i] = k >= 2 ? s[n][i] + x[i] : x[i];
+            }
         }
         if (more) load_keys(t + 1, next_page);
         const int j0 = first_of(t);
         const bool paged = t < my_pages;
         const bool see0 = paged ? seen(j0 + g) : g == 0, see1 = paged && seen(j0 + g + 8);
-        float top[NT][2];
+        float here[NT][2], top[NT][2];                   // the page's largest score, the largest so far
         bool grew = false;
 #pragma unroll
         for (int n = 0; n < NT; ++n)
@@ -257,6 +284,7 @@ attention_decode_grouped_kernel(const GroupedParams p) {
                 v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));
                 v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
                 v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+                here[n][x] = v;
                 top[n][x] = fmaxf(v, m[n][x]);
                 grew = grew || top[n][x] > m[n][x];
             }
@@ -272,31 +300,30 @@ attention_decode_grouped_kernel(const GroupedParams p) {
                     for (int k = 0; k < STEPS; ++k) { acc[n][k][x] *= corr; acc[n][k][2 + x] *= corr; }
                 }
         }
-        // the probabilities, split into 16-bit terms and turned: lane (g, c) gets head g's keys 2c, 2c + 1 (and + 8)
+        // the probabilities against the page's maximum, split into 16-bit terms and turned: lane (g, c) gets head g's keys
+        // 2c, 2c + 1 (and + 8).  times: the page's share of the sums
         uint32_t pt[NT][TERMS][2];
+        float times[NT][2];
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
             float e[4];
 #pragma unroll
+            for (int x = 0; x < 2; ++x) times[n][x] = here[n][x] == -INFINITY ? 0.f : __expf(here[n][x] - m[n][x]);
+#pragma unroll
             for (int i = 0; i < 4; ++i) {
-                e[i] = s[n][i] == -INFINITY ? 0.f : __expf(s[n][i] - m[n][i & 1]);
-                l[n][i & 1] += e[i];
+                e[i] = s[n][i] == -INFINITY ? 0.f : __expf(s[n][i] - here[n][i & 1]);
+                l[n][i & 1] = fmaf(e[i], times[n][i & 1], l[n][i & 1]);
+                e[i] *= SCALE;
             }
 #pragma unroll
             for (int k = 0; k < TERMS; ++k)
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     float &a = e[2 * r], &b = e[2 * r + 1];
-                    uint32_t v;
-                    if (k + 1 < TERMS) {
-                        const h16x2 cut = floats_to_h16x2(a * BELOW, b * BELOW);
-                        const float2 f = h16x2_to_float2(cut);
-                        a -= f.x; b -= f.y;
-                        v = *(const uint32_t*)&cut;
-                    } else {
-                        v = pack(a, b);
-                    }
-                    pt[n][k][r] = turned(v);
+                    const float ta = fmaxf(a, LEAST), tb = fmaxf(b, LEAST);
+                    const h16x2 term = k + 1 < TERMS ? cut(ta, tb) : floats_to_h16x2(ta, tb);
+                    if (k + 1 < TERMS) { const float2 f = h16x2_to_float2(term); a -= f.x; b -= f.y; }
+                    pt[n][k][r] = turned(*(const uint32_t*)&term);
                 }
         }
 #pragma unroll
@@ -304,9 +331,14 @@ attention_decode_grouped_kernel(const GroupedParams p) {
             const uint32_t a0 = __byte_perm(vr[0][k], vr[1][k], 0x5410), a1 = __byte_perm(vr[0][k], vr[1][k], 0x7632);
             const uint32_t a2 = __byte_perm(vr[2][k], vr[3][k], 0x5410), a3 = __byte_perm(vr[2][k], vr[3][k], 0x7632);
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < NT; ++n) {
+                float x[4];                              // small terms first
+                mma_from_zero(x, a0, a1, a2, a3, pt[n][TERMS - 1][0], pt[n][TERMS - 1][1]);
 #pragma unroll
-                for (int x = 0; x < TERMS; ++x) mma(acc[n][k], a0, a1, a2, a3, pt[n][x][0], pt[n][x][1]);
+                for (int y = TERMS - 2; y >= 0; --y) mma(x, a0, a1, a2, a3, pt[n][y][0], pt[n][y][1]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[n][k][i] = fmaf(x[i], times[n][i & 1], acc[n][k][i]);
+            }
         }
         if (more) {
             load_values(t + 1, next_page);
@@ -325,6 +357,7 @@ attention_decode_grouped_kernel(const GroupedParams p) {
             ((uint4*)dst)[piece] = ((const uint4*)src)[piece];
         }
     }
+    __syncwarp();
     // the warps' states into shared memory: tile k of the output holds dims d_k (rows g) and d_k + 1 (rows g + 8)
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
@@ -367,7 +400,7 @@ attention_decode_grouped_kernel(const GroupedParams p) {
             o += f == 0.f ? 0.f : sm_o[(w * HEADS + x) * PITCH + dim] * f;
         }
         if (p.n_splits == 1) {
-            p.out[(size_t)row * p.out_stride + (size_t)(h0 + x) * D + dim] = float_to_h16(o / block_l[x]);
+            p.out[(size_t)row * p.out_stride + (size_t)(h0 + x) * D + dim] = float_to_h16(o * (1.f / SCALE) / block_l[x]);
         } else {
             sm_o[x * PITCH + dim] = o;                   // only this thread reads the warps' numbers of this place
         }
@@ -390,7 +423,7 @@ attention_decode_grouped_kernel(const GroupedParams p) {
 #pragma unroll
         for (int s = 0; s < 8; ++s)
             if (ms[s] != -INFINITY) { const float f = __expf(ms[s] - M); L += ls[s] * f; o += os[s] * f; }
-        p.out[(size_t)row * p.out_stride + (size_t)(h0 + x) * D + dim] = float_to_h16(o / L);
+        p.out[(size_t)row * p.out_stride + (size_t)(h0 + x) * D + dim] = float_to_h16(o * (1.f / SCALE) / L);
     }
     cluster_arrive();                                    // ... and stays until all have read it
     cluster_wait();
@@ -419,14 +452,14 @@ int launch_tiles(int nt, int warps, dim3 grid, cudaStream_t stream, const Groupe
     return nt == 1 ? launch<D, 1>(warps, grid, stream, p) : launch<D, 2>(warps, grid, stream, p);
 }
 
-}  // namespace
-
 // Query heads a block takes (8 or 16), 0 where the kernel does not take these sizes.
-TNX_EXPORT int tnx_attention_decode_grouped_heads(int n_heads, int n_kv_heads, int head_dim) {
+int heads_of_a_block(int n_heads, int n_kv_heads, int head_dim) {
     if (n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads) return 0;
     if (head_dim != 64 && head_dim != 80 && head_dim != 96 && head_dim != 112 && head_dim != 128) return 0;
     return n_heads / n_kv_heads <= 8 ? 8 : 16;
 }
+
+}  // namespace
 
 // Arguments as tnx_attention_decode_append; n_splits 1 .. 8; warps a block: 4, or all that an SM holds (12 with up to 8 query
 // heads a key/value head, else 8).
@@ -437,7 +470,7 @@ TNX_EXPORT int tnx_attention_decode_grouped(const void* q, int q_stride, void* c
                                             const void* k_new, const void* v_new, int kv_stride, int warps, int keep_first, const float* bias_mul, const float* bias_rate,
                                             int has_sink, float sink_score, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    const int heads = tnx_attention_decode_grouped_heads(n_heads, n_kv_heads, head_dim);
+    const int heads = heads_of_a_block(n_heads, n_kv_heads, head_dim);
     if (!heads || page_size != PAGE || q_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)cache & 15)) return TNX_ERR_UNSUPPORTED;
     if ((k_new == nullptr) != (v_new == nullptr)) return TNX_ERR_BAD_ARG;
     if (k_new && (kv_stride % 8 || (((uintptr_t)k_new | (uintptr_t)v_new) & 15))) return TNX_ERR_UNSUPPORTED;

@@ -646,21 +646,25 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
 
     With shared key/value heads always, but for the shortest steps (16 heads on one, 100 tokens: 4.6 us with a block a head,
     6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1).  Without, where the other kernel's lanes idle (head sizes that
-    are no power of two: 80 dims, 8 rows of 32 heads over up to 1,400 tokens 34 and 26 us, 64 rows 164 and 135), with
-    few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 13.8 and 10.7 us, of 12 heads of 64 over 400 7.0
-    and 5.0; 8 rows of 32 heads of 128 35 and 31) and with many long ones (64 rows 172 and 166) if its three blocks an SM leave no
-    more places of the last round empty than the other's four (32 rows of 40 heads up to 700 tokens 38 and 41; of 32
-    heads 49 and 51, with 18 of the rows in use 27 and 30); between those a block a head is as fast or faster (16 rows 53
-    and 56 us; heads of 64, 8 rows over 1,000 tokens 16 and 21)."""
+    are no power of two: 80 dims, 8 rows of 32 heads over up to 1,400 tokens 33 and 29 us, 64 rows 169 and 144) and, for the
+    others, with few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 14.4 and 12.4 us, of 12 heads of 64 over
+    400 7.0 and 5.0); with more rows a block a head is as fast or faster (8 rows of 32 heads of 128 over 1,400 tokens 34.9 and
+    35.2, 64 179.7 and 179.6; heads of 64, 8 rows 20 and 27)."""
     blocks = rows * n_heads
     if max_pages <= 12 and blocks <= sms:
         return False
     if n_heads != n_kv:
         return True
-    if head_dim == 64 or max_pages < 32:
+    if head_dim in (64, 128) or max_pages < 32:
         return max_pages > (16 if head_dim == 64 else 12) and 2 * blocks <= sms
-    rounds = lambda per: -(-blocks // (per * sms)) * per
-    return head_dim != 128 or blocks <= 2 * sms or (blocks > 4 * sms and rounds(3) <= rounds(4))
+    return True
+
+
+def grouped_decode_heads(n_heads: int, n_kv: int, head_dim: int) -> int:
+    """Query heads a block of the grouped decode attention takes (8 or 16), 0 where it does not take these sizes."""
+    if n_kv <= 0 or n_heads % n_kv or head_dim not in (64, 80, 96, 112, 128):
+        return 0
+    return 8 if n_heads // n_kv <= 8 else 16
 
 
 def grouped_decode_plan(blocks: int, sms: int, heads_per_block: int, max_pages: int):
@@ -699,7 +703,6 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
     tokens, which the kernel then writes into their pages itself (no kv_append before it).
     n_splits (with warps, 4 or 8 a block) forces a plan: a test hook.  grouped: with several query heads a key/value
     head a block takes up to 16 of them and reads the head's pages once (True / False: a test hook)."""
-    lib = _lib("attention_decode", cache, q, out)
     _need(cache, "cache", _H16, 5)
     N, width, q_stride = _rows_2d(q, "q")
     No, wo, out_stride = _rows_2d(out, "out")
@@ -720,8 +723,8 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
     # a forced plan is the other kernel's unless `grouped` asks for this one.
     heads_per_block = 0
     if grouped or (grouped is None and n_splits is None and grouped_decode_takes(R, n_heads, n_kv, d, st["sms"], max_pages)):
-        group_lib = _lib("attention_decode_grouped", cache, q, out)
-        heads_per_block = group_lib.tnx_attention_decode_grouped_heads(c_int(n_heads), c_int(n_kv), c_int(d))
+        heads_per_block = grouped_decode_heads(n_heads, n_kv, d)
+    lib = _lib("attention_decode_grouped" if heads_per_block else "attention_decode", cache, q, out)
     if heads_per_block:
         tiles = n_kv * -(-(n_heads // n_kv) // heads_per_block)
         if n_splits is None:
@@ -756,7 +759,7 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
         if v_new.stride(0) != kv_stride:
             raise KernelError("new k and v must have the same row pitch")
     if heads_per_block:
-        _check(group_lib.tnx_attention_decode_grouped(
+        _check(lib.tnx_attention_decode_grouped(
             _p(q), c_int(q_stride), _p(cache), _p(block_tables), c_int(block_tables.stride(0)),
             _p(rows), _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(R),
             c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask_rule(window, chunk)), c_float(scale),
