@@ -182,9 +182,10 @@ def test_queries_and_keys_turn_in_pieces_of_four(H, dk, rot, dtype):
 @pytest.mark.parametrize("gates", [False, True])
 def test_retention_in_chunks_equals_the_recurrence(H, Hq, dk, dv, dtype, gates):
     """Chunks whole and with remainders of 1, 16, 17 and 63 tokens, several requests (one of them padding) with states of their
-    own, fixed and per-token decays (one zero, two negative, strong ones beside weak ones) and key scales.  A product keeps
-    22 bits and more (2^-22 left out, 2^-23 a cut sum), so a result of up to 128 + 64 + 64 of them stays within 2^-20 of the
-    size of its terms, which is at most 16 times the results' root mean square (256 terms of random sign)."""
+    own, a decay per head; and, which stays with the token-by-token kernel, as do shared queries and keys, per-token decays (one
+    zero, two negative, strong ones beside weak ones) and key scales.  A product keeps 24 bits and loses 2^-23 in a cut sum, so
+    a result of up to 128 + 64 + 64 of them stays within 2^-20 of the size of its terms, which is at most 16 times the results'
+    root mean square (256 terms of random sign)."""
     from transformers_neuronx_b200.kernels import ops
     g = torch.Generator().manual_seed(H + dk)
     lens, slots = [64, 1, 0, 145, 127, 16], [3, 0, 1, -1, 2, 5]
@@ -214,6 +215,31 @@ def test_retention_in_chunks_equals_the_recurrence(H, Hq, dk, dv, dtype, gates):
     for got, ref in ((out.cpu().double(), want), (state.cpu().double(), states)):
         assert float((got - ref).abs().max()) <= 2.0 ** -20 * 16 * float(ref.pow(2).mean().sqrt())
     assert torch.equal(state[1].cpu(), state0[1]) and torch.equal(state[4].cpu(), state0[4])      # a request without rows; nobody's slot
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dk, dv", [(128, 128), (64, 64)])
+def test_retention_in_chunks_is_no_further_from_64_bit(dtype, dk, dv):
+    """Per head, outputs and state, at decays from the one that the mixer takes on to one that hardly forgets: the error against
+    64-bit is at most the token-by-token scan's (a tenth more for the draw)."""
+    from transformers_neuronx_b200.kernels import ops
+    from transformers_neuronx_b200.parts.retention import Retention
+    decay = torch.tensor([Retention.CHUNKS_FROM_DECAY, 0.94, 0.96875, 0.98, 0.99, 0.999])
+    T, H = 700, len(decay)
+    g = torch.Generator().manual_seed(dk)
+    q, k = torch.randn(T, H * dk, generator=g), torch.randn(T, H * dk, generator=g) * dk ** -0.5
+    v, state0 = torch.randn(T, H * dv, generator=g).to(dtype), torch.randn(1, H, dv, dk, generator=g)
+    S, want = state0[0].double(), torch.zeros(T, H, dv, dtype=torch.float64)
+    for t in range(T):
+        S = S * decay.double()[:, None, None] + v[t].double().view(H, dv, 1) * k[t].double().view(H, 1, dk)
+        want[t] = (S @ q[t].double().view(H, dk, 1))[..., 0]
+    errors = []
+    for chunked in (False, None):
+        state, out = state0.to(DEV), torch.zeros(T, H * dv, device=DEV)
+        ops.retention_scan(q.to(DEV), k.to(DEV), v.to(DEV), decay.to(DEV), state, _i32([0]), _i32([T]), _i32([0]), out, H, dk, dv, chunked=chunked)
+        o, s = out.view(T, H, dv).cpu().double(), state[0].cpu().double()
+        errors.append(torch.cat([(o - want).norm(dim=(0, 2)) / want.norm(dim=(0, 2)), (s - S).norm(dim=(1, 2)) / S.norm(dim=(1, 2))]))
+    assert bool((errors[1] <= 1.1 * errors[0]).all()), errors
 
 
 @pytest.mark.parametrize("H, dk, dv, rot", [(3, 20, 24, 12), (2, 128, 64, 128), (1, 256, 16, 0), (2, 8, 40, 8)])

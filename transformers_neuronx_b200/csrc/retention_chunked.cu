@@ -1,23 +1,23 @@
 // The recurrence of retention.cu over portions of prompts, in chunks of 64 tokens on the tensor cores:
-//     S_t = a_t S_(t-1) + s_t k_t v_t^T,   o_t = S_t^T q_t        (a_t: a decay of the head or of the token, s_t: a key scale)
-// With L_i = a_1 ... a_i inside a chunk and S the state before it,
-//     o_i = L_i S^T q_i + sum_{j <= i} (L_i / L_j) s_j (q_i . k_j) v_j,      S' = L_64 S + sum_j (L_64 / L_j) s_j k_j v_j^T
+//     S_t = a S_(t-1) + k_t v_t^T,   o_t = S_t^T q_t        (a: the head's decay)
+// With tokens numbered from 0 inside a chunk of n and S the state before it,
+//     o_i = a^(i+1) S^T q_i + sum_{j <= i} a^(i-j) (q_i . k_j) v_j,      S' = a^n S + sum_j a^(n-1-j) k_j v_j^T
 // so that what a chunk adds to the state, and its outputs once its first state is known, are products of matrices; only the
 // states themselves are a chain, of one multiply-add an element and chunk.  Three kernels:
 //   chunk_states    a block per (chunk, head): what the chunk adds to the state, [v_dim x k_dim], into scratch memory
 //   chunk_prefix    a thread per four state elements walks the request's chunks: leaves the state before each in place
 //   chunk_outputs   a block per (chunk, head, half of the value dims): scores q_i . k_j times the decays between, the outputs
 // The token-by-token scan is a chain of as many links as there are tokens, with one block of four warps an SM.  Measured, 16
-// heads of 128 x 128, 16-bit values: 2,048 tokens of one request 332 -> 119 us (states 29, prefix 13, outputs 75), 512 tokens
-// 88 -> 41, 256 tokens 47 -> 38, 8 requests of 128 99 -> 65; 32 heads 439 -> 232.  What bounds it: chunk_outputs issues an
-// instruction in 29 of 100 cycles, seven warps an SM that wait for one another's products (registers hold no more).
+// heads of 128 x 128, 16-bit values: 2,048 tokens of one request 332 -> 122 us, 512 tokens 88 -> 39, four requests of 512
+// 122; 32 heads 439 -> 243.  What bounds it: chunk_outputs, seven warps an SM that wait for one another's products (registers
+// hold no more).
 //
-// Everything stays 32-bit: a product of 32-bit numbers is three tensor-core products of their leading and trailing halves
-// (x = hi + lo, each 11 bits wide: hi hi + hi lo + lo hi, 2^-22 of a product left out), a 16-bit value is a leading half by
-// itself, and the sums are 32-bit.  Ratios of decays come from sums of their logarithms in 64-bit, so they are exact to a
-// rounding however far apart the two tokens are.  Relative error against 64-bit, here and token by token, 2,048 tokens, decays
-// of 1 - 2^-5 to 1 - 2^-11.6: outputs 3.2e-7 and 5.0e-7, state 3.4e-7 and 6.0e-7.  It grows less with the number of tokens
-// that a state remembers and starts higher: equal at a decay of 0.99 (1.9e-7), 1.8e-7 and 1.3e-7 at 0.97.
+// Everything stays 32-bit: a 32-bit number is the sum of three bfloat16 numbers, all its 24 bits, a product of two of them six
+// products of the terms (what is left out is 2^-25 of it), and the sums are 32-bit.  A power of the decay is formed in 64-bit
+// and rounded once.  Relative error against 64-bit, token by token and here, 1,024 tokens (with operands of two times 11 bits
+// and powers from 32-bit logarithms): outputs at a decay of 0.5 8.8e-8 and 8.6e-8 (1.5e-7), at 0.9 1.0e-7 and 8.9e-8 (1.7e-7),
+// at 0.97 1.3e-7 and 9.4e-8 (1.9e-7), at 0.99 2.0e-7 and 1.0e-7 (1.9e-7), at 0.9997 4.7e-7 and 1.2e-7 (2.3e-7); the state at
+// 0.5 4.0e-8 and 6.0e-8, at 0.9 6.4e-8 and 6.3e-8, at 0.97 1.1e-7 and 6.5e-8, at 0.9997 5.8e-7 and 1.1e-7.
 //
 // A value that is not finite leaves the outputs of its request undefined from its chunk of 16 tokens on.
 #include "common.cuh"
@@ -27,17 +27,15 @@ namespace {
 constexpr int CHUNK = 64, THREADS = 256;
 
 struct ChunkParams {
-    const float* q; const float* k;          // [tokens, qk_heads * DK]
+    const float* q; const float* k;          // [tokens, H * DK]
     const void* v; int v_ld;                 // [tokens, H * DV], 16-bit or 32-bit
-    const float* decay;                      // [H] or null
-    const float* decay_tok;                  // [tokens, H] or null
-    const float* kscale_tok;                 // [tokens, H] or null
+    const float* decay;                      // [H]
     float* state;                            // [slots, H, DV, DK]
     const int* q_start; const int* q_len; const int* state_slots;
     float* out;                              // [tokens, H * DV]
     float* adds;                             // [chunks, H, DV, DK]: what a chunk adds, then the state before it
-    float* spans;                            // [chunks, H]: L_64 of the chunk
-    int n_requests, H, qk_heads;
+    float* spans;                            // [chunks, H]: the chunk's decay, a to its number of tokens
+    int n_requests, H;
 };
 
 // Chunk `place` of all requests' chunks laid end to end: its request (-1: none), its first token within it.
@@ -64,77 +62,84 @@ __device__ __forceinline__ Where find_chunk(const ChunkParams& p, int place) {  
     return {-1, 0};
 }
 
-// x = hi + lo: hi is x rounded to the 11 bits of a tensor-core operand, lo the rest cut to as many.  Bit operations: the
-// conversion instruction runs at a quarter of their rate.
-struct Halves { uint32_t hi, lo; };
-__device__ __forceinline__ Halves halves(float x) {
-    Halves h;
-    h.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    h.lo = __float_as_uint(x - __uint_as_float(h.hi)) & 0xffffe000u;      // a NaN becomes a zero and a NaN
-    return h;
-}
-struct HalvesA { Halves x0, x1, x2, x3; };
-__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_from_zero(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-__device__ __forceinline__ void add(float (&sums)[4], const float (&x)[4]) {
+// Two numbers as pairs of bfloat16 numbers, one pair a term: eight bits each, so that three terms are a 32-bit number exactly,
+// two a float16 number and one a bfloat16 number.
+template <int TERMS> __device__ __forceinline__ void split(float x, float y, uint32_t (&out)[TERMS]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) sums[i] += x[i];
-}
-// sums += A B over one step of eight, and over two steps whose B is four neighbouring numbers of a lane.  The tensor cores cut
-// the sums they form where an ordinary addition rounds them, a bias that adds up along a chain of products.  So a product of
-// one or two steps starts from zero, small terms first, and is added to the running sums by ordinary additions (chained through
-// the accumulators, the outputs' error was three times the token-by-token scan's).
-__device__ __forceinline__ void add_one(float (&sums)[4], const HalvesA& a, const Halves& b0, const Halves& b1) {
-    float t[4];
-    mma_from_zero(t, a.x0.lo, a.x1.lo, a.x2.lo, a.x3.lo, b0.hi, b1.hi);
-    mma(t, a.x0.hi, a.x1.hi, a.x2.hi, a.x3.hi, b0.lo, b1.lo);
-    mma(t, a.x0.hi, a.x1.hi, a.x2.hi, a.x3.hi, b0.hi, b1.hi);
-    add(sums, t);
-}
-__device__ __forceinline__ void add_two(float (&sums)[4], const HalvesA& a, const HalvesA& b, float4 with) {
-    const Halves x = halves(with.x), y = halves(with.y), z = halves(with.z), w = halves(with.w);
-    float t[4];
-    mma_from_zero(t, a.x0.lo, a.x1.lo, a.x2.lo, a.x3.lo, x.hi, y.hi);
-    mma(t, a.x0.hi, a.x1.hi, a.x2.hi, a.x3.hi, x.lo, y.lo);
-    mma(t, b.x0.lo, b.x1.lo, b.x2.lo, b.x3.lo, z.hi, w.hi);
-    mma(t, b.x0.hi, b.x1.hi, b.x2.hi, b.x3.hi, z.lo, w.lo);
-    mma(t, a.x0.hi, a.x1.hi, a.x2.hi, a.x3.hi, x.hi, y.hi);
-    mma(t, b.x0.hi, b.x1.hi, b.x2.hi, b.x3.hi, z.hi, w.hi);
-    add(sums, t);
-}
-
-// The chunk's decays: logs[i] = log2 |L_i| in 64-bit, signs[i] = the sign of L_i, scales[i] = s_i (0 from n on).  By one warp.
-// A decay of zero counts as 2^-1100: what lies before it is lost below any 32-bit number.
-__device__ __forceinline__ void chunk_decays(const ChunkParams& p, int h, size_t token0, int n, double* logs, float* signs, float* scales) {
-    const int lane = threadIdx.x & 31;
-    double upto = 0.0;
-    float sign = 1.f;
-#pragma unroll
-    for (int half = 0; half < CHUNK / 32; ++half) {
-        const int i = half * 32 + lane;
-        float a = 1.f, s = 0.f;
-        if (i < n) {
-            a = p.decay_tok ? p.decay_tok[(token0 + i) * p.H + h] : p.decay[h];
-            s = p.kscale_tok ? p.kscale_tok[(token0 + i) * p.H + h] : 1.f;
-        }
-        double x = a == 0.f ? -1100.0 : log2((double)fabsf(a));
-        float sg = a < 0.f ? -1.f : 1.f;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, x, o);
-            const float z = __shfl_up_sync(0xffffffffu, sg, o);
-            if (lane >= o) { x += y; sg *= z; }
-        }
-        logs[i] = upto + x; signs[i] = sign * sg; scales[i] = s;
-        upto += __shfl_sync(0xffffffffu, x, 31);
-        sign *= __shfl_sync(0xffffffffu, sg, 31);
+    for (int i = 0; i < TERMS; ++i) {
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out[i]) : "f"(y), "f"(x));
+        if (i + 1 < TERMS) { x -= __uint_as_float(out[i] << 16); y -= __uint_as_float(out[i] & 0xffff0000u); }
     }
+}
+// Operands of a product over sixteen: a lane has rows g and g + 8 (or column g) at four places, which may be any four as long as
+// both operands agree on them.
+template <int TERMS> struct Rows { uint32_t x[4][TERMS]; };
+template <int TERMS> struct Columns { uint32_t x[2][TERMS]; };
+template <int TERMS> __device__ __forceinline__ Rows<TERMS> rows(float4 a, float4 b) {
+    Rows<TERMS> r;
+    split<TERMS>(a.x, a.y, r.x[0]); split<TERMS>(b.x, b.y, r.x[1]); split<TERMS>(a.z, a.w, r.x[2]); split<TERMS>(b.z, b.w, r.x[3]);
+    return r;
+}
+template <int TERMS> __device__ __forceinline__ Columns<TERMS> columns(float4 a) {
+    Columns<TERMS> c;
+    split<TERMS>(a.x, a.y, c.x[0]); split<TERMS>(a.z, a.w, c.x[1]);
+    return c;
+}
+template <bool FROM_ZERO, int TA, int TB>
+__device__ __forceinline__ void mma(float (&d)[4], const Rows<TA>& a, int i, const Columns<TB>& b, int j) {
+    if constexpr (FROM_ZERO)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a.x[0][i]), "r"(a.x[1][i]), "r"(a.x[2][i]), "r"(a.x[3][i]), "r"(b.x[0][j]), "r"(b.x[1][j]), "f"(0.f));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a.x[0][i]), "r"(a.x[1][i]), "r"(a.x[2][i]), "r"(a.x[3][i]), "r"(b.x[0][j]), "r"(b.x[1][j]));
+}
+// sums += A B over sixteen: the terms' products whose places add up to two, one and none (2^-16, 2^-8 and 1 of the whole; beyond
+// two they are 2^-25 and less) each from zero, then added by ordinary additions, small ones first.  The tensor cores cut the sums
+// they form where an ordinary addition rounds them, a bias that adds up along a chain of products (chained through the
+// accumulators, the outputs' error was three times the token-by-token scan's).
+template <int TA, int TB>
+__device__ __forceinline__ void add_product(float (&sums)[4], const Rows<TA>& a, const Columns<TB>& b) {
+    float lead[4], next[4], last[4];
+    mma<true>(lead, a, 0, b, 0);
+    if constexpr (TB > 1) {
+        mma<true>(next, a, 0, b, 1);
+        if constexpr (TA > 1) mma<false>(next, a, 1, b, 0);
+    } else if constexpr (TA > 1) {
+        mma<true>(next, a, 1, b, 0);
+    }
+    if constexpr (TA > 1 && TB > 1) {
+        mma<true>(last, a, 1, b, 1);
+        if constexpr (TB > 2) mma<false>(last, a, 0, b, 2);
+        if constexpr (TA > 2) mma<false>(last, a, 2, b, 0);
+    } else if constexpr (TA > 2) {
+        mma<true>(last, a, 2, b, 0);
+    } else if constexpr (TB > 2) {
+        mma<true>(last, a, 0, b, 2);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if constexpr (TA > 2 || TB > 2 || (TA > 1 && TB > 1)) next[i] += last[i];
+        if constexpr (TA > 1 || TB > 1) lead[i] += next[i];
+        sums[i] += lead[i];
+    }
+}
+// Terms of a value of the stored type.
+#ifdef TNX_F16
+constexpr int H16_TERMS = 2;
+#else
+constexpr int H16_TERMS = 1;
+#endif
+template <typename T> __host__ __device__ constexpr int terms_of() { return sizeof(T) == 4 ? 3 : H16_TERMS; }
+
+// powers[n] = a^n for n up to CHUNK, formed in 64-bit and rounded once, by the block's first threads (the caller synchronises).
+__device__ __forceinline__ void chunk_decays(float a, float* powers) {
+    if (threadIdx.x > CHUNK) return;
+    double p = 1.0, square = (double)a;
+#pragma unroll
+    for (int bit = 1; bit <= CHUNK; bit <<= 1, square *= square)
+        if ((int)threadIdx.x & bit) p *= square;
+    powers[threadIdx.x] = (float)p;
 }
 
 // Rows [CHUNK] x WIDTH of a matrix into shared memory as floats, rows from n on zero: 32-bit rows by asynchronous copies (the
@@ -167,32 +172,30 @@ __device__ __forceinline__ void stage(float* dst, int pitch, const T* src, size_
 }
 __device__ __forceinline__ void staged() { asm volatile("cp.async.wait_all;" ::: "memory"); __syncthreads(); }
 
-// What the chunk adds to the state: [DV x DK] = V^T (w K), w_j = (L_64 / L_j) s_j, by eight warps of 32 x (DK / WN) each.
-// Rows of 8 more than a multiple of 32 floats: the lanes' reads down four tokens and along eight dims meet no bank twice.
+// What a chunk of n tokens adds to the state: [DV x DK] = V^T (w K), w_j = a^(n - 1 - j), by eight warps of 32 x (DK / WN) each.
+// Rows of 4 more than a multiple of 32 floats: the lanes' reads down every second of eight tokens and along eight dims meet no
+// bank twice.
 template <typename T, int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2)
 chunk_states_kernel(const ChunkParams p) {
-    constexpr int PK = DK + 8, PV = DV + 8, WM = DV / 32, WN = 8 / WM, NT = DK / WN / 8;
+    constexpr int PK = DK + 4, PV = DV + 4, WM = DV / 32, WN = 8 / WM, NT = DK / WN / 8;
     extern __shared__ __align__(16) float sm[];
     float* ks = sm;
     float* vs = ks + CHUNK * PK;
-    __shared__ double logs[CHUNK];
-    __shared__ float signs[CHUNK], scales[CHUNK], w[CHUNK];
+    __shared__ float powers[CHUNK + 1];
     pdl_launch_dependents();
     pdl_wait();
-    const int place = blockIdx.x, h = blockIdx.y, hq = h / (p.H / p.qk_heads);
+    const int place = blockIdx.x, h = blockIdx.y;
     const Where at = find_chunk(p, place);
     if (at.request < 0) return;
     const int n = min(CHUNK, p.q_len[at.request] - at.token);
     const size_t token0 = (size_t)p.q_start[at.request] + at.token;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
-    stage<float, DK, THREADS>(ks, PK, p.k + (token0 * p.qk_heads + hq) * DK, (size_t)p.qk_heads * DK, n);
+    stage<float, DK, THREADS>(ks, PK, p.k + (token0 * p.H + h) * DK, (size_t)p.H * DK, n);
     stage<T, DV, THREADS>(vs, PV, (const T*)p.v + token0 * p.v_ld + (size_t)h * DV, p.v_ld, n);
-    if (warp == 0) chunk_decays(p, h, token0, n, logs, signs, scales);
+    chunk_decays(p.decay[h], powers);
     staged();
-    if (tid < CHUNK) w[tid] = exp2f((float)(logs[CHUNK - 1] - logs[tid])) * signs[CHUNK - 1] * signs[tid] * scales[tid];
-    if (tid == 0) p.spans[(size_t)place * p.H + h] = exp2f((float)logs[CHUNK - 1]) * signs[CHUNK - 1];
-    __syncthreads();
+    if (tid == 0) p.spans[(size_t)place * p.H + h] = powers[n];
     const int m0 = (warp % WM) * 32, n0 = (warp / WM) * (DK / WN);
     float acc[2][NT][4];
 #pragma unroll
@@ -202,26 +205,22 @@ chunk_states_kernel(const ChunkParams p) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[m][t][i] = 0.f;
 #pragma unroll 2
-    for (int j = 0; j < CHUNK; j += 8) {
-        HalvesA a[2];
-        const float *va = vs + (j + c) * PV + m0 + g, *vb = va + 4 * PV;
+    for (int j = 0; j < CHUNK; j += 16) {
+        const int j0 = j + 2 * c;                    // the lane's tokens: j0, j0 + 1, j0 + 8, j0 + 9
+        Rows<terms_of<T>()> a[2];
+        const float* va = vs + j0 * PV + m0 + g;
 #pragma unroll
-        for (int m = 0; m < 2; ++m) a[m] = {halves(va[16 * m]), halves(va[16 * m + 8]), halves(vb[16 * m]), halves(vb[16 * m + 8])};
-        const float w0 = w[j + c], w1 = w[j + c + 4];
+        for (int m = 0; m < 2; ++m, va += 16)
+            a[m] = rows<terms_of<T>()>(make_float4(va[0], va[PV], va[8 * PV], va[9 * PV]),
+                                       make_float4(va[8], va[PV + 8], va[8 * PV + 8], va[9 * PV + 8]));
+        const float w0 = powers[max(n - 1 - j0, 0)], w1 = powers[max(n - 2 - j0, 0)];              // keys from n on are zero
+        const float w2 = powers[max(n - 9 - j0, 0)], w3 = powers[max(n - 10 - j0, 0)];
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            const Halves b0 = halves(ks[(j + c) * PK + n0 + 8 * t + g] * w0), b1 = halves(ks[(j + c + 4) * PK + n0 + 8 * t + g] * w1);
+            const float* ka = ks + j0 * PK + n0 + 8 * t + g;
+            const Columns<3> b = columns<3>(make_float4(ka[0] * w0, ka[PK] * w1, ka[8 * PK] * w2, ka[9 * PK] * w3));
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                if constexpr (sizeof(T) == 4) {
-                    add_one(acc[m][t], a[m], b0, b1);
-                } else {                                     // a 16-bit value has no trailing half
-                    float x[4];
-                    mma_from_zero(x, a[m].x0.hi, a[m].x1.hi, a[m].x2.hi, a[m].x3.hi, b0.lo, b1.lo);
-                    mma(x, a[m].x0.hi, a[m].x1.hi, a[m].x2.hi, a[m].x3.hi, b0.hi, b1.hi);
-                    add(acc[m][t], x);
-                }
-            }
+            for (int m = 0; m < 2; ++m) add_product(acc[m][t], a[m], b);
         }
     }
     float* dst = p.adds + ((size_t)place * p.H + h) * DV * DK;
@@ -275,9 +274,8 @@ chunk_prefix_kernel(const ChunkParams p, int elements) {
 }
 
 // The outputs of half of the value dims: a warp owns 16 tokens; it forms its tokens' scores against the keys up to them,
-// which are then its 16-row operand as they lie in its registers: step t of the contraction takes tokens 8t + 2c and
-// 8t + 2c + 1 for the k of lane c.  Contractions over the key dims take four neighbouring dims a lane and two steps, so that
-// queries, keys and the state come as 16-byte pieces; the state's come straight from memory, a step ahead.
+// which are then its 16-row operand as they lie in its registers (tokens 8t + 2c and 8t + 2c + 1 of two tiles t).
+// Contractions over the key dims take four neighbouring dims a lane, so that queries, keys and the state come as 16-byte pieces; the state's come straight from memory, a step ahead.
 constexpr int OUT_THREADS = 128;
 template <typename T, int DK, int DV>
 __global__ void __launch_bounds__(OUT_THREADS, 2)
@@ -287,25 +285,24 @@ chunk_outputs_kernel(const ChunkParams p) {
     float* qs = sm;
     float* ks = qs + CHUNK * PK;
     float* vs = ks + CHUNK * PK;
-    __shared__ double logs[CHUNK];
-    __shared__ float signs[CHUNK], scales[CHUNK];
+    __shared__ float powers[CHUNK + 1];
     pdl_launch_dependents();
     pdl_wait();
-    const int place = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * HV, hq = h / (p.H / p.qk_heads);
+    const int place = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * HV;
     const Where at = find_chunk(p, place);
     if (at.request < 0) return;
     const int n = min(CHUNK, p.q_len[at.request] - at.token);
     const size_t token0 = (size_t)p.q_start[at.request] + at.token;
     const int tid = threadIdx.x, m = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
-    stage<float, DK, OUT_THREADS>(qs, PK, p.q + (token0 * p.qk_heads + hq) * DK, (size_t)p.qk_heads * DK, n);
-    stage<float, DK, OUT_THREADS>(ks, PK, p.k + (token0 * p.qk_heads + hq) * DK, (size_t)p.qk_heads * DK, n);
+    stage<float, DK, OUT_THREADS>(qs, PK, p.q + (token0 * p.H + h) * DK, (size_t)p.H * DK, n);
+    stage<float, DK, OUT_THREADS>(ks, PK, p.k + (token0 * p.H + h) * DK, (size_t)p.H * DK, n);
     stage<T, HV, OUT_THREADS>(vs, PV, (const T*)p.v + token0 * p.v_ld + (size_t)h * DV + v0, p.v_ld, n);
     const int i0 = 16 * m + g, i1 = i0 + 8;
     const float* before = p.adds + ((size_t)place * p.H + h) * DV * DK + (size_t)(v0 + g) * DK;
     float4 s[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) s[t] = *(const float4*)(before + (size_t)8 * t * DK + 4 * c);
-    if (m == 0) chunk_decays(p, h, token0, n, logs, signs, scales);
+    chunk_decays(p.decay[h], powers);
     staged();
     if (16 * m >= n) return;
     const float *qa = qs + i0 * PK, *qb = qs + i1 * PK;
@@ -321,7 +318,7 @@ chunk_outputs_kernel(const ChunkParams p) {
 #pragma unroll 1
     for (int d = 4 * c; d < DK; d += 16) {
         const float4 a = *(const float4*)(qa + d), b = *(const float4*)(qb + d);
-        const HalvesA q0 = {halves(a.x), halves(b.x), halves(a.y), halves(b.y)}, q1 = {halves(a.z), halves(b.z), halves(a.w), halves(b.w)};
+        const Rows<3> q = rows<3>(a, b);
         float4 now[NT];
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
@@ -330,12 +327,11 @@ chunk_outputs_kernel(const ChunkParams p) {
         }
 #pragma unroll
         for (int t = 0; t < 8; ++t)
-            if (t < 2 * (m + 1)) add_two(sc[t], q0, q1, *(const float4*)(ks + (8 * t + g) * PK + d));
+            if (t < 2 * (m + 1)) add_product(sc[t], q, columns<3>(*(const float4*)(ks + (8 * t + g) * PK + d)));
 #pragma unroll
-        for (int t = 0; t < NT; ++t) add_two(acc[t], q0, q1, now[t]);
+        for (int t = 0; t < NT; ++t) add_product(acc[t], q, columns<3>(now[t]));
     }
-    const double la = logs[i0], lb = logs[i1];
-    const float fa = exp2f((float)la) * signs[i0], fb = exp2f((float)lb) * signs[i1];
+    const float fa = powers[i0 + 1], fb = powers[i1 + 1];
 #pragma unroll
     for (int t = 0; t < NT; ++t) { acc[t][0] *= fa; acc[t][1] *= fa; acc[t][2] *= fb; acc[t][3] *= fb; }
 #pragma unroll
@@ -344,24 +340,20 @@ chunk_outputs_kernel(const ChunkParams p) {
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 const int j = 8 * t + 2 * c + x;
-                const double lj = logs[j];
-                const float sj = scales[j] * signs[j];
-                sc[t][x] = j <= i0 ? sc[t][x] * (exp2f((float)(la - lj)) * signs[i0] * sj) : 0.f;
-                sc[t][2 + x] = j <= i1 ? sc[t][2 + x] * (exp2f((float)(lb - lj)) * signs[i1] * sj) : 0.f;
+                sc[t][x] = j <= i0 ? sc[t][x] * powers[max(i0 - j, 0)] : 0.f;
+                sc[t][2 + x] = j <= i1 ? sc[t][2 + x] * powers[max(i1 - j, 0)] : 0.f;
             }
-            const HalvesA a = {halves(sc[t][0]), halves(sc[t][2]), halves(sc[t][1]), halves(sc[t][3])};
+        }
+#pragma unroll
+    for (int t = 0; t < 8; t += 2)
+        if (t < 2 * (m + 1)) {
+            const Rows<3> a = rows<3>(make_float4(sc[t][0], sc[t][1], sc[t + 1][0], sc[t + 1][1]),
+                                      make_float4(sc[t][2], sc[t][3], sc[t + 1][2], sc[t + 1][3]));
             const float* vr = vs + (8 * t + 2 * c) * PV + g;
 #pragma unroll
             for (int u = 0; u < NT; ++u) {
-                if constexpr (sizeof(T) == 4) {
-                    add_one(acc[u], a, halves(vr[8 * u]), halves(vr[PV + 8 * u]));
-                } else {
-                    const uint32_t b0 = __float_as_uint(vr[8 * u]), b1 = __float_as_uint(vr[PV + 8 * u]);
-                    float x[4];
-                    mma_from_zero(x, a.x0.lo, a.x1.lo, a.x2.lo, a.x3.lo, b0, b1);
-                    mma(x, a.x0.hi, a.x1.hi, a.x2.hi, a.x3.hi, b0, b1);
-                    add(acc[u], x);
-                }
+                const float4 y = make_float4(vr[8 * u], vr[PV + 8 * u], vr[8 * PV + 8 * u], vr[9 * PV + 8 * u]);
+                add_product(acc[u], a, columns<terms_of<T>()>(y));
             }
         }
     float* dst = p.out + (token0 * p.H + h) * DV + v0 + 2 * c;
@@ -381,7 +373,7 @@ int allow_smem(K kernel, size_t smem) {
 
 template <typename T, int DK, int DV>
 int launch(const ChunkParams& p, int chunks, cudaStream_t stream) {
-    const size_t s1 = sizeof(float) * CHUNK * (DK + 8 + DV + 8), s3 = sizeof(float) * CHUNK * (2 * (DK + 16) + DV / 2 + 4);
+    const size_t s1 = sizeof(float) * CHUNK * (DK + 4 + DV + 4), s3 = sizeof(float) * CHUNK * (2 * (DK + 16) + DV / 2 + 4);
     if (const int rc = allow_smem(chunk_states_kernel<T, DK, DV>, s1)) return rc;
     if (const int rc = allow_smem(chunk_outputs_kernel<T, DK, DV>, s3)) return rc;
     if (const int rc = tnx_launch_in_order(chunk_states_kernel<T, DK, DV>, dim3(chunks, p.H), dim3(THREADS), s1, stream, p)) return rc;
@@ -399,21 +391,18 @@ int launch_sizes(const ChunkParams& p, int dk, int dv, int chunks, cudaStream_t 
 
 }  // namespace
 
-// The most chunks that `tokens` tokens of `n_requests` requests can be cut into.
-TNX_EXPORT int tnx_retention_chunks(int tokens, int n_requests) { return tokens / CHUNK + n_requests; }
-
-// As tnx_retention_scan; adds holds tnx_retention_chunks x H x dv x dk floats, spans tnx_retention_chunks x H.
+// As tnx_retention_scan with a decay per head; adds holds (tokens / 64 + n_requests) x H x dv x dk floats, spans
+// (tokens / 64 + n_requests) x H.
 TNX_EXPORT int tnx_retention_chunked(const float* q, const float* k, const void* v, int v_ld, const float* decay, float* state,
                                      const int* q_start, const int* q_len, const int* state_slots, float* out, int tokens,
-                                     int n_requests, int H, int dk, int dv, int v_h16, const float* decay_tok,
-                                     const float* kscale_tok, int qk_heads, float* adds, float* spans, cudaStream_t stream) {
+                                     int n_requests, int H, int dk, int dv, int v_h16, float* adds, float* spans, cudaStream_t stream) {
     if (n_requests <= 0 || tokens <= 0) return 0;
-    if (H <= 0 || H > 65535 || n_requests > 65535 || qk_heads <= 0 || H % qk_heads || (!decay && !decay_tok) || !adds || !spans)
+    if (H <= 0 || H > 65535 || n_requests > 65535 || !decay || !adds || !spans)
         return TNX_ERR_BAD_ARG;
     const int vsize = v_h16 ? 2 : 4;
     if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)state | (uintptr_t)out | (uintptr_t)adds) & 15) || ((uintptr_t)v % (4 * vsize)) || v_ld % 4)
         return TNX_ERR_UNSUPPORTED;
-    const ChunkParams p{q, k, v, v_ld, decay, decay_tok, kscale_tok, state, q_start, q_len, state_slots, out, adds, spans, n_requests, H, qk_heads};
-    const int chunks = tnx_retention_chunks(tokens, n_requests);
+    const ChunkParams p{q, k, v, v_ld, decay, state, q_start, q_len, state_slots, out, adds, spans, n_requests, H};
+    const int chunks = tokens / CHUNK + n_requests;          // the most that the tokens can be cut into
     return v_h16 ? launch_sizes<h16>(p, dk, dv, chunks, stream) : launch_sizes<float>(p, dk, dv, chunks, stream);
 }

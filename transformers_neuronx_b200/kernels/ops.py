@@ -1330,7 +1330,7 @@ RETENTION_CHUNKED_BYTES = 1 << 28     # the most scratch memory of a scan in chu
 
 def retention_chunked_takes(tokens: int, requests: int, n_heads: int, k_dim: int, v_dim: int) -> bool:
     """Whether a scan that may run in chunks of 64 tokens does: where the requests are several chunks long (one request of
-    128 / 256 / 512 tokens, 16 heads of 128 x 128: 27 us token by token and 34 in chunks, 47 and 38, 88 and 41; 8 requests
+    128 / 256 / 512 tokens, 16 heads of 128 x 128: 27 us token by token and 34 in chunks, 47 and 38, 88 and 39; 8 requests
     of 64: 53 and 48, 16 of 16: 29 and 52), the chunks' states (1 MB each there) stay bounded, and the step is long enough
     that the device is what it waits for: the two more launches are the host's time before (a layer over 439 tokens of
     two requests 139 us token by token and 160 in chunks, over 800 of four 180 and 166, over 768 of one 218 and 145)."""
@@ -1347,7 +1347,8 @@ def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_he
     small stages.  decay_tok, kscale_tok (32-bit [N, n_heads]): S <- decay_tok S + kscale_tok k v^T with numbers of the
     token (absent: decay[h], 1); qk_heads: q and k are [N, qk_heads * k_dim] and head h reads those of
     h // (n_heads // qk_heads).  chunked: portions of prompts may run 64 tokens at a time on the tensor cores
-    (csrc/retention_chunked.cu: 32-bit results to a rounding, but where a prompt was cut then shows in the last bits);
+    (csrc/retention_chunked.cu, a decay per head alone: 32-bit results to a rounding, but where a prompt was cut and how many
+    tokens and requests the step has then show in the last bits);
     None: they do wherever the kernels take the sizes (a test hook)."""
     lib = _lib("retention", v)
     N = q.shape[0]
@@ -1381,16 +1382,16 @@ def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_he
     R = q_len.shape[0]
     if q_start.shape[0] < R or state_slots.shape[0] < R:
         raise KernelError("q_start and state_slots must cover every request of q_len")
-    if (chunked is not False and k_dim in (64, 128) and v_dim in (64, 128) and v_ld % 4 == 0 and v.data_ptr() % (4 * v.element_size()) == 0
-            and not any(t.data_ptr() % 16 for t in (q, k, state, out))
-            and (chunked is None or retention_chunked_takes(N, R, n_heads, k_dim, v_dim))):
+    if (chunked is not False and (chunked is None or retention_chunked_takes(N, R, n_heads, k_dim, v_dim))
+            and decay_tok is None and kscale_tok is None and qk_heads == n_heads
+            and k_dim in (64, 128) and v_dim in (64, 128) and v_ld % 4 == 0 and v.data_ptr() % (4 * v.element_size()) == 0
+            and not any(t.data_ptr() % 16 for t in (q, k, state, out))):
         chunk_lib = _lib("retention_chunked", v)
         states = (N // 64 + R) * n_heads * v_dim * k_dim     # one of every chunk and head, and behind them its decays
         adds = torch.empty(states + states // (v_dim * k_dim), dtype=torch.float32, device=q.device)
         _check(chunk_lib.tnx_retention_chunked(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                                _p(state_slots), _p(out), c_int(N), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
-                                               c_int(_is_h16(v)), _p(decay_tok), _p(kscale_tok), c_int(qk_heads), _p(adds),
-                                               c_void_p(adds.data_ptr() + 4 * states), _stream()), "retention_scan")
+                                               c_int(_is_h16(v)), _p(adds), c_void_p(adds.data_ptr() + 4 * states), _stream()), "retention_scan")
         return
     _check(lib.tnx_retention_scan(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                   _p(state_slots), _p(out), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
