@@ -242,6 +242,44 @@ def test_retention_in_chunks_is_no_further_from_64_bit(dtype, dk, dv):
     assert bool((errors[1] <= 1.1 * errors[0]).all()), errors
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what", ["q", "k", "v"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_what_is_not_finite_leaves_earlier_tokens_whole(dtype, what, bad):
+    """A query that is not finite is its own token's alone, a key or value reaches the tokens from its own on, a value those of
+    its dim: every other output and state element has the bits that it has without it."""
+    from transformers_neuronx_b200.kernels import ops
+    H, dk, dv, N, slots = 2, 128, 64, 200, [0]
+    g = torch.Generator().manual_seed(3)
+    x = {"q": torch.randn(N, H * dk, generator=g), "k": torch.randn(N, H * dk, generator=g) * dk ** -0.5,
+         "v": torch.randn(N, H * dv, generator=g).to(dtype)}
+    decay = torch.tensor([0.97, 0.9995]).to(DEV)
+
+    def run():
+        state, out = torch.zeros(1, H, dv, dk, device=DEV), torch.zeros(N, H * dv, device=DEV)
+        ops.retention_scan(x["q"].to(DEV), x["k"].to(DEV), x["v"].to(DEV), decay, state, _i32([0]), _i32([N]), _i32([0]), out, H, dk, dv,
+                           chunked=None)
+        return out.view(N, H, dv), state[0]
+    want_out, want_state = run()
+    for t in (0, 5, 15, 63, 64 + 9, 128 + 17, N - 1):
+        col = 0 * dv + 21 if what == "v" else dk + 100                     # head 0's value dim 21, head 1's key dim 100
+        keep, x[what] = x[what], x[what].clone()
+        x[what][t, col] = bad
+        out, state = run()
+        x[what] = keep
+        hurt, hurt_state = torch.zeros(N, H, dv, dtype=torch.bool), torch.zeros(H, dv, dk, dtype=torch.bool)
+        if what == "q":
+            hurt[t, 1] = True
+        elif what == "k":
+            hurt[t:, 1] = True
+            hurt_state[1, :, 100] = True
+        else:
+            hurt[t:, 0, 21] = True
+            hurt_state[0, 21] = True
+        assert torch.equal(torch.isfinite(out).cpu(), ~hurt) and torch.equal(torch.isfinite(state).cpu(), ~hurt_state)
+        assert torch.equal(out.cpu()[~hurt], want_out.cpu()[~hurt]) and torch.equal(state.cpu()[~hurt_state], want_state.cpu()[~hurt_state])
+
+
 @pytest.mark.parametrize("H, dk, dv, rot", [(3, 20, 24, 12), (2, 128, 64, 128), (1, 256, 16, 0), (2, 8, 40, 8)])
 def test_retention_for_single_tokens_in_one_kernel(H, dk, dv, rot):
     """Rotation, state update, output, head-wise norm, gate and scale of a step of single tokens, against the

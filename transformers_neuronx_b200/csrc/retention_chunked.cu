@@ -18,8 +18,6 @@
 // and powers from 32-bit logarithms): outputs at a decay of 0.5 8.8e-8 and 8.6e-8 (1.5e-7), at 0.9 1.0e-7 and 8.9e-8 (1.7e-7),
 // at 0.97 1.3e-7 and 9.4e-8 (1.9e-7), at 0.99 2.0e-7 and 1.0e-7 (1.9e-7), at 0.9997 4.7e-7 and 1.2e-7 (2.3e-7); the state at
 // 0.5 4.0e-8 and 6.0e-8, at 0.9 6.4e-8 and 6.3e-8, at 0.97 1.1e-7 and 6.5e-8, at 0.9997 5.8e-7 and 1.1e-7.
-//
-// A value that is not finite leaves the outputs of its request undefined from its chunk of 16 tokens on.
 #include "common.cuh"
 
 namespace {
@@ -352,7 +350,21 @@ chunk_outputs_kernel(const ChunkParams p) {
             const float* vr = vs + (8 * t + 2 * c) * PV + g;
 #pragma unroll
             for (int u = 0; u < NT; ++u) {
-                const float4 y = make_float4(vr[8 * u], vr[PV + 8 * u], vr[8 * PV + 8 * u], vr[9 * PV + 8 * u]);
+                float4 y = make_float4(vr[8 * u], vr[PV + 8 * u], vr[8 * PV + 8 * u], vr[9 * PV + 8 * u]);
+                if (t == 2 * m && __any_sync(0xffffffffu, !(isfinite(y.x) && isfinite(y.y) && isfinite(y.z) && isfinite(y.w)))) {
+                    // The tiles have later tokens beside earlier ones, whose scores are zeros, and zero times such a value is
+                    // none: it is left out of the product and marks its own and later tokens by itself.
+                    y.x = isfinite(y.x) ? y.x : 0.f; y.y = isfinite(y.y) ? y.y : 0.f;
+                    y.z = isfinite(y.z) ? y.z : 0.f; y.w = isfinite(y.w) ? y.w : 0.f;
+#pragma unroll 1
+                    for (int j = 8 * t; j < 8 * t + 16; ++j)
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+                            if (!isfinite(vs[j * PV + 8 * u + 2 * c + x])) {
+                                if (j <= i0) acc[u][x] = NAN;
+                                if (j <= i1) acc[u][2 + x] = NAN;
+                            }
+                }
                 add_product(acc[u], a, columns<terms_of<T>()>(y));
             }
         }
