@@ -294,7 +294,8 @@ def test_the_recurrence_across_cuts_and_slots(H, G, dk, dv):
 
 
 @pytest.mark.parametrize("H, G, dk, dv", [(2, 1, 16, 64), (2, 2, 28, 18), (4, 2, 64, 64), (1, 1, 72, 30), (2, 1, 128, 33), (1, 1, 256, 8), (2, 1, 18, 7)])
-def test_the_scan_ahead_over_stage_edges(H, G, dk, dv):
+@pytest.mark.parametrize("ahead", [True, False])
+def test_the_scan_ahead_over_stage_edges(H, G, dk, dv, ahead):
     """Requests of one token, of whole stages (16, 8 and 4 tokens) and of one more and one less, up to four stages and through
     all three buffers, in one call; columns that end inside a lane's pair and a warp's.  An output is a sum of at most 256
     rounded products whose terms' errors are carried on by a state that forgets: 2^-24 x 64 of the largest value."""
@@ -319,9 +320,38 @@ def test_the_scan_ahead_over_stage_edges(H, G, dk, dv):
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
     state, out = state0.to(DEV), torch.zeros(N, H * dv, device=DEV)
     ops.delta_scan(*(x.reshape(N, -1).to(DEV) for x in (q, k, v, beta, decay)), state, i32([sum(lens[:r]) for r in range(R)]), i32(lens),
-                   i32(list(range(R))), out, H, G, dk, dv)
+                   i32(list(range(R))), out, H, G, dk, dv, ahead=ahead)
     for got, ref in ((out.view(N, H, dv).cpu().double(), want), (state.cpu().double(), states)):
         assert float((got - ref).abs().max()) <= 2.0 ** -24 * 64 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("H, G, dk, dv", [(2, 1, 16, 64), (2, 2, 28, 18), (4, 2, 64, 64), (2, 1, 128, 33), (1, 1, 256, 8), (2, 1, 18, 7)])
+def test_where_a_prompt_is_cut_does_not_show_in_the_state(H, G, dk, dv):
+    """One request whole, in portions that end off and on the stages' edges, and token by token: outputs and state bit for bit
+    the same.  The form that sums a token ahead, which a caller has to ask for, differs by its roundings alone: 2^-24 x 64 of the
+    largest value, as above."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(dk)
+    T = 70
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k = unit(torch.randn(T, G, dk, generator=g)) * dk ** -0.5, unit(torch.randn(T, G, dk, generator=g))
+    v, beta = torch.randn(T, H, dv, generator=g), torch.rand(T, H, generator=g)
+    decay = torch.exp(-torch.rand(T, H, dk, generator=g) ** 2)
+    rows = [x.reshape(T, -1).to(DEV) for x in (q, k, v, beta, decay)]
+    state0 = torch.randn(1, H, dv, dk, generator=g).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def run(cuts, **kw):
+        state, out = state0.clone(), torch.zeros(T, H * dv, device=DEV)
+        for lo, hi in zip(cuts, cuts[1:]):
+            ops.delta_scan(*(x[lo:hi] for x in rows), state, i32([0]), i32([hi - lo]), i32([0]), out[lo:hi], H, G, dk, dv, **kw)
+        return out, state
+    want = run([0, T])
+    for cuts in ([0, 1, T], [0, 16, 48, T], [0, 7, 24, 41, T], list(range(T + 1))):
+        for got, ref in zip(run(cuts), want):
+            assert torch.equal(got, ref), cuts
+        for got, ref in zip(run(cuts, ahead=True), want):
+            assert float((got - ref).abs().max()) <= 2.0 ** -24 * 64 * float(ref.abs().max())
 
 
 def test_a_value_written_long_ago_is_read_back_exactly():

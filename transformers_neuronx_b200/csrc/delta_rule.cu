@@ -218,11 +218,12 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool ta
                  "r"(take ? 16u : 0u) : "memory");
 }
 
-// Key sizes that are no multiple of 4, and rows off 16-byte boundaries.  KPT: rows of a column one thread keeps; R: lanes
-// a column's rows are spread over (KPT * R >= k_dim); a block of 128 threads owns 128 / R columns.  The tokens' inputs come in
-// stages through two buffers: while one stage is walked, the next one's copies are in flight, so the walk waits for memory
-// once, at the first stage.
-template <int KPT, int R>
+// One form for every token, so that the state after a token has the same bits however the prompt was cut.  KPT: rows of a
+// column one thread keeps; R: lanes a column's rows are spread over (KPT * R >= k_dim); a block of 128
+// threads owns 128 / R columns.  The tokens' inputs come in stages through two buffers: while one stage is walked, the
+// next one's copies are in flight, so the walk waits for memory once, at the first stage.  VEC: k_dim is a multiple
+// of 4 and the rows are 16-byte aligned (16-byte copies).
+template <int KPT, int R, bool VEC>
 __global__ void __launch_bounds__(128)
 delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ g, float* __restrict__ state,
@@ -245,13 +246,24 @@ delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
 
     auto fetch = [&](int t0, int buf) {               // the inputs of tokens t0 .. t0 + ST - 1 of this request's rows
         const int nt = min(ST, len - t0);
-        for (int e = threadIdx.x; e < nt * DKP; e += 128) {
-            const int tt = e / DKP, i = e % DKP;
-            const size_t t = (size_t)(t_first + t0 + tt);
-            const bool in = i < dk;
-            cp_async4(&qs[buf][tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
-            cp_async4(&ks[buf][tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
-            cp_async4(&gs[buf][tt][i], in ? g + (t * H + h) * dk + i : g, in);
+        if (VEC) {
+            for (int e = threadIdx.x; e < nt * (DKP / 4); e += 128) {
+                const int tt = e / (DKP / 4), i = (e % (DKP / 4)) * 4;
+                const size_t t = (size_t)(t_first + t0 + tt);
+                const bool in = i < dk;
+                cp_async16(&qs[buf][tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
+                cp_async16(&ks[buf][tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
+                cp_async16(&gs[buf][tt][i], in ? g + (t * H + h) * dk + i : g, in);
+            }
+        } else {
+            for (int e = threadIdx.x; e < nt * DKP; e += 128) {
+                const int tt = e / DKP, i = e % DKP;
+                const size_t t = (size_t)(t_first + t0 + tt);
+                const bool in = i < dk;
+                cp_async4(&qs[buf][tt][i], in ? q + (t * G + kvh) * dk + i : q, in);
+                cp_async4(&ks[buf][tt][i], in ? k + (t * G + kvh) * dk + i : k, in);
+                cp_async4(&gs[buf][tt][i], in ? g + (t * H + h) * dk + i : g, in);
+            }
         }
         for (int e = threadIdx.x; e < nt * C; e += 128) {
             const int tt = e / C, c = blockIdx.x * C + e % C;
@@ -325,7 +337,8 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float2 low(const float4& x) { return make_float2(x.x, x.y); }
 __device__ __forceinline__ float2 high(const float4& x) { return make_float2(x.z, x.w); }
 
-// Everything else.  A thread keeps KPT rows, in runs of four neighbours, of two neighbouring columns (what it reads from
+// Where the caller allows it (`ahead`): the first token of a call has no token before it whose write could be corrected for, so
+// where a prompt was cut shows in the last bits.  A thread keeps KPT rows, in runs of four neighbours, of two neighbouring columns (what it reads from
 // shared memory feeds both), and multiplies them in pairs; R lanes share the columns.
 // A token's write waits for the sum u = beta (v - S^T k), and that sum over R lanes is most of a token's chain.  So the walk
 // forms it a token ahead, from the state before the write that comes between, and corrects it by one number:
@@ -335,7 +348,7 @@ __device__ __forceinline__ float2 high(const float4& x) { return make_float2(x.z
 // the columns share (q.k and k.gk) likewise.  The lanes whose top bit is clear end up with S^T k and k.gk and form u, the
 // others with S^T q and q.k and form the output.
 // Measured, 16 heads of 128 x 128 on 4 key heads, against a column a lane and the sum inside the token's chain: three
-// requests of 512 tokens 360 -> 198 us, one of 2,048 650 -> 406 (32 heads 969 -> 557), one of 64 26 -> 19; four columns a
+// requests of 512 tokens 360 -> 198 us, one of 2,048 650 -> 406 (32 heads 969 -> 557), one of 64 26 -> 19, 64 single tokens 39 -> 35; four columns a
 // lane without the sum ahead 251, 799 (799); two 209, 527 (650); eight lanes a column 228, 656.  Errors against 64-bit are equal.
 // What bounds it: one warp a scheduler, about 150 instructions a token and the chain of two tokens in turn.
 // Inputs come in stages through three buffers: one is walked, the next one has landed (the token ahead may be its first), the
@@ -528,18 +541,22 @@ TNX_EXPORT int tnx_delta_prep(const void* proj, int ld, int col0, int b_off, con
 
 TNX_EXPORT int tnx_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* g,
                               float* state, const int* q_start, const int* q_len, const int* state_slots, float* out,
-                              int n_requests, int H, int G, int dk, int dv, cudaStream_t stream) {
+                              int n_requests, int H, int G, int dk, int dv, int ahead, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0) return TNX_ERR_BAD_ARG;
-    const bool vec = dk % 4 == 0 && !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)g | (uintptr_t)state) & 15);
+    const bool vec = dk % 4 == 0 && !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)g) & 15);
+    const bool wide = ahead && vec && !((uintptr_t)state & 15);
 #define DSCAN(KPT, R)                                                                                                   \
     do {                                                                                                                \
-        const int C = (vec ? 2 : 1) * (WIDE_THREADS / (R));                                                             \
+        const int C = wide ? 2 * (WIDE_THREADS / (R)) : 128 / (R);                                                      \
         const dim3 grid((dv + C - 1) / C, H, n_requests);                                                               \
-        if (vec)                                                                                                        \
+        if (wide)                                                                                                       \
             return tnx_launch_in_order(delta_scan_ahead_kernel<KPT, R>, grid, dim3(WIDE_THREADS), 0, stream, q, k, v,   \
                                        beta, g, state, q_start, q_len, state_slots, out, H, G, dk, dv);                 \
-        return tnx_launch_in_order(delta_scan_kernel<KPT, R>, grid, dim3(128), 0, stream, q, k, v, beta, g,             \
+        if (vec)                                                                                                        \
+            return tnx_launch_in_order(delta_scan_kernel<KPT, R, true>, grid, dim3(128), 0, stream, q, k, v, beta, g,   \
+                                       state, q_start, q_len, state_slots, out, H, G, dk, dv);                          \
+        return tnx_launch_in_order(delta_scan_kernel<KPT, R, false>, grid, dim3(128), 0, stream, q, k, v, beta, g,      \
                                    state, q_start, q_len, state_slots, out, H, G, dk, dv);                              \
     } while (0)
     if (dk <= 16) DSCAN(4, 4);

@@ -12,7 +12,8 @@ What the mixer keeps per request, both state of fixed size in the request's slot
 convolved channel in the activation type, exactly what a longer step would have read from its own rows.  Everything
 that enters the recurrence is 32-bit from the projections' output on: the convolution's sums, the unit norms, beta and g
 (their logits leave the second low-rank product in 32-bit).  A step's tokens of one request are walked in order by one
-kernel, portions of prompts and single tokens alike, so the state after a token does not depend on how the prompt was cut.
+kernel, portions of prompts and single tokens alike, so the state after a token does not depend on how the prompt was cut; in a
+16-bit engine, whose products' kernels depend on it anyway, the scan may sum a token ahead, to a 32-bit rounding the same.
 
 All projections of h (q, k, v, the two low-rank first halves, beta) are one product.
 """
@@ -116,7 +117,8 @@ class DeltaRule(Mixer):
         ops.delta_prep(proj, 0, C + ra + rg, a, self.conv_w, s.conv_taps, ctx.cache(1) if self.keep else None, ctx,
                        self.a_log, self.dt_bias, s.unit_eps, s.q_scale, s.conv_activation, q, k, v, beta, g, H, G, dk, dv)
         o = ctx.scratch(N, H * dv, f32)
-        ops.delta_scan(q, k, v, beta, g, ctx.cache(0), ctx.q_start, ctx.q_len, ctx.state_slots, o, H, G, dk, dv)
+        ops.delta_scan(q, k, v, beta, g, ctx.cache(0), ctx.q_start, ctx.q_len, ctx.state_slots, o, H, G, dk, dv,
+                       ahead=ctx.act_dtype != torch.float32)
         inner = ctx.scratch(N, H * dv)
         ops.headwise_gated_rms_norm(o, gate, ctx.token_request, self.norm_w, s.norm_eps, 1.0, inner, H, dv,
                                     gate_activation="sigmoid")
