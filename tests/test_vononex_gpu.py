@@ -152,6 +152,12 @@ def test_many_heads_are_normalised_in_pieces_of_eight(dv, H, N, dtype, step, act
     y, got = (0.7 * y).reshape(N, -1), out.cpu().double()
     keep = torch.arange(N) != 7
     assert bool(((got - y).abs()[keep] <= step * y.abs()[keep] + 1e-6).all()) and float((got[7] - 9.0).abs().max()) == 0.0
+    few = torch.full_like(out, 9.0)                      # calls of at most 511 heads, which the other form takes
+    for lo in range(0, N, 511 // H):
+        part = slice(lo, min(N, lo + 511 // H))
+        ops.headwise_gated_rms_norm(o[part].to(DEV), wide[part].to(DEV)[:, 16:] if activation else None, _i32(rows[part]), w.to(DEV), 1e-5, 0.7,
+                                    few[part], H, dv, gate_activation=activation or "silu")
+    assert torch.equal(few, out)                         # how many tokens come along does not show in a row
 
 
 @pytest.mark.parametrize("H, dk, rot", [(16, 128, 128), (3, 20, 8), (2, 64, 32), (1, 12, 8)])

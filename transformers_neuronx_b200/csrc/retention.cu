@@ -615,12 +615,13 @@ headwise_gated_rms_norm_vec_kernel(const float* __restrict__ o, const T* __restr
     if (w) { Vec8<float> t; t.load(w + c); t.get(wv); }
 #pragma unroll
     for (int i = 0; i < ROUNDS; ++i) {
-        float v[8], s = 0.f;
+        float v[8];
         x[i].get(v);
+        // in the order of the kernel below, whose lanes hold runs of four: bit for bit what a call of fewer heads gives
+        float s0 = (v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3]), s1 = (v[4] * v[4] + v[5] * v[5]) + (v[6] * v[6] + v[7] * v[7]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s = fmaf(v[e], v[e], s);
-#pragma unroll
-        for (int k = LANES / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+        for (int k = LANES / 2; k > 0; k >>= 1) { s0 += __shfl_xor_sync(0xffffffffu, s0, k); s1 += __shfl_xor_sync(0xffffffffu, s1, k); }
+        const float s = s0 + s1;
         const float rinv = 1.0f / sqrtf(s / (float)DV + eps);
         if (!there[i]) continue;
         float g[8];
