@@ -477,6 +477,30 @@ def test_grouped_product_in_pairs(counts, N, K, out_dtype):
     assert bool((out[M - 64:] == 7.0).all())
 
 
+@pytest.mark.parametrize("groups, N, K", [((0,), 128, 64), ((1, -1, 0, 1, -1), 264, 72), ((2, 2, 0), 200, 136), ((-1, -1), 256, 64), ((0,) * 6, 1032, 1096)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_grouped_product_of_128_row_tiles(groups, N, K, out_dtype):
+    """A caller's own layout of whole 128-row tiles, the default: groups in any order, tiles without one anywhere (their rows stay),
+    widths on both sides of the wide tile."""
+    from transformers_neuronx_b200.kernels import ops
+    g = torch.Generator().manual_seed(9)
+    M = 128 * len(groups)
+    a, w = torch.randn(M, K, generator=g).to(torch.bfloat16), torch.randn(3, N, K, generator=g).to(torch.bfloat16)
+    out = torch.full((M, N), 7.0, dtype=out_dtype, device=DEV)
+    ops.gemm_tc_grouped(a.to(DEV), w.to(DEV), out, _i32(groups))
+    ops.raise_on_device_error()
+    out = out.cpu().double()
+    for i, e in enumerate(groups):
+        rows = slice(128 * i, 128 * i + 128)
+        if e < 0:
+            assert bool((out[rows] == 7.0).all())
+            continue
+        x, m = a[rows].double(), w[e].double()
+        # as above: K sums in 32 bits, each off by at most an ulp, and the result's own rounding
+        bound = K * 2.0 ** -23 * (x.abs() @ m.abs().T) + (2.0 ** -8 * (x @ m.T).abs() if out_dtype == torch.bfloat16 else 0)
+        assert bool(((out[rows] - x @ m.T).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("N, W, E, top, F, on_input", [(300, 256, 8, 2, 128, True), (129, 320, 3, 3, 72, True),
                                                       (1000, 64, 40, 1, 200, False), (64, 128, 5, 4, 64, True),
                                                       (2, 2048, 8, 2, 2816, True), (9, 256, 8, 2, 136, True),      # tiles of 16

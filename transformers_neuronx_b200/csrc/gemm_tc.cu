@@ -61,7 +61,7 @@ struct Params {
     int sk_tiles;                // paired kernel: the last sk_tiles output tiles are shared out by K blocks
     int sk_pairs;                // ... over the first sk_pairs pairs
     const int* span_of_tile;     // grouped product in CTA pairs: a tile's rows, (first row / 32) * 8 + rows / 32 - 1
-    const int* group_of_tile;    // grouped product: the group of every tile of tokens (up to 256 of them in CTA pairs, or BN), -1: none;
+    const int* group_of_tile;    // grouped product: the group of every tile of tokens (128 of them, up to 256 in CTA pairs, BN in the swapped form), -1: none;
     int group_rows;              //   W holds group_rows rows per group, a tile of group g reads W's rows from g * group_rows on
     int batch_w_step;            // batched product (not swapped, K not split): blockIdx.z = b multiplies the columns of A from
     int batch_a_step;            //   b * batch_a_step on with W's rows from b * batch_w_step on and writes the columns of C from
@@ -382,13 +382,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     // A grouped product: every tile of tokens belongs to one group (an expert) and multiplies that group's rows of W.
     // Which group is written by the kernel before this one, so it is read behind the dependency wait; a tile without
     // a group has nothing to do (nothing has been set up yet, so the whole CTA may leave).
-    // (The tokens are the Q operand; the CTAs of a cluster share their tile of tokens, so they leave together.)
+    // (In the swapped form the tokens are the Q operand; the CTAs of a cluster share their tile of tokens, so they leave together.)
     int q_row0 = tile_q * BN, p_row0 = tile_p * TILE_P;
-    if (SWAP && p.group_of_tile != nullptr) {
+    if (p.group_of_tile != nullptr) {
         pdl_wait();
-        const int g = p.group_of_tile[tile_q];
+        const int g = p.group_of_tile[SWAP ? tile_q : tile_p];
         if (g < 0) return;
-        p_row0 += g * p.group_rows;
+        if (SWAP) p_row0 += g * p.group_rows; else q_row0 += g * p.group_rows;
     }
     q_row0 += batch * p.batch_w_step;
     // Split K summed in a cluster, swapped form, 2, 4 or 8 splits: every CTA sends the bands of its partial tile
@@ -1631,12 +1631,41 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
     return launch<128, 3, true>(mp, mq, p, grid, stream);
 }
 
+// A grouped product: C[m, :] = A[m, :] W_g^T for the rows m of every 128-row tile, g = group_of_tile[m / 128] (a device
+// array written by an earlier kernel; -1: the tile is skipped).  W holds the groups' matrices one after the other,
+// [groups * N, K]; A is [M, K] with M a multiple of 128; C is [M, ldc] in the 16-bit type or 32-bit.  No bias, no
+// activation: what follows a group's product is the caller's own kernel.
+TNX_EXPORT int tnx_gemm_tc_grouped(const void* A, const void* W, void* C, int M, int N, int K, int groups, int lda, int ldw,
+                                   int ldc, int c_h16, const int* group_of_tile, int* err_word, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || groups <= 0) return 0;
+    if (M % TILE_P || K <= 0 || K % 8 || lda % 8 || ldw % 8 || lda < K || ldw < K || ldc < N) return TNX_ERR_UNSUPPORTED;
+    if ((((uintptr_t)A | (uintptr_t)W) & 15) || (long long)groups * N >= (1ll << 31)) return TNX_ERR_UNSUPPORTED;
+    if (!err_word || !group_of_tile) return TNX_ERR_BAD_ARG;
+    Params p{};
+    p.K = K; p.ldc = ldc; p.act = TNX_ACT_NONE; p.c_is_h16 = c_h16; p.C = C; p.err = err_word;
+    p.rows_p = M; p.rows_q = N; p.splits = 1; p.kb_per_split = (K + BLOCK_K - 1) / BLOCK_K;
+    p.group_of_tile = group_of_tile; p.group_rows = N;
+    CUtensorMap mp, mq;
+    if (!make_map(&mp, A, M, K, lda, TILE_P)) return TNX_ERR_UNSUPPORTED;
+    // tiles of 128 x 256 where a group is wide enough: half as many activation bytes per FLOP into shared memory
+    // (measured on 8 experts of 11008 x 4096 and 4096 x 5504, 4,096 rows: 2.42 against 3.28 ms for four layers' products).
+    // Two stages, so that two CTAs fit on an SM and one's products run while the other stores its tile: 16 experts of
+    // 2048 x 2048 and 2048 x 1024 with about 410 rows each take 100 and 77 us, against 131 and 106 with one CTA of four stages;
+    // 8 of 11008 x 4096 and 4096 x 5504 with about 1,024 rows 763 and 371 against 907 and 449.
+    if (N >= 256) {
+        if (!make_map(&mq, W, groups * N, K, ldw, 256)) return TNX_ERR_UNSUPPORTED;
+        return launch<256, 2, false>(mp, mq, p, dim3(M / TILE_P, (N + 255) / 256, 1), stream);
+    }
+    if (!make_map(&mq, W, groups * N, K, ldw, 128)) return TNX_ERR_UNSUPPORTED;
+    return launch<128, 6, false>(mp, mq, p, dim3(M / TILE_P, (N + 127) / 128, 1), stream);
+}
+
 // A grouped product in CTA pairs: C[m, :] = A[m, :] W_g^T for the rows m of every tile of tokens, g = group_of_tile[tile] (a
 // device array written by an earlier kernel; -1: this tile has no group, nor has one after it).  A tile has up to 256 rows, given
 // by span_of_tile (first row / 32 * 8 + rows / 32 - 1; tiles do not overlap and end by row M, a multiple of 32).  W holds the
 // groups' matrices one after the other, [groups * N, K]; C is [M, ldc] in the 16-bit type or 32-bit.  No bias, no activation:
 // what follows a group's product is the caller's own kernel.
-TNX_EXPORT int tnx_gemm_tc_grouped(const void* A, const void* W, void* C, int M, int N, int K, int groups, int tiles, int lda,
+TNX_EXPORT int tnx_gemm_tc_grouped_pairs(const void* A, const void* W, void* C, int M, int N, int K, int groups, int tiles, int lda,
                                    int ldw, int ldc, int c_h16, const int* group_of_tile, const int* span_of_tile,
                                    int* err_word, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || groups <= 0 || tiles <= 0) return 0;

@@ -1114,19 +1114,19 @@ def moe_grouped_supported(h, gate_up, down) -> bool:
             and gate_up.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0 and E * max(F2, W) < 2 ** 31)
 
 
-def gemm_tc_grouped(a, w, out, group_of_tile, tile=256, used_tiles=0, span_of_tile=None):
+def gemm_tc_grouped(a, w, out, group_of_tile, tile=128, used_tiles=0, span_of_tile=None):
     """out[m] = a[m] @ w[g]^T for the rows m of every tile, g = group_of_tile[tile] (-1: the tile is skipped).  a [M, K] and
-    w [groups, N, K] in one 16-bit type; out [M, N] in that type or 32-bit.  tile 256: CTA pairs, tiles of up to 256 tokens
-    given by span_of_tile (first row / 32 * 8 + rows / 32 - 1), the ones with a group first, M a multiple of 32; 16, 32 or
-    64: tiles of so many tokens (M a multiple of it) against 128 rows of the group's matrix, K split in clusters while
-    the `used_tiles` tiles expected to have a group leave SMs idle."""
+    w [groups, N, K] in one 16-bit type; out [M, N] in that type or 32-bit.  tile 128: tiles of 128 tokens (M a multiple of it);
+    256: CTA pairs, tiles of up to 256 tokens given by span_of_tile (first row / 32 * 8 + rows / 32 - 1), the ones with a
+    group first, M a multiple of 32; 16, 32 or 64: tiles of so many tokens (M a multiple of it) against 128 rows of the
+    group's matrix, K split in clusters while the `used_tiles` tiles expected to have a group leave SMs idle."""
     lib = _lib("gemm_tc", a, w, out)
     _need(a, "a", _H16, 2); _need(w, "w", a.dtype, 3); _need(out, "out", _FLOATS, 2)
     _need(group_of_tile, "group_of_tile", torch.int32, 1)
     M, K = a.shape
     G, N, Kw = w.shape
     tiles = group_of_tile.shape[0]
-    if Kw != K or tuple(out.shape) != (M, N) or tile not in (16, 32, 64, 256) or M % (32 if tile == 256 else tile) \
+    if Kw != K or tuple(out.shape) != (M, N) or tile not in (16, 32, 64, 128, 256) or M % (32 if tile == 256 else tile) \
             or (tile < 256 and tiles < M // tile):
         raise KernelError(f"grouped product shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     st = _state(a.device)
@@ -1134,9 +1134,13 @@ def gemm_tc_grouped(a, w, out, group_of_tile, tile=256, used_tiles=0, span_of_ti
         _need(span_of_tile, "span_of_tile", torch.int32, 1)
         if span_of_tile.shape[0] < tiles:
             raise KernelError("span_of_tile must cover the tiles")
-        _check(lib.tnx_gemm_tc_grouped(_p(a), _p(w), _p(out), c_int(M), c_int(N), c_int(K), c_int(G), c_int(tiles), c_int(K),
-                                       c_int(K), c_int(N), c_int(_is_h16(out)), _p(group_of_tile), _p(span_of_tile),
-                                       _p(st["err"]), _stream()), "gemm_tc_grouped")
+        _check(lib.tnx_gemm_tc_grouped_pairs(_p(a), _p(w), _p(out), c_int(M), c_int(N), c_int(K), c_int(G), c_int(tiles), c_int(K),
+                                             c_int(K), c_int(N), c_int(_is_h16(out)), _p(group_of_tile), _p(span_of_tile),
+                                             _p(st["err"]), _stream()), "gemm_tc_grouped")
+        return
+    if tile == 128:
+        _check(lib.tnx_gemm_tc_grouped(_p(a), _p(w), _p(out), c_int(M), c_int(N), c_int(K), c_int(G), c_int(K), c_int(K), c_int(N),
+                                       c_int(_is_h16(out)), _p(group_of_tile), _p(st["err"]), _stream()), "gemm_tc_grouped")
         return
     _check(lib.tnx_gemm_tc_grouped_few(_p(a), _p(w), _p(out), c_int(M), c_int(N), c_int(K), c_int(G), c_int(tile),
                                        c_int(int(used_tiles)), c_int(K), c_int(K), c_int(N), c_int(_is_h16(out)),
