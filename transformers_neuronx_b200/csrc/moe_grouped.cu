@@ -1,7 +1,7 @@
 // Routed experts on the tensor cores: the (token, chosen expert) pairs are sorted by expert into a layout in which every
-// expert's rows begin at a multiple of the granule, and each tile belongs to one expert: 16, 32, 64 or 128 rows, which are the
-// granule too, where experts get few rows; up to 256 rows, of granules of 32, where they get many. The two products of an expert run as grouped tensor-core products
-// (gemm_tc.cu: tnx_gemm_tc_grouped, tnx_gemm_tc_grouped_few).  The kernels of this file are what lies around those products:
+// expert's rows begin at a multiple of the granule, and each tile belongs to one expert: 16, 32 or 64 rows, which are the granule
+// too, where experts get few rows; up to 256 rows, of granules of 32, where they get many.  The two products of an expert run
+// as grouped tensor-core products (gemm_tc.cu: tnx_gemm_tc_grouped_pairs, tnx_gemm_tc_grouped_few).  The kernels of this file are what lies around those products:
 //
 //   moe_plan_kernel      one block: counts per expert, every expert's first row, the expert of every tile (-1 beyond
 //                        the last used tile), how many of a granule's rows are pairs, and the row of every pair.
@@ -228,7 +228,7 @@ moe_combine_kernel(const float* __restrict__ rows, const h16* __restrict__ h, in
 }  // namespace
 
 // The most tiles that n_pairs pairs spread over n_experts experts can take.
-TNX_EXPORT int tnx_moe_grouped_max_tiles(int n_pairs, int n_experts, int tile) {
+static int max_tiles_of(int n_pairs, int n_experts, int tile) {
     return n_pairs / tile + (n_pairs < n_experts ? n_pairs : n_experts);
 }
 
@@ -237,8 +237,8 @@ TNX_EXPORT int tnx_moe_plan(const int* ids, int n_pairs, int n_experts, int max_
                             int* span_of_tile, int* rows_of_granule, int* row_of_pair, cudaStream_t stream) {
     if (n_pairs <= 0) return 0;
     const int granule = tile == 256 ? 32 : tile;
-    if (n_experts <= 0 || n_experts > MAX_EXPERTS || tile <= 0 || max_tiles < tnx_moe_grouped_max_tiles(n_pairs, n_experts, tile) ||
-        max_granules < tnx_moe_grouped_max_tiles(n_pairs, n_experts, granule) || (tile == 256) != (span_of_tile != nullptr))
+    if (n_experts <= 0 || n_experts > MAX_EXPERTS || tile <= 0 || max_tiles < max_tiles_of(n_pairs, n_experts, tile) ||
+        max_granules < max_tiles_of(n_pairs, n_experts, granule) || (tile == 256) != (span_of_tile != nullptr))
         return TNX_ERR_BAD_ARG;
     return tnx_launch_in_order(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, ids, n_pairs, n_experts, max_tiles, max_granules, tile,
                                granule, group_of_tile, span_of_tile, rows_of_granule, row_of_pair);

@@ -1195,15 +1195,14 @@ def moe_grouped(ctx, h, gate_up, down, ids, weights, out, gate_max, up_min, up_m
     # (16 experts of 4096 x 2048: 32 rows each 181 us in tiles of 64 and 196 in pairs, 64 rows 213 and 206, 128 rows 286 and
     # 223; 128 experts of 1536 x 2048 with 48 rows 337 and 315)
     tile = next((t for t in (16, 32, 64) if 2 * P <= t * E), 256)
-    tiles = lib.tnx_moe_grouped_max_tiles(c_int(P), c_int(E), c_int(tile))
+    tiles = P // tile + min(P, E)                            # the most that the pairs can take
     used = min(E, P) + P // tile // 2
     granule = 32 if tile == 256 else tile                    # of the rows; a tile of 256 takes as many granules as it needs
-    granules = lib.tnx_moe_grouped_max_tiles(c_int(P), c_int(E), c_int(granule))
+    granules = P // granule + min(P, E)
     rows = granules * granule
-    group_of_tile = ctx.scratch(1, tiles, torch.int32).view(-1)
-    span_of_tile = ctx.scratch(1, tiles, torch.int32).view(-1) if tile == 256 else None
-    rows_of_granule = ctx.scratch(1, granules, torch.int32).view(-1)
-    row_of_pair = ctx.scratch(1, P, torch.int32).view(-1)
+    sizes = [tiles, granules, P] + ([tiles] if tile == 256 else [])
+    group_of_tile, rows_of_granule, row_of_pair, *span = ctx.scratch(1, sum(sizes), torch.int32).view(-1).split(sizes)
+    span_of_tile = span[0] if span else None
     x = ctx.scratch(rows, W, h.dtype)
     moe_sort_rows(lib, h, ids, weights, E, tile, group_of_tile, span_of_tile, rows_of_granule, row_of_pair, x, weight_on_input)
     gu = ctx.scratch(rows, F2, h.dtype)
