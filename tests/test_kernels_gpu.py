@@ -502,6 +502,15 @@ def test_attention_simt_portions_and_rows_agree(n_heads, n_kv, d, dtype, options
     assert rel_err(outs[0], want.to(DEV)) <= (1e-5 if dtype == torch.float32 else 1e-2)
 
 
+@pytest.mark.parametrize("rows,window,kernels", [(103, 0, 2), (101, 0, 1), (103, 37, 1)])
+def test_attention_simt_counts_its_kernels(rows, window, kernels):
+    """20 heads: from 2,048 (row, head) pairs on without a window two kernels run, else one."""
+    case = PagedCase([(0, rows)], 20, 20, 32, torch.float32)
+    before = ops().launch_count()
+    ops().attention_simt(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, torch.zeros_like(case.q_flat), 20, 0.1, window)
+    assert ops().launch_count() - before == kernels
+
+
 @pytest.mark.parametrize("n_heads,n_kv,d", ATT_SHAPES)
 @pytest.mark.parametrize("window", [None, 50])
 @pytest.mark.parametrize("n_splits,warps", [(None, None), (1, 4), (3, 4), (7, 4), (1, 8), (2, 8), (5, 8), (1, 16), (3, 16), (20, 8), (44, 4)])

@@ -242,7 +242,9 @@ def test_retention_in_chunks_is_no_further_from_64_bit(dtype, dk, dv):
     errors = []
     for chunked in (False, None):
         state, out = state0.to(DEV), torch.zeros(T, H * dv, device=DEV)
+        before = ops.launch_count()
         ops.retention_scan(q.to(DEV), k.to(DEV), v.to(DEV), decay.to(DEV), state, _i32([0]), _i32([T]), _i32([0]), out, H, dk, dv, chunked=chunked)
+        assert ops.launch_count() - before == (1 if chunked is False else 3)
         o, s = out.view(T, H, dv).cpu().double(), state[0].cpu().double()
         errors.append(torch.cat([(o - want).norm(dim=(0, 2)) / want.norm(dim=(0, 2)), (s - S).norm(dim=(1, 2)) / S.norm(dim=(1, 2))]))
     assert bool((errors[1] <= 1.1 * errors[0]).all()), errors

@@ -32,10 +32,11 @@ def add_launches(n: int) -> None:
     _launches += int(n)
 
 
-def _check(code: int, what: str) -> None:
+def _check(code: int, what: str, kernels: int = 1) -> None:
+    """`kernels`: how many the entry point launches."""
     global _launches
     if code == 0:
-        _launches += 1
+        _launches += kernels
         return
     if code < 0:
         raise KernelError(f"{what}: {_ERRORS.get(code, 'error')} (code {code})")
@@ -306,11 +307,15 @@ def attention_simt(q, cache, block_tables, token_request, positions, out, n_head
     _need(block_tables, "block_tables", torch.int32, 2)
     _need(token_request, "token_request", torch.int32, 1)
     _need(positions, "positions", torch.int32, 1)
+    mask = mask_rule(window, chunk)
+    # as in the entry point: where portions go in tiles, the rows that are alone in theirs follow in a second kernel
+    tiled = (portions and mask == 0 and N * n_heads >= 2048 and d % 4 == 0 and d <= 128 and n_heads <= 65535
+             and cache.data_ptr() % (4 * cache.element_size()) == 0)
     _check(lib.tnx_attention_simt(_p(q), c_int(q_stride), _p(cache), _p(block_tables), c_int(block_tables.stride(0)),
                                   _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(N),
-                                  c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask_rule(window, chunk)),
+                                  c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask),
                                   c_float(scale), *_score_options(keep_first, bias, sink, n_heads, window),
-                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), _stream()), "attention_simt")
+                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), _stream()), "attention_simt", 2 if tiled else 1)
 
 
 def sample(logits, out, temperature=None, top_k=None, top_p=None, seeds=None, counters=None, suppress_id=-1,
@@ -1394,7 +1399,7 @@ def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_he
         adds = torch.empty(states + states // (v_dim * k_dim), dtype=torch.float32, device=q.device)
         _check(chunk_lib.tnx_retention_chunked(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                                _p(state_slots), _p(out), c_int(N), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
-                                               c_int(_is_h16(v)), _p(adds), c_void_p(adds.data_ptr() + 4 * states), _stream()), "retention_scan")
+                                               c_int(_is_h16(v)), _p(adds), c_void_p(adds.data_ptr() + 4 * states), _stream()), "retention_scan", 3)
         return
     _check(lib.tnx_retention_scan(_p(q), _p(k), _p(v), c_int(v_ld), _p(decay), _p(state), _p(q_start), _p(q_len),
                                   _p(state_slots), _p(out), c_int(R), c_int(n_heads), c_int(k_dim), c_int(v_dim),
