@@ -1205,41 +1205,40 @@ def moe_grouped(ctx, h, gate_up, down, ids, weights, out, gate_max, up_min, up_m
     granule = 32 if tile == 256 else tile                    # of the rows; a tile of 256 takes as many granules as it needs
     granules = P // granule + min(P, E)
     rows = granules * granule
-    sizes = [tiles, granules, P] + ([tiles] if tile == 256 else [])
-    group_of_tile, rows_of_granule, row_of_pair, *span = ctx.scratch(1, sum(sizes), torch.int32).view(-1).split(sizes)
-    span_of_tile = span[0] if span else None
+    group_of_tile = ctx.scratch(1, tiles, torch.int32).view(-1)
+    span_of_tile = ctx.scratch(1, tiles, torch.int32).view(-1) if tile == 256 else None
+    plan = ctx.scratch(1, granules + P, torch.int32)         # how many of a granule's rows are pairs; every pair's row
     x = ctx.scratch(rows, W, h.dtype)
-    moe_sort_rows(lib, h, ids, weights, E, tile, group_of_tile, span_of_tile, rows_of_granule, row_of_pair, x, weight_on_input)
+    moe_sort_rows(lib, h, ids, weights, E, tile, group_of_tile, span_of_tile, plan, granules, x, weight_on_input)
     gu = ctx.scratch(rows, F2, h.dtype)
     gemm_tc_grouped(x, gate_up, gu, group_of_tile, tile, used, span_of_tile)
     y = ctx.scratch(rows, F, h.dtype)
-    moe_activation(lib, gu, y, rows_of_granule, granule, gate_max, up_min, up_max, alpha, up_shift, form)
+    moe_activation(lib, gu, y, plan, granule, gate_max, up_min, up_max, alpha, up_shift, form)
     per_pair = ctx.scratch(rows, W, torch.float32)
     gemm_tc_grouped(y, down, per_pair, group_of_tile, tile, used, span_of_tile)
-    moe_combine(lib, per_pair, h, row_of_pair, weights, out, accumulate, weight_on_input)
+    moe_combine(lib, per_pair, h, plan, granules, weights, out, accumulate, weight_on_input)
 
 
-def moe_sort_rows(lib, h, ids, weights, n_experts, tile, group_of_tile, span_of_tile, rows_of_granule, row_of_pair, x,
-                  weight_on_input):
+def moe_sort_rows(lib, h, ids, weights, n_experts, tile, group_of_tile, span_of_tile, plan, granules, x, weight_on_input):
     """The plan (every pair's row, every tile's expert and rows, how many of a granule's rows are pairs) and the rows
     themselves, x[row(pair)] = weight * h[token]."""
     P, top = ids.numel(), ids.shape[1]
-    _check(lib.tnx_moe_plan(_p(ids), c_int(P), c_int(n_experts), c_int(group_of_tile.shape[0]), c_int(rows_of_granule.shape[0]),
-                            c_int(tile), _p(group_of_tile), _p(span_of_tile), _p(rows_of_granule), _p(row_of_pair), _stream()),
-           "moe_plan")
-    _check(lib.tnx_moe_gather(_p(h), c_int(h.stride(0)), _p(weights), _p(row_of_pair), _p(x), c_int(P), c_int(h.shape[1]),
+    row_of_pair = c_void_p(plan.data_ptr() + 4 * granules)
+    _check(lib.tnx_moe_plan(_p(ids), c_int(P), c_int(n_experts), c_int(group_of_tile.shape[0]), c_int(granules),
+                            c_int(tile), _p(group_of_tile), _p(span_of_tile), _p(plan), row_of_pair, _stream()), "moe_plan")
+    _check(lib.tnx_moe_gather(_p(h), c_int(h.stride(0)), _p(weights), row_of_pair, _p(x), c_int(P), c_int(h.shape[1]),
                               c_int(top), c_int(1 if weight_on_input else 0), _stream()), "moe_gather")
 
 
-def moe_activation(lib, gu, y, rows_of_granule, granule, gate_max, up_min, up_max, alpha, up_shift, form="gated_swish"):
-    _check(lib.tnx_moe_act(_p(gu), _p(y), _p(rows_of_granule), c_int(granule), c_int(gu.shape[0]), c_int(y.shape[1]), c_float(gate_max),
+def moe_activation(lib, gu, y, plan, granule, gate_max, up_min, up_max, alpha, up_shift, form="gated_swish"):
+    _check(lib.tnx_moe_act(_p(gu), _p(y), _p(plan), c_int(granule), c_int(gu.shape[0]), c_int(y.shape[1]), c_float(gate_max),
                            c_float(up_min), c_float(up_max), c_float(alpha), c_float(up_shift), c_int(EXPERT_FORMS[form]),
                            _stream()), "moe_act")
 
 
-def moe_combine(lib, per_pair, h, row_of_pair, weights, out, accumulate, weight_on_input):
+def moe_combine(lib, per_pair, h, plan, granules, weights, out, accumulate, weight_on_input):
     N, W = out.shape
-    _check(lib.tnx_moe_combine(_p(per_pair), _p(h), c_int(h.stride(0)), _p(row_of_pair), _p(weights), _p(out), c_int(N), c_int(W), c_int(weights.shape[1]),
+    _check(lib.tnx_moe_combine(_p(per_pair), _p(h), c_int(h.stride(0)), c_void_p(plan.data_ptr() + 4 * granules), _p(weights), _p(out), c_int(N), c_int(W), c_int(weights.shape[1]),
                                c_int(1 if accumulate else 0), c_int(1 if weight_on_input else 0), _stream()), "moe_combine")
 
 
