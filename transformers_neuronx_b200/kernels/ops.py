@@ -1317,7 +1317,7 @@ def retention_prep(proj, q_off, k_off, token_request, positions, inv_freq, rot_d
         raise KernelError("the projection is narrower than its q/k columns")
     for t, nm in ((q_out, "q_out"), (k_out, "k_out")):
         _need(t, nm, torch.float32, 2)
-        if tuple(t.shape) != (N, n_heads * k_dim):
+        if t.shape != (N, n_heads * k_dim):
             raise KernelError(f"{nm} must be [{N}, {n_heads * k_dim}]")
     _f32_vec(inv_freq, "inv_freq", rot_dims // 2 if rot_dims else None)
     n_values = 0
@@ -1365,23 +1365,23 @@ def retention_scan(q, k, v, decay, state, q_start, q_len, state_slots, out, n_he
     for t, nm in ((decay_tok, "decay_tok"), (kscale_tok, "kscale_tok")):
         if t is not None:
             _need(t, nm, torch.float32, 2)
-            if tuple(t.shape) != (N, n_heads):
+            if t.shape != (N, n_heads):
                 raise KernelError(f"{nm} must be [{N}, {n_heads}]")
     if decay is None and decay_tok is None:
         raise KernelError("a decay per head or per token is needed")
     for t, nm in ((q, "q"), (k, "k")):
         _need(t, nm, torch.float32, 2)
-        if tuple(t.shape) != (N, qk_heads * k_dim):
+        if t.shape != (N, qk_heads * k_dim):
             raise KernelError(f"{nm} must be [{N}, {qk_heads * k_dim}]")
     _need(v, "v", _FLOATS, None, contiguous=False)
     Nv, wv, v_ld = _rows_2d(v, "v")
     if (Nv, wv) != (N, n_heads * v_dim):
         raise KernelError(f"v must be [{N}, {n_heads * v_dim}]")
     _need(state, "state", torch.float32, 4)
-    if tuple(state.shape[1:]) != (n_heads, v_dim, k_dim):
+    if state.shape[1:] != (n_heads, v_dim, k_dim):
         raise KernelError(f"state must be [slots, {n_heads}, {v_dim}, {k_dim}]")
     _need(out, "out", torch.float32, 2)
-    if tuple(out.shape) != (N, n_heads * v_dim):
+    if out.shape != (N, n_heads * v_dim):
         raise KernelError(f"out must be [{N}, {n_heads * v_dim}]")
     _f32_vec(decay, "decay", n_heads)
     for t, nm in ((q_start, "q_start"), (q_len, "q_len"), (state_slots, "state_slots")):
