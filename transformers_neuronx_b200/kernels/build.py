@@ -35,6 +35,7 @@ SOURCES: Dict[str, str] = {
     "embedding": "embedding.cu",
     "layernorm": "layernorm.cu",
     "gemm_simt": "gemm_simt.cu",
+    "gemm_split": "gemm_split.cu",
     "kv_cache": "kv_cache.cu",
     "attention_simt": "attention_simt.cu",
     "sampling": "sampling.cu",

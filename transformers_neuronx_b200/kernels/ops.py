@@ -240,6 +240,63 @@ def gemm_simt(a, w, out, bias=None, residual=None, activation=None):
                              c_int(_is_h16(w)), c_int(_is_h16(out)), _stream()), "gemm_simt")
 
 
+_split_scratch = {}                # (M, N, K, SMs) -> bytes of scratch memory, as the library plans them
+SPLIT_TERMS_BYTES = 64 << 20       # of scratch memory for the activations' terms in one call; longer inputs go in slices of rows
+
+
+def gemm_split_supported(a, w, out) -> bool:
+    """32-bit activations and a 16-bit matrix whose rows TMA can fetch.  The number of rows has no part in it, so that a row's
+    result does not depend on how many others a step holds.  Matrices below 256 columns or 128 rows stay on the multiply-add
+    units: 8 tokens by [256 x 256] take 6.2 us here and 8.4 there, below that two launches are what counts."""
+    return (a.dtype == torch.float32 and w.dtype in _H16 and (out.dtype == torch.float32 or out.dtype == w.dtype)
+            and w.shape[1] >= 256 and w.shape[0] >= 128 and w.shape[1] % 8 == 0 and w.stride(0) % 8 == 0
+            and w.data_ptr() % 16 == 0)
+
+
+def gemm_split(a, w, out, bias=None, residual=None, activation=None):
+    """out = epilogue(a @ w^T) for 32-bit activations and a 16-bit matrix on the tensor cores, the activations as the exact sum
+    of three 16-bit terms, 32-bit sums: no further from 64 bits than gemm_simt.  A row's result does not depend on the other
+    rows of the call."""
+    lib = _lib("gemm_split", w, out)
+    act = activation_code(activation)
+    _need(a, "a", torch.float32, None, contiguous=False)
+    _need(w, "w", _H16, None, contiguous=False)
+    _need(out, "out", _FLOATS, None, contiguous=False)
+    M, K, lda = _rows_2d(a, "a")
+    N, Kw, ldw = _rows_2d(w, "w")
+    Mo, No, ldc = _rows_2d(out, "out")
+    if Kw != K or Mo != M or No != N:
+        raise KernelError(f"gemm shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    if K % 8 or ldw % 8 or w.data_ptr() % 16:
+        raise KernelError("w needs K and its row pitch to be multiples of 8 elements and a 16-byte aligned base")
+    if bias is not None:
+        _need(bias, "bias", torch.float32, 1)
+        if bias.shape[0] != N:
+            raise KernelError("bias length differs from the output width")
+    if residual is not None:
+        _need(residual, "residual", torch.float32, None, contiguous=False)
+        if tuple(residual.shape) != (M, N) or _rows_2d(residual, "residual")[2] != ldc or out.dtype != torch.float32:
+            raise KernelError("residual must be float32 with the shape and row stride of a float32 out")
+    st = _state(a.device)
+    slice_rows = max(SPLIT_TERMS_BYTES // (6 * K) // 64, 1) * 64
+    for r in range(0, M, slice_rows):
+        m = min(slice_rows, M - r)
+        nbytes = _split_scratch.get((m, N, K, st["sms"]))
+        if nbytes is None:
+            lib.tnx_gemm_split_scratch.restype = ctypes.c_longlong
+            if len(_split_scratch) > 4096:
+                _split_scratch.clear()
+            nbytes = _split_scratch[(m, N, K, st["sms"])] = lib.tnx_gemm_split_scratch(c_int(m), c_int(N), c_int(K), c_int(st["sms"]))
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=a.device)
+        at = lambda t: c_void_p(0 if t is None else t.data_ptr() + r * t.stride(0) * t.element_size())
+        n = lib.tnx_gemm_split(at(a), _p(w), _p(bias), at(residual), at(out), c_int(m), c_int(N), c_int(K), c_int(lda),
+                               c_int(ldw), c_int(ldc), c_int(act), c_int(_is_h16(out)), c_int(st["sms"]), _p(scratch),
+                               _p(st["err"]), _stream())
+        if n < 0 or n > 1000:
+            _check(n if n < 0 else n - 1000, "gemm_split")
+        _check(0, "gemm_split", n)
+
+
 def kv_append(k_src, v_src, slot_mapping, cache, page_size):
     """k_src, v_src: [N, n_kv_heads * head_dim] views (rows contiguous, one row stride);
     cache: [pages, 2, n_kv_heads, page_size, head_dim]."""

@@ -34,7 +34,7 @@ class PagedAttention(Mixer):
 
     @property
     def libraries(self):
-        libs = ["gemm_simt", "gemm_tc", "gemv", "kv_cache", "attention_simt", "attention_prefill", "attention_prefill_tc", "attention_decode", "attention_decode_grouped"]
+        libs = ["gemm_simt", "gemm_split", "gemm_tc", "gemv", "kv_cache", "attention_simt", "attention_prefill", "attention_prefill_tc", "attention_decode", "attention_decode_grouped"]
         if self.position is not None:
             libs += list(self.position.libraries)
         return tuple(libs)

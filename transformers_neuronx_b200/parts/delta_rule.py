@@ -37,7 +37,7 @@ MAX_K_DIM = 256
 class DeltaRule(Mixer):
     graph_safe = True
     can_overwrite = True
-    libraries = ("gemm_simt", "gemm_tc", "gemv", "delta_rule", "conv_qkv", "retention")
+    libraries = ("gemm_simt", "gemm_split", "gemm_tc", "gemv", "delta_rule", "conv_qkv", "retention")
 
     def __init__(self, spec: DeltaRuleSpec):
         s = self.spec = spec

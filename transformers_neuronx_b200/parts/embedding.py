@@ -92,7 +92,7 @@ class StreamJoin(Part):
 
     @property
     def libraries(self):
-        return ("gemm_simt", "gemm_tc", "gemv", "layernorm")        # the last: a copy of the stream in the activation type
+        return ("gemm_simt", "gemm_split", "gemm_tc", "gemv", "layernorm")        # the last: a copy of the stream in the activation type
 
     def tensor_specs(self):
         w = self.spec.weight
@@ -129,7 +129,7 @@ class Head(Part):
 
     @property
     def libraries(self):
-        libs = ["gemm_simt", "gemm_tc", "gemv"]
+        libs = ["gemm_simt", "gemm_split", "gemm_tc", "gemv"]
         # without a final norm the rows are picked by a kernel of the LayerNorm library
         libs += list(self.final_norm.libraries) if self.final_norm is not None else ["layernorm"]
         return tuple(dict.fromkeys(libs))

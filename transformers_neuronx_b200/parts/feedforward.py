@@ -15,7 +15,7 @@ class DenseFeedForward(FeedForward):
     graph_safe = True
     takes_normed_input = True       # `h` only feeds fc1
     can_overwrite = True
-    libraries = ("gemm_simt", "gemm_tc", "gemv")
+    libraries = ("gemm_simt", "gemm_split", "gemm_tc", "gemv")
 
     def __init__(self, spec: DenseFeedForwardSpec):
         self.spec = spec
@@ -43,7 +43,7 @@ class GatedDenseFeedForward(FeedForward):
     activation and the multiplication one elementwise kernel in 32-bit on its output."""
     graph_safe = True
     can_overwrite = True
-    libraries = ("gemm_simt", "gemm_tc", "gemv", "gated_act")
+    libraries = ("gemm_simt", "gemm_split", "gemm_tc", "gemv", "gated_act")
 
     def __init__(self, spec: GatedFeedForwardSpec):
         self.spec = spec

@@ -52,7 +52,7 @@ class FusableMixer(Mixer):
 
     @property
     def libraries(self):
-        return ("gemm_simt", "gemm_tc", "gemv") + tuple(self.extra_libraries)
+        return ("gemm_simt", "gemm_split", "gemm_tc", "gemv") + tuple(self.extra_libraries)
 
     @property
     def inner_width(self) -> int:

@@ -41,7 +41,7 @@ class LatentAttention(Mixer):
     @property
     def libraries(self):
         prefill = "attention_prefill_tc" if self.pad_dim in (64, 80, 96, 112, 128) else "attention_prefill"
-        return ("gemm_simt", "gemm_tc", "gemv", "latent_attention", "kv_cache", "attention_simt", prefill,
+        return ("gemm_simt", "gemm_split", "gemm_tc", "gemv", "latent_attention", "kv_cache", "attention_simt", prefill,
                 "attention_decode", "attention_decode_grouped")
 
     def __init__(self, spec: LatentAttentionSpec):

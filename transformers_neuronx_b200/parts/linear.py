@@ -5,6 +5,7 @@ orientation and its stored type (parts/base.py: weight_to_device): a matrix stor
 
 Kernel choice: 16-bit activations with a matrix of the same 16-bit type go to the tcgen05 tensor-core
 kernel when its size rules hold (the row length in bytes a multiple of 16, for its TMA descriptors);
+32-bit activations with a 16-bit matrix go to the tensor cores as three exact 16-bit terms (all but small matrices);
 everything else goes to the CUDA-core kernel with 32-bit FMA accumulation.
 """
 from __future__ import annotations
@@ -30,7 +31,7 @@ class Linear(Part):
 
     @property
     def libraries(self):
-        return ("gemm_simt", "gemm_tc", "gemv")
+        return ("gemm_simt", "gemm_split", "gemm_tc", "gemv")
 
     def tensor_specs(self) -> List[TensorSpec]:
         s = self.spec
@@ -70,6 +71,8 @@ class Linear(Part):
 def linear_forward(a, weight, bias, out, residual=None, activation=None):
     if ops.gemm_tc_supported(a, weight, out):
         ops.gemm_tc(a, weight, out, bias=bias, residual=residual, activation=activation)
+    elif ops.gemm_split_supported(a, weight, out):
+        ops.gemm_split(a, weight, out, bias=bias, residual=residual, activation=activation)
     else:
         ops.gemm_simt(a, weight, out, bias=bias, residual=residual, activation=activation)
 

@@ -41,7 +41,7 @@ class RoutedExperts(FeedForward):
 
     @property
     def libraries(self):
-        apart = ("gated_act", "gemm_simt") if self.folded else ()
+        apart = ("gated_act", "gemm_simt", "gemm_split") if self.folded else ()
         return ("moe", "moe_grouped", "gemm_tc") + apart + (tuple(self.shared.libraries) if self.shared is not None and not self.folded else ())
 
     # Rows from which the grouped tensor-core form runs in a 16-bit engine.  Measured at width 2048 (8 experts of inner

@@ -36,7 +36,7 @@ MAX_STATE = 256
 class SelectiveScan(Mixer):
     graph_safe = True
     can_overwrite = True
-    libraries = ("gemm_simt", "gemm_tc", "gemv", "selective_scan", "conv_qkv")
+    libraries = ("gemm_simt", "gemm_split", "gemm_tc", "gemv", "selective_scan", "conv_qkv")
 
     def __init__(self, spec: SelectiveScanSpec):
         s = self.spec = spec

@@ -35,7 +35,7 @@ MAX_STATE = 256        # the scan keeps up to 256 rows of a column in a warp
 class SSD(Mixer):
     graph_safe = True
     can_overwrite = True
-    libraries = ("gemm_simt", "gemm_tc", "gemv", "ssd", "conv_qkv", "retention")
+    libraries = ("gemm_simt", "gemm_split", "gemm_tc", "gemv", "ssd", "conv_qkv", "retention")
 
     def __init__(self, spec: SSDSpec):
         s = self.spec = spec
