@@ -502,6 +502,20 @@ def test_attention_simt_portions_and_rows_agree(n_heads, n_kv, d, dtype, options
     assert rel_err(outs[0], want.to(DEV)) <= (1e-5 if dtype == torch.float32 else 1e-2)
 
 
+@pytest.mark.parametrize("d,n_heads,n_kv", [(64, 16, 4), (128, 16, 16), (20, 16, 2)])
+@pytest.mark.parametrize("lens", [[(0, 64), (3, 1), (700, 1), (5, 62)],              # a tile's last row, the first of the next, a row on the edge
+                                  [(9, 63), (130, 2), (40, 1), (0, 65), (300, 1)],   # a portion over an edge, another's single row left behind it
+                                  [(i * 11, 1) for i in range(70)] + [(64, 130)]])   # more single rows than a tile
+def test_attention_simt_tiles_edges(lens, d, n_heads, n_kv):
+    """Tiles of 64 rows and the rows that are alone in theirs, against the same rows one by one: the same bits."""
+    case = PagedCase(lens, n_heads, n_kv, d, torch.float32, seed=len(lens))
+    assert case.N * n_heads >= 2048
+    outs = [torch.zeros(case.N, n_heads * d, device=DEV) for _ in range(2)]
+    for out, portions in zip(outs, (True, False)):
+        ops().attention_simt(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, n_heads, 0.11, portions=portions)
+    assert torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("rows,window,kernels", [(103, 0, 2), (101, 0, 1), (103, 37, 1)])
 def test_attention_simt_counts_its_kernels(rows, window, kernels):
     """20 heads: from 2,048 (row, head) pairs on without a window two kernels run, else one."""

@@ -15,11 +15,12 @@
 //   rows    one block per (query token, head), heads of up to 128 dims: 64 or 128 keys and values at a time are staged in
 //           shared memory by all four warps; the dot products of the staged keys are formed side by side, the sums over the
 //           keys stay in their order.  It is a chain of stages: load, score, rescale, add.
-//   tiles   for portions of prompts without a mask: a block takes 32 neighbouring rows and one head, 64 staged keys and
+//   tiles   for portions of prompts without a mask: a block takes 64 neighbouring rows and one head, 64 staged keys and
 //           values serve all of them
 // Measured, 32 heads of 64, 32-bit: a portion of 499 tokens behind 256 beside three single rows of 500 to 700 keys, 2,417 us
-// with `wide` for all rows, 1,200 with `rows`, 279 with `tiles` and `rows`; four single rows of 100 to 900 keys 382 us with
-// `wide`, 53 with `rows`; 64 of 100 to 1,360 keys 1,106 and 434; a portion of 2,048 tokens, 16 heads of 128, 17.2 and 1.66 ms.
+// with `wide` for all rows, 1,200 with `rows`, 160 with `tiles` (in tiles of 32 rows with the single rows in a kernel of their own
+// after them 279); four single rows of 100 to 900 keys 382 us with `wide`, 53 with `rows`; 64 of 100 to 1,360 keys 1,106 and 434;
+// a portion of 2,048 tokens, 16 heads of 128, 0.60 ms (tiles of 32 rows 1.66).
 #include "common.cuh"
 
 namespace {
@@ -117,10 +118,10 @@ struct SimtParams {
     int keep_first;
     DistanceBias bias;
     SoftmaxSink sink;
-    int tiled;                           // the tiles kernel takes the rows that share their request within a tile
+    int page_shift;                      // page_size = 2^page_shift, or -1
 };
 
-constexpr int TILE_ROWS = 32;            // rows of a tile: tile t holds rows 32 t .. 32 t + 31 of the batch
+constexpr int TILE_ROWS = 64;            // rows of a tile: tile t holds rows 64 t .. 64 t + 63 of the batch
 
 __device__ __forceinline__ float4 load4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 load4(const h16* p) {
@@ -129,267 +130,374 @@ __device__ __forceinline__ float4 load4(const h16* p) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// The rows kernel: 128 threads a (row, head).  With `tiled`, blockIdx.x names a tile and one of its SLOTS: the block takes
-// every SLOTS-th of the rows that are alone with their request in that tile, which the tiles kernel leaves.
-constexpr int SLOTS = 8;
-template <typename T, int KEYS>
-__global__ void __launch_bounds__(128)
-attention_simt_rows_kernel(const SimtParams<T> p) {
-    extern __shared__ __align__(16) float sm[];
+// One row and one head by a block of THREADS (a multiple of 32, and no fewer than KEYS and the head's dims).
+template <typename T, int KEYS, int THREADS>
+__device__ __forceinline__ void attend_row(const SimtParams<T>& p, float* sm, int n, int h) {
     const int d = p.head_dim, d4 = d / 4;
     float* ks = sm;                                 // [KEYS][d + 4]: a warp's 16-byte reads down the rows meet all banks evenly
     float* vs = ks + KEYS * (d + 4);                // [KEYS][d]
     float* qs = vs + KEYS * d;                      // [d]
     float* ss = qs + d;                             // [KEYS] the staged keys' scores
-    pdl_launch_dependents();
-    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31;
-    const int h = blockIdx.y, kvh = h / (p.n_heads / p.n_kv_heads);
+    const int kvh = h / (p.n_heads / p.n_kv_heads);
     const size_t head_block = (size_t)p.page_size * d;
     const float mul = p.bias.mul ? p.bias.mul[h] : 0.f, rate = p.bias.mul ? p.bias.rate[h] : 0.f;
-    unsigned todo = 1;                              // bit r: row row0 + r is still to do (the same in every thread)
-    int row0 = blockIdx.x;
-    if (p.tiled) {
-        row0 = blockIdx.x / SLOTS * TILE_ROWS;
-        const int mine = row0 + lane < p.n_tokens ? p.token_request[row0 + lane] : -1;
-        bool alone = mine >= 0;
-        for (int i = 0; i < TILE_ROWS; ++i) {
-            const int other = __shfl_sync(0xffffffffu, mine, i);
-            alone = alone && (i == lane || other != mine);
-        }
-        todo = __ballot_sync(0xffffffffu, alone);
-        const int place = __popc(todo & ((1u << lane) - 1));
-        todo = __ballot_sync(0xffffffffu, alone && place % SLOTS == (int)blockIdx.x % SLOTS);
-    }
-    for (; todo; todo &= todo - 1) {
-        const int n = row0 + __ffs(todo) - 1;
-        const int req = p.token_request[n];
-        if (req < 0) continue;                      // a padded row of a captured batch
-        const int pos = p.positions[n];
-        const int* bt = p.block_tables + (size_t)req * p.bt_stride;
-        // the visible keys, numbered without the gap between the first ones that are kept and the window
-        const int first = first_visible_key(pos, p.window);
-        const int kept = p.keep_first < first ? p.keep_first : first, gap = first - kept;
-        const int n_keys = pos + 1 - gap;
-        float m = p.sink.on ? p.sink.score : -INFINITY, l = p.sink.on ? 1.f : 0.f, acc = 0.f;
-        const bool has_dim = tid < d;               // the thread owns dim `tid` of the output
-        for (int k0 = 0; k0 < n_keys; k0 += KEYS) {
-            const int staged = min(KEYS, n_keys - k0);
-            __syncthreads();                        // the keys before are done with
-            if (k0 == 0)
-                for (int c = tid; c < d; c += 128) qs[c] = to_float(p.q[(size_t)n * p.q_stride + (size_t)h * d + c]);
+    const int req = p.token_request[n];
+    if (req < 0) return;                            // a padded row of a captured batch
+    const int pos = p.positions[n];
+    const int* bt = p.block_tables + (size_t)req * p.bt_stride;
+    // the visible keys, numbered without the gap between the first ones that are kept and the window
+    const int first = first_visible_key(pos, p.window);
+    const int kept = p.keep_first < first ? p.keep_first : first, gap = first - kept;
+    const int n_keys = pos + 1 - gap;
+    float m = p.sink.on ? p.sink.score : -INFINITY, l = p.sink.on ? 1.f : 0.f, acc = 0.f;
+    const bool has_dim = tid < d;               // the thread owns dim `tid` of the output
+    for (int k0 = 0; k0 < n_keys; k0 += KEYS) {
+        const int staged = min(KEYS, n_keys - k0);
+        __syncthreads();                        // the keys before are done with
+        if (k0 == 0)
+            for (int c = tid; c < d; c += THREADS) qs[c] = to_float(p.q[(size_t)n * p.q_stride + (size_t)h * d + c]);
 #pragma unroll 8
-            for (int i = tid; i < staged * d4; i += 128) {
-                const int kk = i / d4, c = (i % d4) * 4, i_key = k0 + kk, j = i_key < kept ? i_key : i_key + gap;
-                const T* krow = p.cache + ((size_t)bt[j / p.page_size] * 2 * p.n_kv_heads + kvh) * head_block
-                                + (size_t)(j % p.page_size) * d + c;
-                *(float4*)(ks + kk * (d + 4) + c) = load4(krow);
-                *(float4*)(vs + kk * d + c) = load4(krow + (size_t)p.n_kv_heads * head_block);
-            }
-            __syncthreads();
-            if (tid < staged) {
-                const float* kr = ks + tid * (d + 4);
-                float dot = 0.f;
+        for (int i = tid; i < staged * d4; i += THREADS) {
+            const int kk = i / d4, c = (i % d4) * 4, i_key = k0 + kk, j = i_key < kept ? i_key : i_key + gap;
+            const T* krow = p.cache + ((size_t)bt[j / p.page_size] * 2 * p.n_kv_heads + kvh) * head_block
+                            + (size_t)(j % p.page_size) * d + c;
+            *(float4*)(ks + kk * (d + 4) + c) = load4(krow);
+            *(float4*)(vs + kk * d + c) = load4(krow + (size_t)p.n_kv_heads * head_block);
+        }
+        __syncthreads();
+        if (tid < staged) {
+            const float* kr = ks + tid * (d + 4);
+            float dot = 0.f;
 #pragma unroll 4
-                for (int c = 0; c < d; c += 4) {
-                    const float4 k4 = *(const float4*)(kr + c), q4 = *(const float4*)(qs + c);
-                    dot = fmaf(q4.x, k4.x, dot); dot = fmaf(q4.y, k4.y, dot);
-                    dot = fmaf(q4.z, k4.z, dot); dot = fmaf(q4.w, k4.w, dot);
-                }
-                float s = dot * p.scale;
-                const int i_key = k0 + tid, j = i_key < kept ? i_key : i_key + gap;
-                if (p.bias.mul) s -= mul * log1pf(rate * (float)(pos - j));
-                ss[tid] = s;
+            for (int c = 0; c < d; c += 4) {
+                const float4 k4 = *(const float4*)(kr + c), q4 = *(const float4*)(qs + c);
+                dot = fmaf(q4.x, k4.x, dot); dot = fmaf(q4.y, k4.y, dot);
+                dot = fmaf(q4.z, k4.z, dot); dot = fmaf(q4.w, k4.w, dot);
             }
-            __syncthreads();
-            for (int c0 = 0; c0 < staged; c0 += 32) {               // every warp keeps the running maximum and sum for itself
-                const int cnt = min(32, staged - c0);
-                const float s = lane < cnt ? ss[c0 + lane] : -INFINITY;
-                const float m_new = fmaxf(m, warp_max(s));
-                const float e = lane < cnt ? expf(s - m_new) : 0.f;
-                const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
-                l = l * corr + warp_sum(e);
-                m = m_new;
-                acc *= corr;
-                const float* vr = vs + c0 * d + tid;
-                if (cnt == 32) {
+            float s = dot * p.scale;
+            const int i_key = k0 + tid, j = i_key < kept ? i_key : i_key + gap;
+            if (p.bias.mul) s -= mul * log1pf(rate * (float)(pos - j));
+            ss[tid] = s;
+        }
+        __syncthreads();
+        for (int c0 = 0; c0 < staged; c0 += 32) {               // every warp keeps the running maximum and sum for itself
+            const int cnt = min(32, staged - c0);
+            const float s = lane < cnt ? ss[c0 + lane] : -INFINITY;
+            const float m_new = fmaxf(m, warp_max(s));
+            const float e = lane < cnt ? expf(s - m_new) : 0.f;
+            const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
+            l = l * corr + warp_sum(e);
+            m = m_new;
+            acc *= corr;
+            const float* vr = vs + c0 * d + tid;
+            if (cnt == 32) {
 #pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        const float pj = __shfl_sync(0xffffffffu, e, jj);
-                        if (has_dim) acc = fmaf(pj, vr[jj * d], acc);
-                    }
-                } else {
-                    for (int jj = 0; jj < cnt; ++jj) {
-                        const float pj = __shfl_sync(0xffffffffu, e, jj);
-                        if (has_dim) acc = fmaf(pj, vr[jj * d], acc);
-                    }
+                for (int jj = 0; jj < 32; ++jj) {
+                    const float pj = __shfl_sync(0xffffffffu, e, jj);
+                    if (has_dim) acc = fmaf(pj, vr[jj * d], acc);
+                }
+            } else {
+                for (int jj = 0; jj < cnt; ++jj) {
+                    const float pj = __shfl_sync(0xffffffffu, e, jj);
+                    if (has_dim) acc = fmaf(pj, vr[jj * d], acc);
                 }
             }
         }
-        if (has_dim) p.out[(size_t)n * p.out_stride + (size_t)h * d + tid] = from_float<T>(acc * (1.0f / l));
     }
+    if (has_dim) p.out[(size_t)n * p.out_stride + (size_t)h * d + tid] = from_float<T>(acc * (1.0f / l));
 }
 
-// The tiles kernel.  Grid (tiles, heads), four warps of eight rows.  The requests that have two rows and more in the tile
-// are taken one after the other (nearly always there is one); rows of other requests idle meanwhile.
-//   scores   a lane owns keys `lane` and `lane + 32` of the 64 staged, the row's q comes as a broadcast: two 16-byte
-//            shared-memory reads of keys and eight of q feed 64 multiply-adds
-//   values   a lane owns dims lane, lane + 32, ..; the row's probabilities come as a broadcast
-// It is bound by those reads (16 bytes a thread take a warp four cycles, broadcast or not).  A row's own 32-key steps
-// (maximum, sum, rescaling) are those of the other kernels.
-template <typename T, int DPL>
+template <typename T, int KEYS>
 __global__ void __launch_bounds__(128)
-attention_simt_tiles_kernel(const SimtParams<T> p) {
-    constexpr int KEYS = 64, RPW = TILE_ROWS / 4;
+attention_simt_rows_kernel(const SimtParams<T> p) {
     extern __shared__ __align__(16) float sm[];
-    const int d = p.head_dim;
-    float* qs = sm;                                 // [TILE_ROWS][d]
-    float* ks = qs + TILE_ROWS * d;                 // [KEYS][d + 4]
-    float* vs = ks + KEYS * (d + 4);                // [KEYS][d]
-    float* ps = vs + KEYS * d;                      // [TILE_ROWS][32]
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TILE_ROWS, h = blockIdx.y;     // later rows have more keys: first
+    attend_row<T, KEYS, 128>(p, sm, blockIdx.x, blockIdx.y);
+}
+
+// The rows that are alone with their request in their tile: list[0] of them, list[1 ..].  One block.
+__global__ void __launch_bounds__(1024)
+attention_simt_lone_list_kernel(const int* __restrict__ token_request, int n_tokens, int* __restrict__ list) {
+    __shared__ int count;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    for (long long row0 = warp * TILE_ROWS; row0 < n_tokens; row0 += 32 * TILE_ROWS) {       // a tile a warp
+        auto req_at = [&](long long n) { return n < n_tokens ? token_request[n] : -1; };
+        const int a = req_at(row0 + lane), b = req_at(row0 + 32 + lane), lead = __shfl_sync(0xffffffffu, a, 0);
+        if (__all_sync(0xffffffffu, a == lead && b == lead)) continue;             // one request's rows, as nearly always
+        int same_a = 0, same_b = 0;
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+            const int oa = __shfl_sync(0xffffffffu, a, i), ob = __shfl_sync(0xffffffffu, b, i);
+            same_a += (oa == a) + (ob == a); same_b += (oa == b) + (ob == b);
+        }
+        if (a >= 0 && same_a == 1) list[1 + atomicAdd(&count, 1)] = (int)row0 + lane;
+        if (b >= 0 && same_b == 1) list[1 + atomicAdd(&count, 1)] = (int)row0 + 32 + lane;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) list[0] = count;
+}
+
+// The tiles kernel.  Grid (heads, tiles and lone blocks): blocks of like length lie side by side, so the SMs get like shares.
+// A tile's requests with two rows and more in it are taken one after the other (nearly always there is one); rows of other
+// requests idle meanwhile.  64 keys and values are staged at a time:
+//   scores   a thread owns PR rows and PK keys: PR + PK 16-byte reads of shared memory feed 4 PR PK multiply-adds, in the order
+//            of the dims; they go to shared memory
+//   softmax  a thread owns a row's 32-key step (maximum, sum, rescaling: those of the other kernels)
+//   values   a thread owns PV_ROWS rows and four dims, the keys in their order
+// The rows that are alone with their request in their tile go to `lone` blocks of every head, a row a block at a time, which come
+// after the first tiles, about one an SM, and work beside them.
+// It starts while the kernel that lists those rows runs (which was launched in order, so what both read is there), and waits for
+// that one's end only where it reads the list and before it writes.
+// Of a stage's 17,800 cycles (heads of 64, two blocks an SM) the scores take 6,000, the values 5,000, the softmax 3,500 and the
+// wait for the keys 3,000; half of the issue slots are used, and the SMs' shares are uneven (256 blocks, 12 to 5 stages long).
+template <typename T, int DIMS, int THREADS>
+__global__ void __launch_bounds__(THREADS, DIMS == 64 ? 4 : 2)
+attention_simt_tiles_kernel(const SimtParams<T> p, const int* list, int lone, int first_tiles, int at_once) {
+    constexpr int KEYS = 64;
+    constexpr int DG = DIMS / 4;                                  // groups of four dims
+    constexpr int PV_ROWS = TILE_ROWS * DG / THREADS, RG_V = TILE_ROWS / PV_ROWS;      // thread: rows rv, rv + RG_V, ..; dims 4 dv ..
+    constexpr int PK = 4, KG = KEYS / PK, RG = THREADS / KG, PR = TILE_ROWS / RG;      // thread: rows rq, rq + RG, ..; keys kq, kq + KG, ..
+    const int SP = max(p.head_dim, KEYS) + 4;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ int reqs[TILE_ROWS], poss[TILE_ROWS], keys_of[TILE_ROWS];
+    __shared__ float corr_of[2][TILE_ROWS], m_of[TILE_ROWS], l_of[TILE_ROWS];
+    __shared__ int most_of[TILE_ROWS], least_of[TILE_ROWS];
+    __shared__ unsigned leads_of[2];
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.x;
+    const int tiles = (int)gridDim.y - lone;
+    int tile = (int)blockIdx.y;
+    if (tile >= first_tiles && tile < first_tiles + lone) {
+        pdl_wait();
+        const int count = *(const volatile int*)list;
+        for (int i = tile - first_tiles; i < count; i += lone) attend_row<T, 64, THREADS>(p, sm, ((const volatile int*)list)[1 + i], h);
+        return;
+    }
+    // The tiles with the most keys first; where all blocks are on the GPU at once, those after the first round of it from the
+    // fewest on, so that an SM's blocks add up to like sums.
+    if (tile < first_tiles) tile = tiles - 1 - tile;
+    else { tile -= first_tiles + lone; if (!at_once) tile = tiles - first_tiles - 1 - tile; }
+    const int d = p.head_dim, d4 = d / 4, dp = d + 4;
+    float* qs = sm;                                 // [TILE_ROWS][d + 4]
+    float* ks = qs + TILE_ROWS * dp;                // [KEYS][d + 4]
+    float* vs = ks + KEYS * SP;                     // [KEYS][d]
+    float* ps = ks;                                 // [TILE_ROWS][KEYS + 4]: scores, then probabilities, over the keys once these are used
+    const int row0 = tile * TILE_ROWS;
     const int kvh = h / (p.n_heads / p.n_kv_heads);
-    const int my_n = row0 + lane;
-    const int my_req = my_n < p.n_tokens ? p.token_request[my_n] : -1;
-    const int my_pos = my_n < p.n_tokens ? p.positions[my_n] : 0;
     const size_t head_block = (size_t)p.page_size * d;
     const float mul = p.bias.mul ? p.bias.mul[h] : 0.f, rate = p.bias.mul ? p.bias.rate[h] : 0.f;
-    const int d4 = d / 4;
-    unsigned todo = __ballot_sync(0xffffffffu, my_req >= 0);
-    while (todo) {                                  // the same for every warp of the block
-        const int lead = __ffs(todo) - 1;
-        const int req = __shfl_sync(0xffffffffu, my_req, lead);
-        const unsigned mine = __ballot_sync(0xffffffffu, my_req == req);
-        todo &= ~mine;
-        if (!(mine & (mine - 1))) continue;         // a request's only row here: the rows kernel's
-        int most = my_req == req ? my_pos + 1 : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    if (tid < TILE_ROWS) {
+        const int n = row0 + tid;
+        reqs[tid] = n < p.n_tokens ? p.token_request[n] : -1;
+        poss[tid] = n < p.n_tokens ? p.positions[n] : 0;
+    }
+    __syncthreads();
+    if (tid < TILE_ROWS) {                           // the requests' first rows, and the most and the fewest keys of their rows
+        const int req = reqs[tid];
+        int most = 0, least = 0x7fffffff, count = 0;
+        bool first = req >= 0;
+#pragma unroll 8
+        for (int i = 0; i < TILE_ROWS; ++i) {
+            if (reqs[i] != req) continue;
+            if (i < tid) first = false;
+            most = max(most, poss[i] + 1); least = min(least, poss[i] + 1); ++count;
+        }
+        most_of[tid] = most; least_of[tid] = least;
+        const unsigned leads = __ballot_sync(0xffffffffu, first && count > 1);     // a request's only row is a lone block's
+        if (lane == 0) leads_of[warp] = leads;
+    }
+    __syncthreads();
+    const int rq = tid / KG, kq = tid % KG, rv = tid / DG, dv = tid % DG;
+    const bool has_dims = 4 * dv < d;
+    for (unsigned long long todo = leads_of[0] | (unsigned long long)leads_of[1] << 32; todo; todo &= todo - 1) {      // the same for every thread
+        const int lead = __ffsll((long long)todo) - 1;
+        const int req = reqs[lead], most = most_of[lead], least = least_of[lead];
         const int* bt = p.block_tables + (size_t)req * p.bt_stride;
-        __syncthreads();                            // the request before is done with q
-        for (int i = tid; i < TILE_ROWS * d4; i += 128) {
+        __syncthreads();                            // the request before is done with q and the rows' numbers
+        if (tid < TILE_ROWS) {
+            keys_of[tid] = reqs[tid] == req ? poss[tid] + 1 : 0;
+            m_of[tid] = p.sink.on ? p.sink.score : -INFINITY;
+            l_of[tid] = p.sink.on ? 1.f : 0.f;
+        }
+        for (int i = tid; i < TILE_ROWS * d4; i += THREADS) {
             const int r = i / d4, c = (i % d4) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (mine >> r & 1) {
+            if (reqs[r] == req) {
                 const T* src = p.q + (size_t)(row0 + r) * p.q_stride + (size_t)h * d + c;
                 v = make_float4(to_float(src[0]), to_float(src[1]), to_float(src[2]), to_float(src[3]));
             }
-            *(float4*)(qs + r * d + c) = v;
+            *(float4*)(qs + r * dp + c) = v;
         }
-        float m[RPW], l[RPW], acc[RPW][DPL];
-        int n_keys[RPW];
+        float4 acc[PV_ROWS];
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const int row = warp * RPW + r, at = __shfl_sync(0xffffffffu, my_pos, row);
-            n_keys[r] = (mine >> row & 1) ? at + 1 : 0;
-            m[r] = p.sink.on ? p.sink.score : -INFINITY; l[r] = p.sink.on ? 1.f : 0.f;
-#pragma unroll
-            for (int i = 0; i < DPL; ++i) acc[r][i] = 0.f;
-        }
-        int warp_keys = 0;
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) warp_keys = max(warp_keys, n_keys[r]);
+        for (int r = 0; r < PV_ROWS; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int k0 = 0; k0 < most; k0 += KEYS) {
             __syncthreads();                        // the keys before are done with
-            for (int i = tid; i < KEYS * d4; i += 128) {
-                const int kk = i / d4, c = (i % d4) * 4, j = k0 + kk;
-                float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;
-                if (j < most) {
-                    const T* krow = p.cache + ((size_t)bt[j / p.page_size] * 2 * p.n_kv_heads + kvh) * head_block
-                                    + (size_t)(j % p.page_size) * d + c;
-                    k4 = load4(krow);
-                    v4 = load4(krow + (size_t)p.n_kv_heads * head_block);
+            // thread: dims 4 dv .. of keys rv, rv + THREADS / DG, ..; 32-bit pages are copied without passing through registers, the
+            // values still on their way while the scores are formed
+#pragma unroll
+            for (int which = 0; which < 2; ++which) {
+#pragma unroll 8
+                for (int it = 0; it < KEYS * DG / THREADS; ++it) {
+                    const int kk = rv + it * (THREADS / DG), j = min(k0 + kk, most - 1);     // (keys beyond: some key's numbers, none looks at them)
+                    const int page = p.page_shift >= 0 ? j >> p.page_shift : j / p.page_size, at = j - page * p.page_size;
+                    const T* src = p.cache + (((size_t)bt[page] * 2 + which) * p.n_kv_heads + kvh) * head_block + (size_t)at * d + 4 * dv;
+                    float* dst = (which ? vs + kk * d : ks + kk * dp) + 4 * dv;
+                    if (!has_dims) continue;
+                    if constexpr (sizeof(T) == 4) {
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+                    } else {
+                        *(float4*)dst = load4(src);
+                    }
                 }
-                *(float4*)(ks + kk * (d + 4) + c) = k4;
-                *(float4*)(vs + kk * d + c) = v4;
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            {
+                float s[PR][PK];
+#pragma unroll
+                for (int r = 0; r < PR; ++r)
+#pragma unroll
+                    for (int k = 0; k < PK; ++k) s[r][k] = 0.f;
+                const float *qr = qs + rq * dp, *kr = ks + kq * dp;
+#pragma unroll 2
+                for (int c = 0; c < d; c += 4) {
+                    float4 b[PK];
+#pragma unroll
+                    for (int k = 0; k < PK; ++k) b[k] = *(const float4*)(kr + k * KG * dp + c);
+#pragma unroll
+                    for (int r = 0; r < PR; ++r) {
+                        const float4 a = *(const float4*)(qr + r * RG * dp + c);
+#pragma unroll
+                        for (int k = 0; k < PK; ++k) {
+                            s[r][k] = fmaf(a.x, b[k].x, s[r][k]); s[r][k] = fmaf(a.y, b[k].y, s[r][k]);
+                            s[r][k] = fmaf(a.z, b[k].z, s[r][k]); s[r][k] = fmaf(a.w, b[k].w, s[r][k]);
+                        }
+                    }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < PR; ++r)
+#pragma unroll
+                    for (int k = 0; k < PK; ++k) ps[(rq + r * RG) * SP + kq + k * KG] = s[r][k];
             }
             __syncthreads();
-            if (k0 >= warp_keys) continue;
-            float s0[RPW], s1[RPW];
+            if (tid < 2 * TILE_ROWS) {
+                // A thread takes a row's 32-key step; the sum over its keys is the tree that a warp's exchanges form in the other
+                // kernels.  Steps beyond a row's keys leave its numbers as they are.  (With a lane a key and a warp a row this took
+                // twice as long as the scores: 9,000 cycles of a stage's 24,000.)
+                const int row = tid >> 1, half = tid & 1, n_keys = keys_of[row], first = k0 + 32 * half;
+                float* pr = ps + row * SP + 32 * half;
+                float e[32], top = -INFINITY, scale = p.scale;
+                if (p.bias.mul) {                                // apart, so that the loops below stay short
+#pragma unroll 1
+                    for (int i = 0; i < 32; ++i)
+                        pr[i] = fmaf(-mul, log1pf(rate * (float)(n_keys - 1 - first - i)), __fmul_rn(pr[i], scale));    // rounded as in the other kernels
+                    scale = 1.f;
+                }
 #pragma unroll
-            for (int r = 0; r < RPW; ++r) s0[r] = s1[r] = 0.f;
-            const float *ka = ks + lane * (d + 4), *kb = ka + 32 * (d + 4), *qw = qs + warp * RPW * d;
-#pragma unroll 2
-            for (int c = 0; c < d; c += 4) {
-                const float4 a = *(const float4*)(ka + c), b = *(const float4*)(kb + c);
+                for (int i = 0; i < 32; i += 4) { const float4 v = *(const float4*)(pr + i); e[i] = v.x; e[i + 1] = v.y; e[i + 2] = v.z; e[i + 3] = v.w; }
 #pragma unroll
-                for (int r = 0; r < RPW; ++r) {
-                    const float4 q = *(const float4*)(qw + r * d + c);
-                    s0[r] = fmaf(q.x, a.x, s0[r]); s0[r] = fmaf(q.y, a.y, s0[r]);
-                    s0[r] = fmaf(q.z, a.z, s0[r]); s0[r] = fmaf(q.w, a.w, s0[r]);
-                    s1[r] = fmaf(q.x, b.x, s1[r]); s1[r] = fmaf(q.y, b.y, s1[r]);
-                    s1[r] = fmaf(q.z, b.z, s1[r]); s1[r] = fmaf(q.w, b.w, s1[r]);
+                for (int i = 0; i < 32; ++i) {
+                    e[i] *= scale;
+                    if (first + i >= n_keys) e[i] = -INFINITY;
+                    top = fmaxf(top, e[i]);
+                }
+                const float m_old = m_of[row], l_old = l_of[row];
+                const float top0 = __shfl_sync(0xffffffffu, top, lane & 30), top1 = __shfl_sync(0xffffffffu, top, lane | 1);
+                const float m0 = fmaxf(m_old, top0), m1 = fmaxf(m0, top1), m_before = half ? m0 : m_old, m_new = half ? m1 : m0;
+                const float corr = (m_before == -INFINITY) ? 0.f : expf(m_before - m_new);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) e[i] = (first + i < n_keys) ? expf(e[i] - m_new) : 0.f;
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) *(float4*)(pr + i) = make_float4(e[i], e[i + 1], e[i + 2], e[i + 3]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < o; ++i) e[i] += e[i + o];
+                const float corr0 = __shfl_sync(0xffffffffu, corr, lane & 30), sum0 = __shfl_sync(0xffffffffu, e[0], lane & 30);
+                corr_of[half][row] = corr;
+                if (half) {
+                    const float l0 = l_old * corr0 + sum0;
+                    l_of[row] = l0 * corr + e[0];
+                    m_of[row] = m1;
                 }
             }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (has_dims) {
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int c0 = k0 + 32 * half, i = c0 + lane;
-                bool whole = true;                  // every row of the warp that is at work sees all 32 keys
+                for (int half = 0; half < 2; ++half) {
+                    const int c0 = k0 + 32 * half;
+                    if (c0 >= most) break;
+                    const float* vr = vs + 32 * half * d + 4 * dv;
+                    const float* pr = ps + rv * SP + 32 * half;
 #pragma unroll
-                for (int r = 0; r < RPW; ++r) {
-                    const int cnt = n_keys[r] - c0;
-                    whole = whole && (cnt >= 32 || n_keys[r] == 0);
-                    if (cnt <= 0) continue;         // the same for the whole warp
-                    float s = (half ? s1[r] : s0[r]) * p.scale;
-                    if (p.bias.mul) s -= mul * log1pf(rate * (float)(n_keys[r] - 1 - i));
-                    if (i >= n_keys[r]) s = -INFINITY;
-                    const float m_new = fmaxf(m[r], warp_max(s));
-                    const float e = (i < n_keys[r]) ? expf(s - m_new) : 0.f;
-                    const float corr = (m[r] == -INFINITY) ? 0.f : expf(m[r] - m_new);
-                    l[r] = l[r] * corr + warp_sum(e);
-                    m[r] = m_new;
+                    for (int r = 0; r < PV_ROWS; ++r) {
+                        const float corr = corr_of[half][rv + r * RG_V];
+                        acc[r].x *= corr; acc[r].y *= corr; acc[r].z *= corr; acc[r].w *= corr;
+                    }
+                    if (c0 + 32 <= least) {                      // every row at work sees all 32 keys
+#pragma unroll 2
+                        for (int jj = 0; jj < 32; jj += 4) {
+                            float4 v[4];
 #pragma unroll
-                    for (int x = 0; x < DPL; ++x) acc[r][x] *= corr;
-                    ps[(warp * RPW + r) * 32 + lane] = e;
-                }
-                __syncwarp();
-                const float* vrow = vs + 32 * half * d + lane;
-                if (whole && c0 < warp_keys) {
-                    for (int jj = 0; jj < 32; jj += 4) {
-                        float v[4][DPL];
+                            for (int u = 0; u < 4; ++u) v[u] = *(const float4*)(vr + (jj + u) * d);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
+                            for (int r = 0; r < PV_ROWS; ++r) {
+                                const float4 e = *(const float4*)(pr + r * RG_V * SP + jj);
+                                const float w[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
-                            for (int x = 0; x < DPL; ++x) v[u][x] = lane + 32 * x < d ? vrow[(jj + u) * d + 32 * x] : 0.f;
+                                for (int u = 0; u < 4; ++u) {
+                                    acc[r].x = fmaf(w[u], v[u].x, acc[r].x); acc[r].y = fmaf(w[u], v[u].y, acc[r].y);
+                                    acc[r].z = fmaf(w[u], v[u].z, acc[r].z); acc[r].w = fmaf(w[u], v[u].w, acc[r].w);
+                                }
+                            }
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int jj = 0; jj < 32; jj += 4) {
+                            float4 v[4];
 #pragma unroll
-                        for (int r = 0; r < RPW; ++r) {
-                            if (n_keys[r] == 0) continue;
-                            const float4 e = *(const float4*)(ps + (warp * RPW + r) * 32 + jj);
+                            for (int u = 0; u < 4; ++u) v[u] = *(const float4*)(vr + (jj + u) * d);
 #pragma unroll
-                            for (int x = 0; x < DPL; ++x) {
-                                acc[r][x] = fmaf(e.x, v[0][x], acc[r][x]); acc[r][x] = fmaf(e.y, v[1][x], acc[r][x]);
-                                acc[r][x] = fmaf(e.z, v[2][x], acc[r][x]); acc[r][x] = fmaf(e.w, v[3][x], acc[r][x]);
+                            for (int r = 0; r < PV_ROWS; ++r) {
+                                const int cnt = keys_of[rv + r * RG_V] - c0 - jj;
+                                const float4 e = *(const float4*)(pr + r * RG_V * SP + jj);
+                                const float w[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {    // a key that the row does not see may hold anything
+                                    if (u >= cnt) continue;
+                                    acc[r].x = fmaf(w[u], v[u].x, acc[r].x); acc[r].y = fmaf(w[u], v[u].y, acc[r].y);
+                                    acc[r].z = fmaf(w[u], v[u].z, acc[r].z); acc[r].w = fmaf(w[u], v[u].w, acc[r].w);
+                                }
                             }
                         }
                     }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < RPW; ++r) {
-                        const int cnt = min(32, n_keys[r] - c0);
-                        for (int jj = 0; jj < cnt; ++jj) {
-                            const float e = ps[(warp * RPW + r) * 32 + jj];
-#pragma unroll
-                            for (int x = 0; x < DPL; ++x)
-                                if (lane + 32 * x < d) acc[r][x] = fmaf(e, vrow[jj * d + 32 * x], acc[r][x]);
-                        }
-                    }
                 }
-                __syncwarp();
             }
         }
+        pdl_wait();                                 // (returns at once from the second request on)
+        if (has_dims) {
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            if (n_keys[r] == 0) continue;
-            const float inv = 1.0f / l[r];
-            T* orow = p.out + (size_t)(row0 + warp * RPW + r) * p.out_stride + (size_t)h * d;
-#pragma unroll
-            for (int x = 0; x < DPL; ++x)
-                if (lane + 32 * x < d) orow[lane + 32 * x] = from_float<T>(acc[r][x] * inv);
+            for (int r = 0; r < PV_ROWS; ++r) {
+                const int row = rv + r * RG_V;
+                if (reqs[row] != req) continue;
+                const float inv = 1.0f / l_of[row];
+                T* orow = p.out + (size_t)(row0 + row) * p.out_stride + (size_t)h * d + 4 * dv;
+                orow[0] = from_float<T>(acc[r].x * inv); orow[1] = from_float<T>(acc[r].y * inv);
+                orow[2] = from_float<T>(acc[r].z * inv); orow[3] = from_float<T>(acc[r].w * inv);
+            }
         }
     }
+    pdl_wait();                                     // also without a row to write: a kernel ends after the one ahead of it
 }
 
 template <typename T>
@@ -420,40 +528,43 @@ template <typename T, int KEYS>
 int launch_rows(const SimtParams<T>& p, cudaStream_t stream) {
     const size_t smem = sizeof(float) * (KEYS * (2 * p.head_dim + 4) + p.head_dim + KEYS);
     if (const int rc = allow_smem(attention_simt_rows_kernel<T, KEYS>, smem)) return rc;
-    const int blocks = p.tiled ? (p.n_tokens + TILE_ROWS - 1) / TILE_ROWS * SLOTS : p.n_tokens;
-    return tnx_launch_in_order(attention_simt_rows_kernel<T, KEYS>, dim3(blocks, p.n_heads), dim3(128), smem, stream, p);
+    return tnx_launch_in_order(attention_simt_rows_kernel<T, KEYS>, dim3(p.n_tokens, p.n_heads), dim3(128), smem, stream, p);
 }
 
-template <typename T, int DPL>
-int launch_tiles(const SimtParams<T>& p, cudaStream_t stream) {
-    const size_t smem = sizeof(float) * (TILE_ROWS * p.head_dim + 64 * (2 * p.head_dim + 4) + TILE_ROWS * 32);
-    if (const int rc = allow_smem(attention_simt_tiles_kernel<T, DPL>, smem)) return rc;
-    return tnx_launch_in_order(attention_simt_tiles_kernel<T, DPL>, dim3((p.n_tokens + TILE_ROWS - 1) / TILE_ROWS, p.n_heads), dim3(128), smem, stream, p);
+template <typename T, int DIMS, int THREADS>
+int launch_tiles(const SimtParams<T>& p, int* list, cudaStream_t stream) {
+    constexpr int KEYS = 64;                             // (a lone row's needs are less: the same without a tile's q)
+    const int d = p.head_dim, keys_pitch = (d > KEYS ? d : KEYS) + 4;
+    const size_t smem = sizeof(float) * (TILE_ROWS * (d + 4) + KEYS * keys_pitch + KEYS * d);
+    if (const int rc = allow_smem(attention_simt_tiles_kernel<T, DIMS, THREADS>, smem)) return rc;
+    const int tiles = (p.n_tokens + TILE_ROWS - 1) / TILE_ROWS, places = 148 * (DIMS == 64 ? 4 : 2);
+    int lone = places / p.n_heads;
+    lone = lone < 1 ? 1 : lone > p.n_tokens ? p.n_tokens : lone;
+    const int round = (148 + p.n_heads - 1) / p.n_heads, first_tiles = round < tiles ? round : tiles;
+    if (const int rc = tnx_launch_in_order(attention_simt_lone_list_kernel, dim3(1), dim3(1024), 0, stream, p.token_request, p.n_tokens, list)) return rc;
+    return tnx_launch_ex(1, attention_simt_tiles_kernel<T, DIMS, THREADS>, dim3(p.n_heads, tiles + lone), dim3(THREADS), smem, stream, p,
+                         list, lone, first_tiles, (int)((long long)tiles * p.n_heads <= places));
 }
 
 // portions: some request may have several rows.  The tiles take them where no mask shifts the 32-key steps of neighbouring
-// rows against one another and the rows are enough to give the SMs tiles (64 rows of 16 heads: 24 us row by row, 33 in
-// tiles; 140 rows of 2 heads: 19 and 53); the rows kernel follows for those that are alone in their tile.
+// rows against one another and the rows are enough to give the SMs tiles.
 template <typename T>
-int launch_all(SimtParams<T> p, int portions, cudaStream_t stream) {
-    const bool staged = p.head_dim % 4 == 0 && p.head_dim <= 128 && (uintptr_t)p.cache % (4 * sizeof(T)) == 0 && p.n_heads <= 65535;
+int launch_all(SimtParams<T> p, int portions, int* list, cudaStream_t stream) {
+    const bool staged = p.head_dim % 4 == 0 && p.head_dim <= 128 && (uintptr_t)p.cache % (4 * sizeof(T)) == 0 && p.n_heads <= 65535 && p.n_tokens <= 2000000;
     if (!staged) return launch_wide<T>(p, stream);
-    p.tiled = portions && p.window == 0 && (long long)p.n_tokens * p.n_heads >= 2048;
-    if (p.tiled) {
-        const int rc = p.head_dim <= 32 ? launch_tiles<T, 1>(p, stream) : p.head_dim <= 64 ? launch_tiles<T, 2>(p, stream)
-                                                                        : launch_tiles<T, 4>(p, stream);
-        if (rc) return rc;
-    }
+    if (portions && p.window == 0 && list && (long long)p.n_tokens * p.n_heads >= 2048)
+        return p.head_dim <= 64 ? launch_tiles<T, 64, 128>(p, list, stream) : launch_tiles<T, 128, 256>(p, list, stream);
     return p.head_dim <= 64 ? launch_rows<T, 128>(p, stream) : launch_rows<T, 64>(p, stream);
 }
 }  // namespace
 
-// portions: 0 where every request of the batch has one row (the rows kernel alone), else 1.
+// portions: 0 where every request of the batch has one row (the rows kernel alone), else 1; list: scratch memory of n_tokens + 1
+// numbers for the tiles (null: row by row).
 TNX_EXPORT int tnx_attention_simt(const void* q, int q_stride, const void* cache, const int* block_tables,
                                   int bt_stride, const int* token_request, const int* positions, void* out,
                                   int out_stride, int n_tokens, int n_heads, int n_kv_heads, int head_dim,
                                   int page_size, int window, float scale, int keep_first, const float* bias_mul,
-                                  const float* bias_rate, int has_sink, float sink_score, int is_h16, int portions,
+                                  const float* bias_rate, int has_sink, float sink_score, int is_h16, int portions, int* list,
                                   cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (head_dim <= 0 || head_dim > 32 * WIDE_DIMS_PER_LANE || n_kv_heads <= 0 || n_heads % n_kv_heads)
@@ -461,10 +572,12 @@ TNX_EXPORT int tnx_attention_simt(const void* q, int q_stride, const void* cache
     if (keep_first < 0 || (bias_mul && !bias_rate)) return TNX_ERR_BAD_ARG;
     const DistanceBias bias{bias_mul, bias_rate};
     const SoftmaxSink sink{has_sink, sink_score};
+    int page_shift = -1;
+    for (int i = 0; i < 31; ++i) if (page_size == 1 << i) page_shift = i;
 #define ASIMT(T)                                                                                                        \
     return launch_all<T>(SimtParams<T>{(const T*)q, q_stride, (const T*)cache, block_tables, bt_stride, token_request,  \
                                        positions, (T*)out, out_stride, n_tokens, n_heads, n_kv_heads, head_dim,         \
-                                       page_size, window, scale, keep_first, bias, sink, 0}, portions, stream)
+                                       page_size, window, scale, keep_first, bias, sink, page_shift}, portions, list, stream)
     if (is_h16) ASIMT(h16);
     ASIMT(float);
 #undef ASIMT
