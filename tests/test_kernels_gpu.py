@@ -257,6 +257,23 @@ def test_gemm_tc_every_many_token_kernel(M, N, K):
     assert {"tiles_128", "pairs", "persistent"} <= set(ran), ran
 
 
+@pytest.mark.parametrize("M,N,K", [(200, 2048, 2048), (512, 2048, 2048), (500, 768, 3072), (1536, 3216, 2048), (1536, 2048, 64), (257, 2048, 64)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_tc_plans_of_narrow_matrices(M, N, K, f32):
+    """Sizes for which the estimates choose clusters of 8, 4 and 2, whole pair tiles beside a few more, and pairs for a K of one
+    block; the choice may depend on the result's type."""
+    o = ops()
+    g = torch.Generator(device="cpu").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(N, K, generator=g) / math.sqrt(K)).bfloat16().to(DEV)
+    want = a.float() @ w.float().t()
+    out = torch.randn(M, N, generator=g).to(DEV) if f32 else torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    want = want + out if f32 else want
+    o.gemm_tc(a, w, out, residual=out if f32 else None)
+    o.raise_on_device_error()
+    assert rel_err(out, want) <= (2e-5 if f32 else 5e-3)
+
+
 def test_gemm_tc_plan_is_near_the_best_kernel():
     """The estimates that choose a kernel for more than 128 tokens were fitted on some layer sizes; here
     they are held against the fastest of all kernels at others (the 30B model's K of 7,168 and 28,672,

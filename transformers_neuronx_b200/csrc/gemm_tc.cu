@@ -1401,7 +1401,7 @@ struct ManyTokensPlan { int kind; int pairs; int sk_tiles; int sk_pairs; int spl
 static int g_forced_plan = -1;
 TNX_EXPORT void tnx_gemm_tc_force_plan(int plan) { g_forced_plan = plan; }
 
-static ManyTokensPlan plan_many_tokens(int M, int N, int K, int sms) {
+static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) {
     ManyTokensPlan r{2, 0, 0, 0, 1};
     const int kb = (K + BLOCK_K - 1) / BLOCK_K;
     const int tiles_m = (M + TILE_P - 1) / TILE_P;
@@ -1420,94 +1420,63 @@ static ManyTokensPlan plan_many_tokens(int M, int N, int K, int sms) {
         }
         return r;
     }
-    // Estimated times in microseconds, from measurements at 256..2,048 tokens: a K block of a
-    // 256 x 256 pair tile takes 0.45 us, of a 128 x 128 single tile 0.38 us; start and drain 8 / 6 us.
-    const float t_single = (float)((tiles_m * ((N + 127) / 128) + sms - 1) / sms) * kb * 0.38f + 6.f;
+    // Estimated times in microseconds.  Fitted to every plan's time at 140 .. 2,048 tokens by 25 matrices, [768 x 3072] to
+    // [20480 x 5120] and one of 64 columns (425 sizes, weights from memory): the estimates lie within 3 to 10 % of a plan's
+    // time, and the plan that they choose takes 0.2 % longer than the fastest one, on average (the rule before this one, fitted
+    // at widths of 4,096 and more, 8 %: 512 tokens by [2048 x 2048] 20.8 us where four K ranges in clusters take 13.0, 1,536 by
+    // [3216 x 2048] 54 where pairs take 42, 1,536 by [2048 x 64] 21 and 9.5).
+    // 32-bit results cost the kernels different amounts: the pairs' go out through TMA.
+    const float f32 = c_h16 ? 0.f : 1.f;
+    const int tiles_p = tiles_m * ((N + 255) / 256);                    // 128 x 256 tiles
+    auto rounds = [](int tiles, int places) { return (float)((tiles + places - 1) / places); };
+    const float t_single = rounds(tiles_m * ((N + 127) / 128), sms) * (kb * 0.303f + 8.6f + 1.5f * f32) + 1.4f;
     const int G = sms / 2;
     const int n_tiles = ((M + 255) / 256) * ((N + 255) / 256);          // 256 x 256 tiles of the paired kernel
     const int full = n_tiles / G, rest = n_tiles % G;
-    const float t_tile = kb * 0.45f;
-    float t_pair = (float)(full + (rest > 0)) * t_tile + 8.f;
-    // The tiles of a partly filled last wave (all tiles, when there are fewer than pairs) can be
-    // shared out by K blocks over GS pairs, at most four to a tile: that wave then takes rest / GS
-    // of a tile's time, but GS + rest partial tiles are written and read again (0.1 us each at the
-    // rate the second-level cache gives beside the main loop's loads) and the warp that adds them
-    // up needs 2.8 us per contributor, which hides behind a following whole tile if there is one.
-    // A margin of 1.3 on these costs; every pair must get at least four K blocks.
-    int sk_pairs = rest * 4 < G ? rest * 4 : G;
+    const float t_pair = rounds(n_tiles, G) * (kb * 0.386f + 1.8f - 3.f * f32) + 10.f;
+    const float t_persistent = rounds(tiles_p, sms) * (kb * 0.44f + 0.9f + 6.f * f32) + 15.f;
+    // The tiles of a partly filled last round (all tiles, when there are fewer than pairs) shared out by K blocks over
+    // sk_pairs pairs, at most four to a tile, every pair with at least four K blocks.  What the partial tiles cost depends on
+    // whether every shared tile is cut into exactly four runs (a pair then holds part of one tile only) or runs straddle tiles,
+    // and on whether a whole round of tiles hides the adding up.
+    const int sk_pairs = rest * 4 < G ? rest * 4 : G;
     float t_share = 1e30f;
-    // Measured at 129..2,048 tokens over the layer products of the 6.7B, 13B and 30B sizes and a
-    // vocabulary-sized N: sharing out pays where every shared tile is cut into exactly four runs (a pair
-    // then holds part of one tile only: 5-32 % faster behind a whole wave, and without one when K is long).
-    // With runs that straddle two tiles it pays while the last wave holds at most 0.55 tiles per pair and
-    // K is 256 blocks or more (10-35 %; up to 0.75 tiles per pair behind a whole wave), or 100 blocks or
-    // more behind a whole wave, 80 behind two (3-16 %); with a fuller last wave or a shorter K it lost
-    // 5-40 % against whole tiles in one more wave.
-    const bool four_runs = rest * 4 <= G;
-    const bool sparse_rest = rest * 100 <= G * 55;
-    const bool long_k = kb >= 256 && (full > 0 ? rest * 100 <= G * 75 : sparse_rest);
-    const bool behind_waves = sparse_rest && ((full >= 1 && kb >= 100) || (full >= 2 && kb >= 80));
-    if (rest > 0 && (long long)rest * kb >= 4LL * sk_pairs && (four_runs || long_k || behind_waves)) {
-        const float reduce = ((float)sk_pairs / rest + 1.f) * 2.8f;
-        const float exposed = full > 0 ? (reduce > t_tile ? reduce - t_tile : 0.f) : reduce;
-        t_share = ((float)full + (float)rest / sk_pairs) * t_tile + 8.f + 1.3f * ((sk_pairs + rest) * 0.1f + exposed);
+    if (rest > 0 && (long long)rest * kb >= 4LL * sk_pairs) {
+        const float blocks = ((float)full + (float)rest / sk_pairs) * kb;
+        if (rest * 4 <= G) t_share = full ? blocks * 0.306f + 33.f + 4.1f * full : blocks * 0.425f + 30.f + 0.05f * (sk_pairs + rest);
+        else t_share = full ? blocks * 0.36f + 60.f + 1.3f * full - 0.2f * (sk_pairs + rest) : blocks * 0.447f + 51.f - 0.138f * (sk_pairs + rest);
     }
-    if (M < 256) {
-        // 129..255 tokens: the weights are streamed once and the tensor cores idle.  Few 128 x 256
-        // tiles would leave SMs idle: 128 x 128 tiles, one per CTA, fill the GPU better then;
-        // otherwise the single-CTA persistent kernel with 128 x 256 tiles (a K block 0.45 us).  The
-        // paired kernel (half of whose 256 token rows may be empty) wins where K is long and the
-        // tiles are few, by sharing them out.
-        const int tiles_p = tiles_m * ((N + 255) / 256);
-        // Few tiles and a long K (the output projections of a layer): 128 x 256 tiles with K split 4 or
-        // 8 ways over the CTAs of a cluster, which add up through shared memory like the few-token
-        // form does (measured at 129..255 tokens: 22 against 28 us for [4096 x 4096], 44-50 against 60 us
-        // for [4096 x 16384]; with more tiles and a split of 2 the kernels below are faster).
-        {
-            int sp = MAX_CLUSTER;
-            while (sp > 1 && (tiles_p * sp > sms || sp * 4 > kb)) sp >>= 1;
-            if (sp >= 4) { r.kind = 3; r.splits = sp; return r; }
-        }
-        const bool single = tiles_p * 4 < sms * 3;
-        // In as many waves the persistent kernel is 5-8 % slower than the pairs (measured), so it must win outright.
-        const float t_here = single ? t_single : (float)((tiles_p + sms - 1) / sms) * kb * 0.45f * 1.05f + 8.f;
-        if (t_here <= t_pair && t_here <= t_share) { r.kind = single ? 0 : 2; return r; }
-    } else {
-        // 256 tokens and more: where the 128 x 256 tiles fit the GPU in one wave they can split K 1, 2, 4 or
-        // 8 ways in clusters as above.  A K block of such a tile takes 0.45 us; start and drain 8 us, the sum
-        // over a cluster 2 + splits us (measured at 256..768 tokens: [4096 x 16384] 43 / 69 / 71 us at
-        // 256 / 384 / 512 tokens against 63 / 87 / 89 us; [12288 x 4096] 40 against 50 us at 384).  It has to
-        // win by a tenth: where the estimates tie, the paired kernel was the faster one.
-        const int tiles_p = tiles_m * ((N + 255) / 256);
-        int best_sp = 0;
-        float t_split = 1e30f;
-        for (int sp = 1; sp <= MAX_CLUSTER && tiles_p * sp <= sms && (sp == 1 || sp * 4 <= kb); sp <<= 1) {
-            const float t = (float)((kb + sp - 1) / sp) * 0.45f + 8.f + (sp > 1 ? 2.f + (float)sp : 0.f);
-            if (t < t_split) { t_split = t; best_sp = sp; }
-        }
-        // The persistent kernel's 128 x 256 tiles waste less of a last token tile than the pairs' 256 rows
-        // (320 tokens: three tiles of 128 against two of 256): where that saves a wave it is 15-25 % faster
-        // (measured at 320, 384 and 640 tokens), in as many waves 3-7 % slower.
-        const float t_persistent = (float)((tiles_p + sms - 1) / sms) * kb * 0.45f * 1.05f + 8.f;
-        const float t_other = fminf(fminf(t_single, t_persistent), fminf(t_pair, t_share));
-        if (best_sp > 0 && t_split * 1.1f < t_other) { r.kind = 3; r.splits = best_sp; return r; }
-        if (t_single <= t_pair && t_single <= t_share && t_single <= t_persistent) { r.kind = 0; return r; }
-        if (t_persistent < t_pair && t_persistent < t_share) { r.kind = 2; return r; }
+    // 128 x 256 tiles, K split 1, 2, 4 or 8 ways over the CTAs of a cluster, all CTAs on the GPU at once; the CTAs of a cluster
+    // lie in one GPC, so clusters of four fill nine places in ten and of eight seven (200 tokens by [2048 x 2048] in eight
+    // ranges, 128 CTAs: 18.6 us, in four 11.7).
+    int splits = 0;
+    float t_split = 1e30f;
+    for (int sp = 1; sp <= MAX_CLUSTER; sp <<= 1) {
+        const int most = sp == 8 ? sms * 7 / 10 : sp == 4 ? sms * 9 / 10 : sms;
+        if (tiles_p * sp > most || (sp > 1 && sp * 4 > kb)) break;
+        const float t = sp == 1 ? kb * 0.37f + 16.2f + 2.2f * f32 : (float)((kb + sp - 1) / sp) * 0.405f + 9.2f;
+        if (t < t_split) { t_split = t; splits = sp; }
     }
-    r.kind = 1;
-    if (t_share < t_pair) { r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs; }
-    else r.pairs = n_tiles < G ? n_tiles : G;
+    const float best = fminf(fminf(fminf(t_single, t_pair), fminf(t_persistent, t_share)), t_split);
+    if (best == t_split) { r.kind = 3; r.splits = splits; }
+    else if (best == t_single) r.kind = 0;
+    else if (best == t_persistent) r.kind = 2;
+    else {
+        r.kind = 1;
+        if (t_share < t_pair) { r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs; }
+        else r.pairs = n_tiles < G ? n_tiles : G;
+    }
     return r;
 }
 
 // Bytes of 32-bit scratch and number of tile counters that tnx_gemm_tc needs for these sizes (0
 // when K is not split).  The caller owns both; the counters must be zero before the first call and
 // are left zero by every call.
-TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int n_sms, int* splits, long long* scratch_bytes, int* n_counters) {
+TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int c_h16, int n_sms, int* splits, long long* scratch_bytes, int* n_counters) {
     *splits = 1; *scratch_bytes = 0; *n_counters = 0;
     if (M > few_tokens_max()) {
         // paired kernel: two partial 256 x 256 tiles per pair, and a counter per shared tile, CTA and epilogue warp
-        const ManyTokensPlan mt = plan_many_tokens(M, N, K, n_sms);
+        const ManyTokensPlan mt = plan_many_tokens(M, N, K, c_h16, n_sms);
         if (mt.sk_tiles > 0) {
             *scratch_bytes = (long long)mt.pairs * 2 * 256 * 256 * 4;
             *n_counters = mt.sk_tiles * 8;
@@ -1573,7 +1542,7 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
             sms = cached_sms[dev];
         }
         const int tiles_m = (M + TILE_P - 1) / TILE_P, tiles_n = (N + PBN - 1) / PBN;
-        ManyTokensPlan mt = plan_many_tokens(M, N, K, sms);
+        ManyTokensPlan mt = plan_many_tokens(M, N, K, c_h16, sms);
         if (mt.kind < 0) return TNX_ERR_UNSUPPORTED;
         if (mt.kind == 0) {
             if (!make_map(&mq, W, N, K, ldw, 128)) return TNX_ERR_UNSUPPORTED;
