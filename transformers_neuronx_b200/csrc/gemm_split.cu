@@ -93,19 +93,6 @@ template <int BN, int NT> struct Shape {
     static_assert(NT * X_SLOTS <= SLOTS, "one barrier serves both rings");
 };
 
-// One place of a ring of N slots and the parity of its pass.
-template <int N> struct Ring {
-    int slot = 0;
-    uint32_t pass = 0;
-    __device__ __forceinline__ void next() { if (++slot == N) { slot = 0; pass ^= 1; } }
-};
-
-// True in one lane of the (whole) warp.
-__device__ __forceinline__ bool elected() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-    return e != 0;
-}
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"

@@ -117,6 +117,21 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[32]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// One place of a ring of N slots and the parity of its pass.
+template <int N> struct Ring {
+    int slot = 0;
+    uint32_t pass = 0;
+    __device__ __forceinline__ void next() { if (++slot == N) { slot = 0; pass ^= 1; } }
+};
+
+// True in one lane of the (whole) warp.  The warp that issues MMAs walks its loop as a whole and only the issue is one lane's:
+// what the loop computes then stays in uniform registers, while a loop that one lane walks alone moves every descriptor there for
+// every MMA (a K block of four MMAs cost the paired product 0.386 us of issue; the MMAs run 0.27).
+__device__ __forceinline__ bool elected() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes, 128-byte swizzled
 // (what TMA writes with CU_TENSOR_MAP_SWIZZLE_128B): groups of 8 rows are 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
