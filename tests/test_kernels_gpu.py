@@ -624,6 +624,27 @@ def test_attention_decode_with_a_key_value_heads_query_heads_in_one_block(n_head
         assert torch.equal(case.cache[written], full[written])
 
 
+@pytest.mark.parametrize("n_heads,n_kv,d", [(8, 8, 64), (8, 2, 80), (6, 3, 96), (8, 8, 112), (32, 2, 128), (8, 4, 128)])
+@pytest.mark.parametrize("n_splits,warps", [(1, 4), (3, 4), (8, 4), (1, 12), (4, 12)])
+@pytest.mark.parametrize("window,keep_first", [(0, 0), (70, 20)])
+@pytest.mark.parametrize("append", [False, True])
+def test_attention_decode_grouped_single_row(n_heads, n_kv, d, n_splits, warps, window, keep_first, append):
+    """A call of one row keeps its pages in registers, one of several in rings in shared memory: the same bits, over contexts of
+    fewer pages than splits, of whole and of begun pages."""
+    lens = [(n, 1) for n in (0, 15, 16, 40, 255, 300, 701)]
+    case = PagedCase(lens, n_heads, n_kv, d, torch.bfloat16, seed=d + n_splits)
+    g = torch.Generator().manual_seed(3)
+    new = [torch.randn(case.N, n_kv * d, generator=g).bfloat16().to(DEV) for _ in range(2)] if append else None
+    caches = [case.cache.clone() for _ in range(2)]
+    outs = [torch.zeros_like(case.q_flat) for _ in range(2)]
+    call = lambda i, **kw: ops().attention_decode(case.q_flat, caches[i], case.bt, case.tok_req, case.positions, outs[i], n_heads, 0.1, window=window,
+                                                  keep_first=keep_first, new_kv=new, n_splits=n_splits, warps=warps, grouped=True, **kw)
+    call(0)
+    for r in range(case.N):
+        call(1, rows=torch.tensor([r], dtype=torch.int32, device=DEV), n_rows=1)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(caches[0].view(torch.int16), caches[1].view(torch.int16))
+
+
 @pytest.mark.parametrize("n_heads,n_kv,d", [(3, 1, 64), (8, 1, 80), (9, 1, 96), (16, 1, 112), (17, 1, 128), (40, 2, 128), (3, 3, 128), (5, 5, 80)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("window", [None, 50])

@@ -708,19 +708,27 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
     """Whether decode attention runs the tensor-core kernel (csrc/attention_decode_grouped.cu) where that takes the sizes.
 
     With shared key/value heads always, but for the shortest steps (16 heads on one, 100 tokens: 4.6 us with a block a head,
-    6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1).  Without, where the other kernel's lanes idle (head sizes that
-    are no power of two: 80 dims, 8 rows of 32 heads over up to 1,400 tokens 33 and 29 us, 64 rows 169 and 144) and, for the
-    others, with few rows (one row of 32 heads of 128 over 250 / 1,400 tokens 7.6 and 5.2, 14.4 and 12.4 us, of 12 heads of 64 over
-    400 7.0 and 5.0); with more rows a block a head is as fast or faster (8 rows of 32 heads of 128 over 1,400 tokens 34.9 and
-    35.2, 64 179.7 and 179.6; heads of 64, 8 rows 20 and 27)."""
+    6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1), and always at head sizes that are no power of two, where the other
+    kernel's lanes idle (80 dims, 8 rows of 32 heads over up to 1,400 tokens 33 and 25 us, 64 rows over 1,500 180 and 120).
+    With equal heads of 64 or 128 dims where the other kernel's blocks do not happen to fill the SMs: it holds two blocks of
+    eight or four of four warps an SM, and up to 128 pages three quarters of those places and more in one round are its best
+    (512 blocks of 128 dims over 700 tokens 30.8 us and 31.3, 256 of 64 over 800 13.3 and 14.1; but 64 rows of 40 heads over
+    400 76.8 and 71.4, 31 over 900 82.5 and 71.4, 4 of 32 over 1,500 21.7 and 17.9).  Up to 16 pages: 128 dims 256 blocks 10.7
+    and 9.7, 640 21.8 and 18.7, 2,560 44.9 and 47.1; 64 dims never (12 blocks 4.7 and 5.1, 1,024 15.6 and 16.4), and up to 32
+    for few blocks and for a second round of the other kernel's that is not full (640 blocks 20.5 and 17.3, 1,024 21.2 and 22.1)."""
     blocks = rows * n_heads
-    if max_pages <= 12 and blocks <= sms:
+    if max_pages <= 12 and blocks <= sms or max_pages <= 16 and n_heads > 8 * n_kv and blocks <= 2 * sms:
         return False
-    if n_heads != n_kv:
+    if n_heads != n_kv or head_dim not in (64, 128):
         return True
-    if head_dim in (64, 128) or max_pages < 32:
-        return max_pages > (16 if head_dim == 64 else 12) and 2 * blocks <= sms
-    return True
+    if max_pages <= 16:
+        return head_dim == 128 and not 3 * sms < blocks <= 4 * sms and blocks < 6 * sms
+    fills = 32 * sms < 10 * blocks <= 40 * sms
+    if head_dim == 64:
+        if max_pages < 64:
+            return blocks <= sms or 4 * sms < blocks <= 6 * sms
+        fills = fills or 3 * sms < 2 * blocks <= 4 * sms
+    return max_pages >= 128 or not fills
 
 
 def grouped_decode_heads(n_heads: int, n_kv: int, head_dim: int) -> int:
@@ -730,32 +738,38 @@ def grouped_decode_heads(n_heads: int, n_kv: int, head_dim: int) -> int:
     return 8 if n_heads // n_kv <= 8 else 16
 
 
-def grouped_decode_plan(blocks: int, sms: int, heads_per_block: int, max_pages: int):
+def grouped_decode_plan(blocks: int, sms: int, heads_per_block: int, max_pages: int, head_dim: int = 128):
     """(warps a block, splits of the context) for `blocks` (row, head tile) blocks of the grouped decode attention.
 
-    An SM holds twelve of its warps with up to eight query heads a block (one block of twelve or three of four), eight with
-    sixteen.  Splits are a cluster's blocks, and clusters leave places empty: those of up to four blocks fill nine places in
-    ten, wider ones seven (16 blocks in eight splits each, 128 places of 148, ran in two rounds: 21 against 14 us with six)."""
-    big = 12 if heads_per_block == 8 else 8
-    if blocks > sms:
-        # More blocks than SMs: short contexts in blocks of four warps (512 blocks of 8 pages: 15 us, of twelve warps 22),
-        # and so many blocks that ragged contexts leave the big ones' last rounds uneven (1,024 of up to 88 pages: 70
-        # against 80 us, equal ones of 128 pages 187 against 177).  Else whichever leaves the fewer places of its
-        # last round empty (256 blocks of 128 pages: 53 us with twelve warps, 57 with four; 512: 102 and 121, 384 ragged
-        # ones 62 and 58).
-        if max_pages < 2 * big or blocks > 4 * sms:
+    An SM holds twelve of its warps with up to eight query heads a block (one block of twelve or three of four; four of heads of
+    64), eight with sixteen.  Splits are a cluster's blocks, and clusters leave places empty: those of up to four blocks fill nine places in
+    ten, wider ones seven (16 blocks in eight splits each, 128 places of 148, ran in two rounds: 21 against 14 us with six).
+    Drawn from 2 to 64 rows of 12 to 40 heads over 190 to 1,900 tokens, every plan against the others (us):
+      * up to 16 pages: small blocks, in four splits of few pairs (32 blocks 5.9, of twelve warps 6.3), twelve warps for up to one
+        block an SM (96 blocks 6.2; four 6.7), else four (192 blocks 9.2, twelve 11.7);
+      * few pairs over many pages: big blocks in three splits and more (32 blocks of 64 pages 7.5, small ones in four 8.2);
+      * else small blocks in as many splits as find places at once (96 blocks of 64 pages in four 11.6, twelve warps 14; 128 of 128
+        pages in three 17.9, twelve warps 18.9; 160 in two 23.5, one 31; 384 ragged ones of 119 pages in one 53.8, twelve warps 55.9;
+        512 of 25 pages 24.6 and 31.9).  With sixteen heads a block two splits of four warps lose to one of eight (128
+        blocks of 64 pages 23.0 and 19.4)."""
+    big, places = (12, (4 if head_dim == 64 else 3) * sms) if heads_per_block == 8 else (8, 2 * sms)
+
+    def splits(places):
+        if 20 * 2 * blocks <= 19 * places < 20 * 3 * blocks:
+            return 2
+        s = (9 * places) // (10 * blocks)
+        return s if s <= 4 else min(8, max(4, (7 * places) // (10 * blocks)))
+
+    if max_pages <= 16:
+        if blocks > sms:
             return 4, 1
-        fill = lambda per: blocks / (-(-blocks // (per * sms)) * per * sms)
-        return (4, 1) if fill(big // 4) >= fill(1) else (big, 1)
-    # Fewer: big blocks, split while the SMs last; few pages (under four a warp of a big block) in splits of four warps
-    # (one row of 32 heads on 8 over 400 tokens: 5.4 us in eight splits of four warps, 6.4 of twelve).
-    short = max_pages < 4 * big
-    warps, places = (4, sms * big // 4) if short else (big, sms)
-    most = max(1, max_pages // (3 if short else 8))
-    splits = min(most, (9 * places) // (10 * blocks))
-    if splits > 4:
-        splits = min(most, 8, max(4, (7 * places) // (10 * blocks)))
-    return warps, max(1, splits)
+        return (4, 4) if heads_per_block == 8 and 8 * blocks <= 3 * sms and max_pages >= 8 else (big, 1)
+    if max_pages >= 4 * big and splits(sms) >= 3:
+        return big, min(splits(sms), max_pages // 8)
+    s = splits(places)
+    if heads_per_block == 16 and blocks <= sms and s < 3:
+        return big, 1
+    return 4, max(1, min(s, max_pages // 4))
 
 
 def attention_decode(q, cache, block_tables, token_request, positions, out, n_heads, scale, window=0, rows=None,
@@ -791,7 +805,7 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
     if heads_per_block:
         tiles = n_kv * -(-(n_heads // n_kv) // heads_per_block)
         if n_splits is None:
-            warps, n_splits = grouped_decode_plan(R * tiles, st["sms"], heads_per_block, max_pages)
+            warps, n_splits = grouped_decode_plan(R * tiles, st["sms"], heads_per_block, max_pages, d)
         most_warps = 12 if heads_per_block == 8 else 8     # a forced plan's warps: 4, or all that an SM holds
         warps = 4 if warps in (None, 4) else most_warps
         n_splits = max(1, min(int(n_splits), max_pages, 8))
@@ -826,7 +840,7 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
             _p(q), c_int(q_stride), _p(cache), _p(block_tables), c_int(block_tables.stride(0)),
             _p(rows), _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(R),
             c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask_rule(window, chunk)), c_float(scale),
-            c_int(n_splits), c_int(pps), _p(k_new), _p(v_new), c_int(kv_stride), c_int(warps),
+            c_int(n_splits), _p(k_new), _p(v_new), c_int(kv_stride), c_int(warps),
             *_score_options(keep_first, bias, sink, n_heads, window), _stream()), "attention_decode")
         return
     _check(lib.tnx_attention_decode_append(
