@@ -410,15 +410,14 @@ attention_decode_grouped_kernel(const GroupedParams p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
     const int row = p.rows ? p.rows[ri] : ri;
     if (row < 0) return;                                        // a padded entry of the row list of a captured step
-    const int req = p.token_request[row];
-    if (req < 0) return;                                        // a padded row of a captured batch
-    const int pos = p.positions[row];
-    const int* bt = p.block_tables + (size_t)req * p.bt_stride;
-
+    const int req = p.token_request[row], pos = p.positions[row];       // asked for together, and the queries beside them
     Heads<D, NT, BIAS> w;
     w.g = g; w.c = c;
     uint8_t* const ring = smem_raw + warp * WARP_BYTES;
     uint2* const qs = (uint2*)(ring + (RING ? w.SLOTS * w.SLOT : 0)) + lane;
+    w.load_queries(p, row, h0, n_mine, qs);
+    if (req < 0) return;                                        // a padded row of a captured batch
+    const int* bt = p.block_tables + (size_t)req * p.bt_stride;
     const int kv_len = pos + 1;
     const int first_key = first_visible_key(pos, p.window);
     const int n_pages = (kv_len + PAGE - 1) / PAGE;
@@ -430,7 +429,8 @@ attention_decode_grouped_kernel(const GroupedParams p) {
     const bool own_here = p.k_new != nullptr && walk.place(pos / PAGE) / per_split == split;    // one answer for the block
     const int cached_len = p.k_new != nullptr ? pos : kv_len;
     const int my_pages = page_hi > page_lo + warp ? (page_hi - page_lo - warp + WARPS - 1) / WARPS : 0;
-    const int n_chunks = my_pages + (own_here && warp == 0 ? 1 : 0);         // the token's own key is a chunk of one key
+    // the token's own key is a chunk of one key, of the warp whose turn comes after the pages' (warp 0 may have one page more)
+    const int n_chunks = my_pages + (own_here && warp == max(page_hi - page_lo, 0) % WARPS ? 1 : 0);
 
     w.start(p, h0, n_mine, p.sink.on && split == 0 && warp == 0);
 
@@ -442,7 +442,6 @@ attention_decode_grouped_kernel(const GroupedParams p) {
         if (t < my_pages) return p.cache + (((size_t)page * 2 + which) * p.n_kv_heads + kvh) * head_block;
         return (which ? p.v_new : p.k_new) + (size_t)row * p.kv_stride + (size_t)kvh * D;
     };
-    w.load_queries(p, row, h0, n_mine, qs);
     auto ask = [&](int t, int page) {
         if (t < n_chunks) w.ask(shared_address(ring) + t % w.SLOTS * w.SLOT, rows_of(t, page, 0), rows_of(t, page, 1), t < my_pages, first_of(t), lane, seen);
         w.asked();
