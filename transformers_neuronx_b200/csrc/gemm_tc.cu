@@ -1500,9 +1500,11 @@ TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int c_h16, int n_sms, int* 
     // 72 and 74 tiles split 4 ways (288 and 296 CTAs for 296 places) took 38 and 21 us where a split of 2 takes 31
     // and 16, while 56 tiles split 4 ways (224) and 32 tiles split 8 ways (256) are the fastest of their kind and
     // 148 tiles split 2 ways (296) still beat no split.  So clusters of 4 and 8 may take nine places in ten.
+    // A split keeps four K blocks, of four three (16 tokens by [768 x 768] 5.4 us in two, 4.5 in four); beyond 32 tokens eight ways
+    // cost more than they save below 48 K blocks (100 tokens by [2048 x 2048] 10.2 us, 8.6 in four; by [768 x 3072] 8.8 and 9.5).
     int s = MAX_CLUSTER;
     for (; s > 1; s >>= 1) {
-        if (s * 4 > kb) continue;
+        if (s * (s == 4 ? 3 : 4) > kb || (s == 8 && M > 32 && kb < 48)) continue;
         if (s == 2 ? tiles * s <= 2 * n_sms : tiles * s * 10 <= 2 * n_sms * 9) break;
     }
     *splits = s;
