@@ -76,6 +76,8 @@ class DecoderModel:
         if act_dtype == torch.float32:
             libs = [l for l in libs if l not in ("gemm_tc", "gemv", "attention_prefill", "attention_prefill_tc", "attention_decode", "attention_decode_grouped",
                                                  "moe_grouped")]
+        else:
+            libs = [l for l in libs if l != "gemm_split"]            # for 32-bit activations
         return list(dict.fromkeys(libs))
 
     @property
