@@ -533,6 +533,20 @@ def test_attention_simt_tiles_edges(lens, d, n_heads, n_kv):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d", [48, 52, 56, 60, 64, 68, 124])
+def test_attention_simt_tiles_take_every_head_size(d, dtype):
+    """Head sizes around the one whose tiles need more than 48 KB of shared memory, static arrays among them."""
+    case = PagedCase([(7, 66), (30, 1), (0, 65)], 16, 4, d, dtype, seed=d)
+    assert case.N * 16 >= 2048
+    outs = [torch.zeros(case.N, 16 * d, dtype=dtype, device=DEV) for _ in range(2)]
+    for out, portions in zip(outs, (True, False)):
+        ops().attention_simt(case.q_flat, case.cache, case.bt, case.tok_req, case.positions, out, 16, 0.13, portions=portions)
+    assert torch.equal(outs[0], outs[1])
+    want = torch.cat([exact_attention(q, k, v, 0.13, c).reshape(len(q), -1) for (c, _), q, k, v in zip(case.lens, case.q, case.k, case.v)])
+    assert rel_err(outs[0], want.to(DEV)) <= (1e-5 if dtype == torch.float32 else 1e-2)
+
+
 @pytest.mark.parametrize("rows,window,kernels", [(103, 0, 2), (101, 0, 1), (103, 37, 1)])
 def test_attention_simt_counts_its_kernels(rows, window, kernels):
     """20 heads: from 2,048 (row, head) pairs on without a window two kernels run, else one."""

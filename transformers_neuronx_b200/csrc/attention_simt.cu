@@ -516,9 +516,11 @@ int launch_wide(const SimtParams<T>& p, cudaStream_t stream) {
 #undef WIDE
 }
 
+// More than 48 KB of shared memory have to be asked for, and a kernel's static arrays count as well (the tiles' take 2.3 KB: heads of 56
+// and 60 dims stay below with their dynamic part alone).
 template <typename K>
 int allow_smem(K kernel, size_t smem) {
-    if (smem <= 48 * 1024) return 0;
+    if (smem + 3 * 1024 <= 48 * 1024) return 0;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) cudaGetLastError();
     return (int)e;
