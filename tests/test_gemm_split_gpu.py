@@ -102,6 +102,28 @@ def test_gemm_split_elements_that_are_not_finite(dtype):
         assert bool(((out[7] - fma[7]).abs()[torch.isfinite(fma[7])] <= K * 2.0 ** -132).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("small", [1e-10, -1e-10, 1e-30, -1e-42])
+def test_gemm_split_small_elements_opposite_infinite_weights(small, dtype):
+    """An infinite weight times any number but zero is infinite, however small the number is beside the others in its row: in rows
+    that are finite, that reach the largest number, and that hold an infinity or a NaN themselves."""
+    inf = float("inf")
+    a, w, _, _ = _operands(5, 128, 256, dtype, 3)
+    a[:, 7], a[:, 9] = small, 0.0
+    a[1, 100] = 3e38                                    # scaled down by 2^113 for float16
+    a[2, 100], a[3, 100], a[4, 100] = inf, -inf, float("nan")
+    w[:, 100] = w[:, 100].abs() + 1e-3
+    w[1, 7], w[2, 7], w[3, 9] = inf, -inf, inf          # (the last: infinity times zero has no value)
+    out, fma = torch.empty(5, 128, device=DEV), torch.empty(5, 128, device=DEV)
+    ops().gemm_split(a, w, out)
+    ops().gemm_simt(a, w, fma)
+    ops().raise_on_device_error()
+    assert bool(torch.isinf(fma[0, 1:3]).all()) and bool(torch.isnan(fma[:, 3]).all())
+    assert torch.equal(torch.isnan(out), torch.isnan(fma))
+    big = torch.isinf(fma)
+    assert torch.equal(out[big], fma[big]) and bool(torch.isfinite(out[torch.isfinite(fma)]).all())
+
+
 def test_gemm_split_in_slices_of_rows(monkeypatch):
     o = ops()
     a, w, bias, res = _operands(300, 256, 512, torch.float16, 3)

@@ -20,8 +20,8 @@
 // of the call, bit for bit.
 //
 // Infinities and NaN come out as from 32-bit multiplications: such an element is its own first term (and the terms of the
-// others in its row are cut to a representable size, they cannot matter beside it); a sum of first terms that is not
-// finite stands, whatever the other terms say.
+// others in its row are cut to a representable size, they cannot matter beside it, but opposite an infinite weight, so that none
+// but zero becomes zero); a sum of first terms that is not finite stands, whatever the other terms say.
 //
 // Warp roles as in gemm_tc.cu: warp 0 TMA, warp 1 MMAs, warps from 2 on the accumulators; every wait is bounded.  Persistent
 // CTAs, one an SM, walk over tiles of 128 NT features by BN tokens (tokens fastest: the CTAs at work share weights in the
@@ -385,20 +385,22 @@ __global__ void __launch_bounds__(128) split_sum_kernel(const Params p, int segs
 constexpr int SPLIT_THREADS = 256;
 __device__ __forceinline__ bool not_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
 
-// h, m, l of one (scaled) element; odd: its row holds an element that is not finite.
-__device__ __forceinline__ void terms(float x, bool odd, h16& h, h16& m, h16& l) {
+// h, m, l of one element v; odd: its row holds an element that is not finite.
+__device__ __forceinline__ void terms(float v, float scale, bool odd, h16& h, h16& m, h16& l) {
 #ifdef TNX_F16
+    const float x = v * scale;
+    h = __float2half_rn(odd && !not_finite(x) ? fminf(fmaxf(x, -1.f), 1.f) : x);
+    // no element but zero becomes zero: an infinite weight tells them apart
+    if ((uint16_t)(__half_as_ushort(h) << 1) == 0 && v != 0.f) h = __ushort_as_half(v < 0.f ? 0x8001 : 0x0001);
     if (odd) {
-        h = not_finite(x) ? __float2half_rn(x) : __float2half_rn(fminf(fmaxf(x, -1.f), 1.f));
         m = l = __float2half_rn(0.f);
         return;
     }
-    h = __float2half_rn(x);
-    if (__half_as_ushort(h) << 1 == 0 && x != 0.f) h = __ushort_as_half(x < 0.f ? 0x8001 : 0x0001);    // (an infinite weight times a small number)
     const float r = (x - __half2float(h)) * 2048.f;
     m = __float2half_rn(r);
     l = __float2half_rn((r - __half2float(m)) * 2048.f);
 #else
+    const float x = v;
     const uint32_t u = __float_as_uint(x);
     if (not_finite(x)) {                 // infinities keep their sign; a NaN stays one when its low bits go
         h = __ushort_as_bfloat16((unsigned short)((u >> 16) | ((u & 0x7fffffu) ? 0x40u : 0u)));
@@ -463,10 +465,10 @@ split_terms_kernel(const float* __restrict__ A, h16* __restrict__ planes, float*
 #endif
     const size_t plane = (size_t)M * K;
     auto put = [&](int q, float4 v) {
-        const float x[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+        const float x[4] = {v.x, v.y, v.z, v.w};
         __align__(8) h16 h[4], m[4], l[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) terms(x[i], odd, h[i], m[i], l[i]);
+        for (int i = 0; i < 4; ++i) terms(x[i], scale, odd, h[i], m[i], l[i]);
         h16* dst = planes + (size_t)row * K + 4 * (size_t)q;
         *(uint2*)dst = *(const uint2*)h;
         *(uint2*)(dst + plane) = *(const uint2*)m;
