@@ -547,6 +547,32 @@ def test_attention_simt_tiles_take_every_head_size(d, dtype):
     assert rel_err(outs[0], want.to(DEV)) <= (1e-5 if dtype == torch.float32 else 1e-2)
 
 
+@pytest.mark.parametrize("d,n_heads,n_kv", [(64, 16, 4), (128, 16, 16), (100, 20, 5), (20, 16, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", [[(3 * i, 2) for i in range(50)] + [(60, 2), (63, 2)] * 10,          # many to a tile, around one stage of keys
+                                  [(5, 8), (0, 9), (70, 16), (3, 17), (9, 31), (1, 1), (0, 32), (130, 33), (7, 7), (62, 3), (61, 3), (2, 4), (64, 1), (0, 63), (11, 64)],
+                                  [(40, 3)] * 400 + [(5, 1)] * 90])                                   # more tiles than are looked over at a time
+@pytest.mark.parametrize("mixed", [False, True])
+def test_attention_simt_several_portions_in_a_tile(lens, mixed, d, n_heads, n_kv, dtype):
+    """Portions of 2 to 64 rows that share tiles, their rows in order or mixed, padded rows among them, against the same rows one by
+    one: the same bits, with a distance bias and a sink as well."""
+    case = PagedCase(lens, n_heads, n_kv, d, dtype, seed=d)
+    assert case.N * n_heads >= 2048
+    g = torch.Generator().manual_seed(2)
+    q, req, pos = case.q_flat, case.tok_req, case.positions
+    if mixed:
+        at = torch.randperm(case.N, generator=g).to(DEV)
+        q, req, pos = q[at].contiguous(), req[at].clone(), pos[at].contiguous()
+        req[::17] = -1
+    more = dict(bias=(torch.rand(n_heads, generator=g).to(DEV), torch.rand(n_heads, generator=g).to(DEV)), sink=0.3) if mixed else {}
+    outs = [torch.full((case.N, n_heads * d), 7.0, dtype=dtype, device=DEV) for _ in range(2)]
+    for out, portions in zip(outs, (True, False)):
+        ops().attention_simt(q, case.cache, case.bt, req, pos, out, n_heads, 0.11, portions=portions, **more)
+    assert torch.equal(outs[0], outs[1])
+    if mixed:
+        assert bool((outs[0][::17] == 7.0).all())
+
+
 @pytest.mark.parametrize("rows,window,kernels", [(103, 0, 2), (101, 0, 1), (103, 37, 1)])
 def test_attention_simt_counts_its_kernels(rows, window, kernels):
     """20 heads: from 2,048 (row, head) pairs on without a window two kernels run, else one."""

@@ -365,15 +365,14 @@ def attention_simt(q, cache, block_tables, token_request, positions, out, n_head
     _need(token_request, "token_request", torch.int32, 1)
     _need(positions, "positions", torch.int32, 1)
     mask = mask_rule(window, chunk)
-    # as in the entry point: where portions go in tiles, the rows that are alone in theirs are listed first
+    # as in the entry point: where portions go in tiles, a kernel of its own takes what a tile holds beside its largest one
     tiled = (portions and mask == 0 and N * n_heads >= 2048 and d % 4 == 0 and d <= 128 and n_heads <= 65535 and N <= 2000000
              and cache.data_ptr() % (4 * cache.element_size()) == 0)
-    lone = torch.empty(N + 1, dtype=torch.int32, device=q.device) if tiled else None
     _check(lib.tnx_attention_simt(_p(q), c_int(q_stride), _p(cache), _p(block_tables), c_int(block_tables.stride(0)),
                                   _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(N),
                                   c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask),
                                   c_float(scale), *_score_options(keep_first, bias, sink, n_heads, window),
-                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), _p(lone), _stream()), "attention_simt", 2 if tiled else 1)
+                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), _stream()), "attention_simt", 2 if tiled else 1)
 
 
 def sample(logits, out, temperature=None, top_k=None, top_p=None, seeds=None, counters=None, suppress_id=-1,
