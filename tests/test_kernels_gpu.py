@@ -274,6 +274,37 @@ def test_gemm_tc_plans_of_narrow_matrices(M, N, K, f32):
     assert rel_err(out, want) <= (2e-5 if f32 else 5e-3)
 
 
+@pytest.mark.parametrize("M,N,K,most", [(45, 2048, 2048, 1 / 7), (100, 2560, 2560, 1 / 7), (65, 2050, 3000, 1 / 7),       # eight runs, or four in halves
+                                        (200, 2048, 2048, 1 / 7), (300, 3072, 3072, 2 / 7), (536, 768, 10240, 1 / 7), (1557, 256, 8192, 1 / 7),
+                                        (1816, 5120, 5120, 0.9), (920, 7168, 7168, 0.9), (2048, 2560, 2560, 0.9)])       # the last round's chains halved
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gemm_tc_chains_of_additions(M, N, K, most, dtype):
+    """What a sum of positive products loses in the accumulators grows with the chain of additions: in R runs added up in 32 bits it
+    is at most 1/R of what one chain over the whole of K loses.  `most` is that with the runs' rounding, where the plan cuts K."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g, device=DEV).abs().to(dtype)
+    w = torch.randn(N, K, generator=g, device=DEV).abs().mul(0.02).to(dtype)
+    want = a.double() @ w.double().t()
+    err = lambda out: float((out.double() - want).norm() / want.norm())
+    out, whole = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    o.gemm_tc(a, w, out)
+    try:
+        if M > 128:
+            o.gemm_tc_force_plan("tiles_128", dtype)
+        o.gemm_tc(a, w, whole, splits=1 if M <= 128 else None)
+    finally:
+        o.gemm_tc_force_plan(None, dtype)
+    o.raise_on_device_error()
+    assert err(out) <= most * err(whole)
+    bias, res = torch.randn(N, generator=g, device=DEV), torch.randn(M, N, generator=g, device=DEV)
+    joined, half = res.clone(), torch.empty(M, N, dtype=dtype, device=DEV)
+    o.gemm_tc(a, w, joined, bias=bias, residual=joined)
+    o.gemm_tc(a, w, half, bias=bias, activation="relu")
+    o.raise_on_device_error()
+    assert rel_err(joined, want + bias + res) <= 1e-4 and rel_err(half, torch.relu(want + bias)) <= 5e-3
+
+
 def test_gemm_tc_plan_is_near_the_best_kernel():
     """The estimates that choose a kernel for more than 128 tokens were fitted on some layer sizes; here
     they are held against the fastest of all kernels at others (the 30B model's K of 7,168 and 28,672,

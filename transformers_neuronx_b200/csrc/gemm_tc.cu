@@ -60,6 +60,7 @@ struct Params {
                                  // through distributed shared memory instead of scratch memory
     int sk_tiles;                // paired kernel: the last sk_tiles output tiles are shared out by K blocks
     int sk_pairs;                // ... over the first sk_pairs pairs
+    int halve_from;              // ... with HALVES: the first pair whose last tile's chains are halved
     const int* span_of_tile;     // grouped product in CTA pairs: a tile's rows, (first row / 32) * 8 + rows / 32 - 1
     const int* group_of_tile;    // grouped product: the group of every tile of tokens (128 of them, up to 256 in CTA pairs, BN in the swapped form), -1: none;
     int group_rows;              //   W holds group_rows rows per group, a tile of group g reads W's rows from g * group_rows on
@@ -87,7 +88,7 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t cluster_addr) {
     return v;
 }
 
-template <int BN, bool SWAP>
+template <int BN, bool SWAP, bool BIAS_STAGED = false>
 __device__ __forceinline__ void store_tile_row(const Params& p, int lane_row, int col0, const float (&v)[32], int ncols,
                                                const float* bias_s = nullptr) {
     // lane_row: index on the P axis; col0..col0+ncols: indices on the Q axis.
@@ -140,14 +141,14 @@ __device__ __forceinline__ void store_tile_row(const Params& p, int lane_row, in
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     float t = v[j];
-                    if (p.bias) t += bias_s ? bias_s[j] : __ldg(p.bias + col0 + j);
+                    if (p.bias) t += BIAS_STAGED ? bias_s[j] : __ldg(p.bias + col0 + j);
                     x[j] += gelu_new_fast(t);
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     float t = v[j];
-                    if (p.bias) t += bias_s ? bias_s[j] : __ldg(p.bias + col0 + j);
+                    if (p.bias) t += BIAS_STAGED ? bias_s[j] : __ldg(p.bias + col0 + j);
                     t = apply_activation(t, p.act);
                     x[j] += t;
                 }
@@ -361,13 +362,29 @@ __device__ __forceinline__ void cluster_sum_received(const Params& p, const floa
     }
 }
 
-template <int BN, int STAGES, bool SWAP>
+// LD_COLS columns of an accumulator; with `second`, the sums with the one BN columns further.
+template <int LD_COLS, int BN, bool HALVES>
+__device__ __forceinline__ void load_sums(uint32_t taddr, uint32_t (&r)[32], bool second) {
+    if (LD_COLS == 32) tmem_ld32(taddr, r); else tmem_ld16(taddr, r);
+    tmem_ld_wait();
+    if (HALVES && second) {
+        uint32_t s[32];
+        if (LD_COLS == 32) tmem_ld32(taddr + BN, s); else tmem_ld16(taddr + BN, s);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < LD_COLS; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(s[j]));
+    }
+}
+
+// HALVES: two accumulators, one for each half of the CTA's K blocks (see add_accumulator).  Only forms that leave an SM's 512 columns to
+// one CTA or two can.
+template <int BN, int STAGES, bool SWAP, bool HALVES>
 __global__ void __launch_bounds__(NUM_THREADS, SWAP ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, const Params p) {
     constexpr int A_BYTES = TILE_P * BLOCK_K * 2;            // 16 KB
     constexpr int B_BYTES = BN * BLOCK_K * 2;
     constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+    constexpr uint32_t TMEM_COLS = (BN < 32 ? 32 : BN) * (HALVES ? 2 : 1);
     constexpr int LD_COLS = BN < 32 ? 16 : 32;
 
     extern __shared__ uint8_t smem_raw[];
@@ -404,6 +421,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     const int kb_begin = split * p.kb_per_split;
     const int kb_end = min(num_kb_total, kb_begin + p.kb_per_split);
     const int num_kb = max(0, kb_end - kb_begin);
+    const int first_half = HALVES && num_kb > 1 ? (num_kb + 1) / 2 : num_kb;         // K blocks of the first accumulator
 
     // One K block = one stage: the weight tile and the activation tile complete the same barrier.
     // The weights are never written by a kernel, so their loads may start before the preceding
@@ -494,8 +512,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 #pragma unroll
                 for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
                     // advancing 16 elements along K = 32 bytes = 2 units of the address field
-                    umma_h16(tmem_base, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc,
-                              (i > 0 || k > 0) ? 1u : 0u);
+                    umma_h16(tmem_base + (HALVES && i >= first_half ? BN : 0), adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc,
+                              ((i > 0 && i != first_half) || k > 0) ? 1u : 0u);
                 }
                 umma_commit(&empty_bar[r.slot]);         // the stage is free once these MMAs have read it
                 if (i == num_kb - 1) umma_commit(&tmem_full_bar);             // accumulators complete
@@ -519,8 +537,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 for (int c = 0; c < BN; c += LD_COLS) {
                     uint32_t r[32];
                     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c;
-                    if (LD_COLS == 32) tmem_ld32(taddr, r); else tmem_ld16(taddr, r);
-                    tmem_ld_wait();
+                    load_sums<LD_COLS, BN, HALVES>(taddr, r, first_half < num_kb);
                     float v[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = (j < LD_COLS && num_kb > 0) ? __uint_as_float(r[j]) : 0.f;
@@ -536,8 +553,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 for (int c = 0; c < BN; c += LD_COLS) {
                     uint32_t r[32];
                     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c;
-                    if (LD_COLS == 32) tmem_ld32(taddr, r); else tmem_ld16(taddr, r);
-                    tmem_ld_wait();
+                    load_sums<LD_COLS, BN, HALVES>(taddr, r, first_half < num_kb);
                     if (SWAP) {
 #pragma unroll
                         for (int j = 0; j < LD_COLS; ++j) part[(c + j) * TILE_P] = num_kb > 0 ? __uint_as_float(r[j]) : 0.f;
@@ -558,8 +574,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 for (int c = 0; c < BN; c += LD_COLS) {
                     uint32_t r[32];
                     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c;
-                    if (LD_COLS == 32) tmem_ld32(taddr, r); else tmem_ld16(taddr, r);
-                    tmem_ld_wait();
+                    load_sums<LD_COLS, BN, HALVES>(taddr, r, first_half < num_kb);
 #pragma unroll
                     for (int j = 0; j < LD_COLS; ++j)
                         __stcg(dst + (size_t)(c + j) * TILE_P, num_kb > 0 ? __uint_as_float(r[j]) : 0.f);
@@ -583,8 +598,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 uint32_t v[32];
                 if (ok) {
                     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c;
-                    if (LD_COLS == 32) tmem_ld32(taddr, v); else tmem_ld16(taddr, v);
-                    tmem_ld_wait();
+                    load_sums<LD_COLS, BN, HALVES>(taddr, v, first_half < num_kb);
                 }
 #pragma unroll
                 for (int j = 0; j < LD_COLS; ++j) part[(c + j) * nr] = (ok && num_kb > 0) ? __uint_as_float(v[j]) : 0.f;    // defined even if a wait ran out
@@ -777,6 +791,25 @@ __device__ __forceinline__ void acc_load_end(const AccSource& a) {
     if (!FROM_SCRATCH) tmem_ld_wait();
 }
 
+// One warp's lanes of an accumulator += those of another.  An addition to an accumulator cuts off what it shifts out, so what a sum
+// loses grows with the length of the chain: positive operands, 32-bit results, relative errors 1.2e-6 over chains of 256, 2.7e-6 of 512,
+// 5.9e-6 of 1,024, 1.2e-5 of 2,048.  Where a plan has longer chains than another that is only a little slower, each half of them goes to
+// an accumulator of its own.
+template <int WIDTH>
+__device__ __forceinline__ void add_accumulator(uint32_t addr, uint32_t other) {
+#pragma unroll 1
+    for (int c = 0; c < WIDTH; c += 32) {
+        uint32_t a[32], b[32];
+        tmem_ld32(addr + (uint32_t)c, a);
+        tmem_ld32(other + (uint32_t)c, b);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(__uint_as_float(a[j]) + __uint_as_float(b[j]));
+        tmem_st32(addr + (uint32_t)c, a);
+    }
+    tmem_st_wait();
+}
+
 // Epilogue of one warp of the many-token kernels: its 32 accumulator rows x WIDTH columns -> C.
 // With a residual (32-bit, possibly C itself) the loads of the next 32 columns are issued before
 // the current ones are stored, so that a tile costs one memory round trip, not one per chunk.
@@ -796,7 +829,7 @@ __device__ __forceinline__ void drain_accumulator(const Params& p, const AccSour
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            store_tile_row<WIDTH, false>(p, row, col_base + c, v, 32, p.bias ? bias_tile + c : nullptr);
+            store_tile_row<WIDTH, false, true>(p, row, col_base + c, v, 32, bias_tile + c);
         }
         return;
     }
@@ -1096,7 +1129,7 @@ __host__ __device__ constexpr uint32_t instr_desc_pair(int n) {      // M = 256 
 // that has finished), whole tiles only.  16 experts of 2048 x 4096 and 4096 x 2048 with 512 rows each and all that
 // lies around them take 517 us (614 in 128 x 256 tiles of one CTA each, whose last tiles were 128 rows whatever they held); with
 // 128 rows each 223 (295), with 64 206 (209); 128 experts of 1536 x 2048 and 2048 x 768 with 128 rows each 454 (608).
-template <bool GROUPED>
+template <bool GROUPED, bool HALVES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                     const __grid_constant__ CUtensorMap map_res, const __grid_constant__ CUtensorMap map_out,
@@ -1150,6 +1183,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         } else {
             tile = g + (i - n_seg) * G; kb0 = 0; kb1 = num_kb;
         }
+    };
+    // HALVES: the last item of the pairs from p.halve_from on has both accumulators: the K blocks from here on go to the other one,
+    // whose sums of the item before have nearly always been taken out by then (28 K blocks take as long as that).  Elsewhere the
+    // other accumulator is the next tile's.
+    auto second_from = [&](int i) {
+        if (!HALVES || i != n_items - 1 || g < p.halve_from) return num_kb;
+        const int half = (num_kb + 1) / 2, late = min(28, (3 * num_kb + 3) / 4);
+        return i > 0 && late > half ? late : half;
     };
     // GROUPED: a tile's first token, and the columns its tokens take of the accumulator; each CTA of the pair brings half of them
     auto row_of = [&](int tm) { return (p.span_of_tile[tm] >> 3) * 32; };
@@ -1238,15 +1279,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_ph ^ 1, p.err, 22));      // both CTAs drained this accumulator
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
+                uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
+                const int second = second_from(t);
                 for (int kb = kb0; kb < kb1; ++kb) {
+                    if (HALVES && kb == second) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc ^ 1], (uint32_t)(((t + 1) >> 1) & 1) ^ 1, p.err, 25));
+                        if (!ok) break;
+                        tc_fence_after();
+                        d_tmem = tmem_base + (uint32_t)((acc ^ 1) * 256);
+                    }
                     ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[r.slot], r.pass, p.err, 23));
                     if (!ok) break;
                     const uint64_t adesc = desc0 + (uint64_t)(r.slot * (STAGE_BYTES >> 4)), bdesc = adesc + (uint64_t)(A_BYTES >> 4);
                     if (elected()) {
 #pragma unroll
                         for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
-                            umma_h16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                            umma_h16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, ((kb > kb0 && !(HALVES && kb == second)) || k > 0) ? 1u : 0u);
                         umma_commit_pair(&empty_bar[r.slot]);                // the stage is free in both CTAs
                         if (kb == kb1 - 1) umma_commit_pair(&acc_full[acc]);
                     }
@@ -1305,6 +1353,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             tc_fence_after();
             AccSource src{tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256), nullptr, 0, 0, 0};
             if (whole) {
+                if (HALVES && second_from(t) < num_kb) add_accumulator<256>(src.tmem_addr, tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)((acc ^ 1) * 256));
                 if (tma_epilogue) ok = drain_accumulator_tma<256>(p, epi, src, row0, tn * 256, bias_tile[acc], lane);
                 else drain_accumulator<256>(p, src, row0 + lane, tn * 256, bias_tile[acc]);
                 tc_fence_before();
@@ -1370,18 +1419,18 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
 }
 
 // ---- host side ----------------------------------------------------------------------------------
-template <int BN, int STAGES, bool SWAP>
+template <int BN, int STAGES, bool SWAP, bool HALVES = false>
 int launch(const CUtensorMap& mp, const CUtensorMap& mq, const Params& p, dim3 grid, cudaStream_t stream) {
     constexpr size_t smem = (size_t)STAGES * (TILE_P * BLOCK_K * 2 + BN * BLOCK_K * 2) + 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, SWAP, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
     if (p.cluster_reduce)
-        return tnx_launch_cluster(1, dim3(1, 1, grid.z), gemm_tc_kernel<BN, STAGES, SWAP>, grid, dim3(NUM_THREADS), smem, stream, mp, mq, p);
-    return tnx_launch_ex(1, gemm_tc_kernel<BN, STAGES, SWAP>, grid, dim3(NUM_THREADS), smem, stream, mp, mq, p);
+        return tnx_launch_cluster(1, dim3(1, 1, grid.z), gemm_tc_kernel<BN, STAGES, SWAP, HALVES>, grid, dim3(NUM_THREADS), smem, stream, mp, mq, p);
+    return tnx_launch_ex(1, gemm_tc_kernel<BN, STAGES, SWAP, HALVES>, grid, dim3(NUM_THREADS), smem, stream, mp, mq, p);
 }
 
 }  // namespace
@@ -1395,7 +1444,7 @@ static constexpr int FEW_TOKENS_MAX = 128;
 static int few_tokens_max() { return FEW_TOKENS_MAX; }
 TNX_EXPORT int tnx_gemm_tc_few_tokens() { return few_tokens_max(); }
 
-struct ManyTokensPlan { int kind; int pairs; int sk_tiles; int sk_pairs; int splits; };   // kind 0: 128 x 128 tiles, 1: CTA pairs, 2: persistent, 3: 128 x 256 tiles with K split in clusters
+struct ManyTokensPlan { int kind; int pairs; int sk_tiles; int sk_pairs; int splits; int halves = 0; int halve_from = 0; };   // kind 0: 128 x 128 tiles, 1: CTA pairs, 2: persistent, 3: 128 x 256 tiles with K split in clusters
 // A plan imposed from outside (-1: the estimates below choose).  0: 128 x 128 tiles; 1: CTA pairs, whole
 // tiles; 2: persistent 128 x 256 tiles; 4: CTA pairs with the last wave shared out by K blocks; 31, 32,
 // 34, 38: 128 x 256 tiles with K split 1, 2, 4, 8 ways in clusters.  It exists so that a test can time
@@ -1418,7 +1467,7 @@ static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) 
             r.kind = 1; r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs;
         } else if (g_forced_plan > 30 && g_forced_plan <= 30 + MAX_CLUSTER) {
             const int sp = g_forced_plan - 30;
-            if ((sp & (sp - 1)) == 0 && tiles_p * sp <= sms && (sp == 1 || sp * 4 <= kb)) { r.kind = 3; r.splits = sp; }
+            if ((sp & (sp - 1)) == 0 && tiles_p * sp <= sms && (sp == 1 || sp * 4 <= kb)) { r.kind = 3; r.splits = sp; r.halves = sp > 1; }
         }
         return r;
     }
@@ -1462,15 +1511,21 @@ static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) 
     // Over a long K the tiles that are shared out also have the smaller errors (an accumulator cuts off what an addition shifts
     // out: 1,280 tokens by [2048 x 16384] 2.4e-5 of the largest result in whole tiles, 1e-5 shared), so near ties are theirs.
     const float t_whole = fminf(fminf(t_single, t_pair), fminf(t_persistent, splits == 1 ? t_split : 1e30f));
+    if (splits > 1 && t_split <= 1.1f * t_share) t_share = 1e30f;            // (a split's chains are shorter still)
     if (kb >= 100 && t_share <= 1.1f * t_whole && (splits <= 1 || t_share < t_split)) t_share = 0.f;
     const float best = fminf(fminf(fminf(t_single, t_pair), fminf(t_persistent, t_share)), t_split);
-    if (best == t_split) { r.kind = 3; r.splits = splits; }
+    if (best == t_split) { r.kind = 3; r.splits = splits; r.halves = splits > 1 && splits < MAX_CLUSTER; }
     else if (best == t_single) r.kind = 0;
     else if (best == t_persistent) r.kind = 2;
     else {
         r.kind = 1;
-        if (t_share < t_pair) { r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs; }
-        else r.pairs = n_tiles < G ? n_tiles : G;
+        // For the same reason less than a round of tiles is shared out over a long K whatever the estimates say, and behind whole rounds
+        // a long K has its last chains halved: those of the pairs without a tile of the last round, which costs no time, and where these
+        // are few (less would be gained than by sharing out) of all pairs (2 us).
+        const bool quarters = rest * 4 <= G, sparse = rest * 100 <= G * 55;
+        const int long_from = full == 0 ? (quarters ? 54 + 7 * rest / 4 : sparse ? 256 : 1 << 30) : quarters ? 20 + 2 * rest / 3 : sparse ? (full > 1 ? 80 : 100) : 256;
+        if (t_share < t_pair || (full == 0 && t_share < 1e30f && kb >= long_from)) { r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs; }
+        else { r.pairs = n_tiles < G ? n_tiles : G; r.halves = full > 0 && rest > 0 && rest * 100 <= G * 75 && kb >= long_from; r.halve_from = rest * 5 <= G * 2 ? rest : 0; }
     }
     return r;
 }
@@ -1500,28 +1555,28 @@ TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int c_h16, int n_sms, int* 
     // 72 and 74 tiles split 4 ways (288 and 296 CTAs for 296 places) took 38 and 21 us where a split of 2 takes 31
     // and 16, while 56 tiles split 4 ways (224) and 32 tiles split 8 ways (256) are the fastest of their kind and
     // 148 tiles split 2 ways (296) still beat no split.  So clusters of 4 and 8 may take nine places in ten.
-    // A split keeps four K blocks, of four three (16 tokens by [768 x 768] 5.4 us in two, 4.5 in four); beyond 32 tokens eight ways
-    // cost more than they save below 48 K blocks (100 tokens by [2048 x 2048] 10.2 us, 8.6 in four; by [768 x 3072] 8.8 and 9.5).
+    // A split keeps four K blocks, of four three (16 tokens by [768 x 768] 5.4 us in two, 4.5 in four); beyond 64 tokens eight ways
+    // cost more than they save below 48 K blocks (100 tokens by [2048 x 2048] 10.2 us, 8.6 in four; but 64 tokens 7.9 and 8.4).
     int s = MAX_CLUSTER;
     for (; s > 1; s >>= 1) {
-        if (s * (s == 4 ? 3 : 4) > kb || (s == 8 && M > 32 && kb < 48)) continue;
+        if (s * (s == 4 ? 3 : 4) > kb || (s == 8 && M > 64 && kb < 48)) continue;
         if (s == 2 ? tiles * s <= 2 * n_sms : tiles * s * 10 <= 2 * n_sms * 9) break;
     }
     *splits = s;
     return 0;
 }
 
-template <bool GROUPED>
+template <bool GROUPED, bool HALVES = false>
 static int launch_pair(int ctas, cudaStream_t stream, const CUtensorMap& mp, const CUtensorMap& mq, const CUtensorMap& mres,
                        const CUtensorMap& mout, const Params& p, int tiles_m, int tiles_n, int tma_epilogue) {
     constexpr size_t smem = (size_t)CSTAGES * (TILE_P * BLOCK_K * 2 + 128 * BLOCK_K * 2) + PAIR_EPI_BYTES + 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<GROUPED, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return tnx_launch_ex(1, gemm_tc_pair_kernel<GROUPED>, dim3(ctas), dim3(NUM_THREADS), smem, stream, mp, mq, mres, mout, p,
+    return tnx_launch_ex(1, gemm_tc_pair_kernel<GROUPED, HALVES>, dim3(ctas), dim3(NUM_THREADS), smem, stream, mp, mq, mres, mout, p,
                          tiles_m, tiles_n, tma_epilogue);
 }
 
@@ -1561,6 +1616,7 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
             if (!make_map(&mq, W, N, K, ldw, 256)) return TNX_ERR_UNSUPPORTED;
             p.splits = mt.splits; p.kb_per_split = (kb + mt.splits - 1) / mt.splits; p.cluster_reduce = mt.splits > 1;
             dim3 grid((M + TILE_P - 1) / TILE_P, (N + 255) / 256, mt.splits);
+            if (mt.halves) return launch<256, 4, false, true>(mp, mq, p, grid, stream);
             return launch<256, 4, false>(mp, mq, p, grid, stream);
         }
         if (mt.kind == 1) {
@@ -1569,13 +1625,14 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
                 mt.sk_tiles = 0; mt.sk_pairs = 0;
                 if (mt.pairs > ptiles_m * ptiles_n) mt.pairs = ptiles_m * ptiles_n;
             }
-            p.sk_tiles = mt.sk_tiles; p.sk_pairs = mt.sk_pairs;
+            p.sk_tiles = mt.sk_tiles; p.sk_pairs = mt.sk_pairs; p.halve_from = mt.halve_from;
             if (!make_map(&mq, W, N, K, ldw, 128)) return TNX_ERR_UNSUPPORTED;
             // A 32-bit residual goes through TMA boxes when the row pitch and the addresses allow it.
             CUtensorMap mres = mp, mout = mp;
             int tma_epilogue = 0;
             if (residual && !c_h16 && ldc % 4 == 0 && !(((uintptr_t)residual | (uintptr_t)C) & 15))
                 tma_epilogue = make_map_f32(&mres, residual, M, N, ldc, 32) && make_map_f32(&mout, C, M, N, ldc, 32);
+            if (mt.halves) return launch_pair<false, true>(2 * mt.pairs, stream, mp, mq, mres, mout, p, ptiles_m, ptiles_n, tma_epilogue);
             return launch_pair<false>(2 * mt.pairs, stream, mp, mq, mres, mout, p, ptiles_m, ptiles_n, tma_epilogue);
         }
         if (!make_map(&mq, W, N, K, ldw, PBN)) return TNX_ERR_UNSUPPORTED;
@@ -1605,6 +1662,8 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
     if (bn == 16) return launch<16, 6, true>(mp, mq, p, grid, stream);
     if (bn == 32) return launch<32, 5, true>(mp, mq, p, grid, stream);
     if (bn == 64) return launch<64, 4, true>(mp, mq, p, grid, stream);
+    // (half the chains of four splits: those of the eight that the plan leaves for speed)
+    if (splits == 4 && kb >= 32 && kb < 48) return launch<128, 3, true, true>(mp, mq, p, grid, stream);
     return launch<128, 3, true>(mp, mq, p, grid, stream);
 }
 
