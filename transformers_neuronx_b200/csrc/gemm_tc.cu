@@ -1452,7 +1452,11 @@ struct ManyTokensPlan { int kind; int pairs; int sk_tiles; int sk_pairs; int spl
 static int g_forced_plan = -1;
 TNX_EXPORT void tnx_gemm_tc_force_plan(int plan) { g_forced_plan = plan; }
 
-static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) {
+// What a product's result is: the kernels' epilogues cost different amounts.
+enum { RESULT_16_BIT, RESULT_32_BIT, RESULT_WITH_RESIDUAL };
+static int result_kind(int c_h16, const void* residual) { return c_h16 ? RESULT_16_BIT : residual ? RESULT_WITH_RESIDUAL : RESULT_32_BIT; }
+
+static ManyTokensPlan plan_many_tokens(int M, int N, int K, int result, int has_bias, int sms) {
     ManyTokensPlan r{2, 0, 0, 0, 1};
     const int kb = (K + BLOCK_K - 1) / BLOCK_K;
     const int tiles_m = (M + TILE_P - 1) / TILE_P;
@@ -1471,21 +1475,25 @@ static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) 
         }
         return r;
     }
-    // Estimated times in microseconds.  Fitted to every plan's time at 140 .. 2,048 tokens by 25 matrices, [768 x 3072] to
-    // [20480 x 5120] and one of 64 columns (425 sizes, weights from memory): the estimates lie within 3 to 10 % of a plan's
-    // time, and the plan that they choose takes 0.2 % longer than the fastest one, on average (the rule before this one, fitted
-    // at widths of 4,096 and more, 8 %: 512 tokens by [2048 x 2048] 20.8 us where four K ranges in clusters take 13.0, 1,536 by
-    // [3216 x 2048] 54 where pairs take 42, 1,536 by [2048 x 64] 21 and 9.5).
-    // 32-bit results cost the kernels different amounts: the pairs' go out through TMA.
-    const float f32 = c_h16 ? 0.f : 1.f;
+    // Estimated times in microseconds.  Fitted to every plan's time at 140 .. 2,048 tokens by matrices of [64 x 64] to [50272 x 4096]
+    // and [16384 x 16384], weights from memory: the plan that they choose takes 0.1 % longer than the fastest one, on average over 3,500
+    // sizes (with one figure for all 32-bit results and none for a bias 2 %: without a residual pairs were chosen at small K and N, 2,048
+    // tokens by [64 x 64] 16.5 us and 9.3; with a bias, which the forms that take a tile a CTA read element by element, single tiles: 300 by
+    // [12288 x 4096] 58 us and 48; the rule before, fitted at widths of 4,096 and more, 8 %: 512 tokens by [2048 x 2048] 20.8 us
+    // where four K ranges in clusters take 13.0, 1,536 by [3216 x 2048] 54 where pairs take 42).
+    // With a residual the pairs fetch and store through TMA, the others row by row.
+    struct Costs { float single, pair, pair_start, persistent, share, tile, split; };                 // beside those of a 16-bit result
+    static constexpr Costs COSTS[3] = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, {1.2f, 0.8f, 2.f, 1.f, 3.f, 0.5f, 0.f}, {1.2f, -3.3f, 0.f, 11.f, 0.f, 1.6f, 1.f}};
+    const Costs c = COSTS[result];
+    const float bias_cost = !has_bias ? 0.f : result == RESULT_WITH_RESIDUAL ? 8.6f : 5.4f;            // of a 128 x 128 tile; 2.2 times that of a 128 x 256 one
     const int tiles_p = tiles_m * ((N + 255) / 256);                    // 128 x 256 tiles
     auto rounds = [](int tiles, int places) { return (float)((tiles + places - 1) / places); };
-    const float t_single = rounds(tiles_m * ((N + 127) / 128), sms) * (kb * 0.286f + 8.6f + 1.2f * f32) + 1.5f;
+    const float t_single = rounds(tiles_m * ((N + 127) / 128), sms) * (kb * 0.286f + 8.6f + c.single + bias_cost) + 1.5f;
     const int G = sms / 2;
     const int n_tiles = ((M + 255) / 256) * ((N + 255) / 256);          // 256 x 256 tiles of the paired kernel
     const int full = n_tiles / G, rest = n_tiles % G;
-    const float t_pair = rounds(n_tiles, G) * (kb * 0.32f + 1.6f - 3.3f * f32) + 10.f;
-    const float t_persistent = rounds(tiles_p, sms) * (kb * 0.4f + 4.f + 1.8f * f32) + 15.3f;
+    const float t_pair = rounds(n_tiles, G) * fmaxf(kb * 0.32f + 1.6f + c.pair, 1.f) + 10.f + c.pair_start;
+    const float t_persistent = rounds(tiles_p, sms) * (kb * 0.4f + 4.f + c.persistent) + 15.3f;
     // The tiles of a partly filled last round (all tiles, when there are fewer than pairs) shared out by K blocks over
     // sk_pairs pairs, at most four to a tile, every pair with at least four K blocks.  What the partial tiles cost depends on
     // whether every shared tile is cut into exactly four runs (a pair then holds part of one tile only) or runs straddle tiles,
@@ -1496,6 +1504,7 @@ static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) 
         const float blocks = ((float)full + (float)rest / sk_pairs) * kb;
         if (rest * 4 <= G) t_share = full ? blocks * 0.262f + 33.2f + 5.5f * full : blocks * 0.376f + 29.4f + 0.05f * (sk_pairs + rest);
         else t_share = full ? blocks * 0.322f + 62.5f + 1.1f * full - 0.208f * (sk_pairs + rest) : blocks * 0.424f + 52.4f - 0.156f * (sk_pairs + rest);
+        t_share += c.share;
     }
     // 128 x 256 tiles, K split 1, 2, 4 or 8 ways over the CTAs of a cluster, all CTAs on the GPU at once; the CTAs of a cluster
     // lie in one GPC, so clusters of four fill nine places in ten and of eight seven (200 tokens by [2048 x 2048] in eight
@@ -1505,39 +1514,42 @@ static ManyTokensPlan plan_many_tokens(int M, int N, int K, int c_h16, int sms) 
     for (int sp = 1; sp <= MAX_CLUSTER; sp <<= 1) {
         const int most = sp == 8 ? sms * 7 / 10 : sp == 4 ? sms * 9 / 10 : sms;
         if (tiles_p * sp > most || (sp > 1 && sp * 4 > kb)) break;
-        const float t = sp == 1 ? kb * 0.38f + 16.3f + 1.6f * f32 : (float)((kb + sp - 1) / sp) * 0.41f + 9.3f;
+        const float t = sp == 1 ? kb * 0.38f + 16.3f + c.tile + 2.2f * bias_cost : (float)((kb + sp - 1) / sp) * 0.41f + 9.3f + c.split;
         if (t < t_split) { t_split = t; splits = sp; }
     }
+    // What a chain of additions loses shows in 32-bit results, and over a long K in 16-bit ones (up to 8,192 the errors agree to 0.2 %).
+    // Halved chains are kernels of their own, whose code comes cold between products of the others (6 us).
+    const bool shows = result != RESULT_16_BIT || kb >= 128;
     // Over a long K the tiles that are shared out also have the smaller errors (an accumulator cuts off what an addition shifts
     // out: 1,280 tokens by [2048 x 16384] 2.4e-5 of the largest result in whole tiles, 1e-5 shared), so near ties are theirs.
     const float t_whole = fminf(fminf(t_single, t_pair), fminf(t_persistent, splits == 1 ? t_split : 1e30f));
-    if (splits > 1 && t_split <= 1.1f * t_share) t_share = 1e30f;            // (a split's chains are shorter still)
+    if (shows && splits > 1 && t_split <= 1.1f * t_share) t_share = 1e30f;   // (a split's chains are shorter still)
     if (kb >= 100 && t_share <= 1.1f * t_whole && (splits <= 1 || t_share < t_split)) t_share = 0.f;
     const float best = fminf(fminf(fminf(t_single, t_pair), fminf(t_persistent, t_share)), t_split);
-    if (best == t_split) { r.kind = 3; r.splits = splits; r.halves = splits > 1 && splits < MAX_CLUSTER; }
+    if (best == t_split) { r.kind = 3; r.splits = splits; r.halves = shows && splits > 1 && splits < MAX_CLUSTER; }
     else if (best == t_single) r.kind = 0;
     else if (best == t_persistent) r.kind = 2;
     else {
         r.kind = 1;
-        // For the same reason less than a round of tiles is shared out over a long K whatever the estimates say, and behind whole rounds
-        // a long K has its last chains halved: those of the pairs without a tile of the last round, which costs no time, and where these
+        // Where it shows, less than a round of tiles is shared out over a long K whatever the estimates say, and behind whole rounds
+        // a long K has its last chains halved: those of the pairs without a tile of the last round, which end early, and where these
         // are few (less would be gained than by sharing out) of all pairs (2 us).
         const bool quarters = rest * 4 <= G, sparse = rest * 100 <= G * 55;
         const int long_from = full == 0 ? (quarters ? 54 + 7 * rest / 4 : sparse ? 256 : 1 << 30) : quarters ? 20 + 2 * rest / 3 : sparse ? (full > 1 ? 80 : 100) : 256;
-        if (t_share < t_pair || (full == 0 && t_share < 1e30f && kb >= long_from)) { r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs; }
-        else { r.pairs = n_tiles < G ? n_tiles : G; r.halves = full > 0 && rest > 0 && rest * 100 <= G * 75 && kb >= long_from; r.halve_from = rest * 5 <= G * 2 ? rest : 0; }
+        if (t_share < t_pair || (shows && full == 0 && t_share < 1e30f && kb >= long_from)) { r.pairs = G; r.sk_tiles = rest; r.sk_pairs = sk_pairs; }
+        else { r.pairs = n_tiles < G ? n_tiles : G; r.halves = shows && full > 0 && rest > 0 && rest * 100 <= G * 75 && kb >= long_from; r.halve_from = rest * 5 <= G * 2 ? rest : 0; }
     }
     return r;
 }
 
 // Bytes of 32-bit scratch and number of tile counters that tnx_gemm_tc needs for these sizes (0
-// when K is not split).  The caller owns both; the counters must be zero before the first call and
-// are left zero by every call.
-TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int c_h16, int n_sms, int* splits, long long* scratch_bytes, int* n_counters) {
+// when K is not split).  result: 0 16-bit, 1 32-bit, 2 32-bit added to a residual.  The
+// caller owns both; the counters must be zero before the first call and are left zero by every call.
+TNX_EXPORT int tnx_gemm_tc_plan(int M, int N, int K, int result, int has_bias, int n_sms, int* splits, long long* scratch_bytes, int* n_counters) {
     *splits = 1; *scratch_bytes = 0; *n_counters = 0;
     if (M > few_tokens_max()) {
         // paired kernel: two partial 256 x 256 tiles per pair, and a counter per shared tile, CTA and epilogue warp
-        const ManyTokensPlan mt = plan_many_tokens(M, N, K, c_h16, n_sms);
+        const ManyTokensPlan mt = plan_many_tokens(M, N, K, result, has_bias, n_sms);
         if (mt.sk_tiles > 0) {
             *scratch_bytes = (long long)mt.pairs * 2 * 256 * 256 * 4;
             *n_counters = mt.sk_tiles * 8;
@@ -1605,7 +1617,7 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
             sms = cached_sms[dev];
         }
         const int tiles_m = (M + TILE_P - 1) / TILE_P, tiles_n = (N + PBN - 1) / PBN;
-        ManyTokensPlan mt = plan_many_tokens(M, N, K, c_h16, sms);
+        ManyTokensPlan mt = plan_many_tokens(M, N, K, result_kind(c_h16, residual), bias != nullptr, sms);
         if (mt.kind < 0) return TNX_ERR_UNSUPPORTED;
         if (mt.kind == 0) {
             if (!make_map(&mq, W, N, K, ldw, 128)) return TNX_ERR_UNSUPPORTED;
@@ -1663,7 +1675,7 @@ TNX_EXPORT int tnx_gemm_tc(const void* A, const void* W, const float* bias, cons
     if (bn == 32) return launch<32, 5, true>(mp, mq, p, grid, stream);
     if (bn == 64) return launch<64, 4, true>(mp, mq, p, grid, stream);
     // (half the chains of four splits: those of the eight that the plan leaves for speed)
-    if (splits == 4 && kb >= 32 && kb < 48) return launch<128, 3, true, true>(mp, mq, p, grid, stream);
+    if (!c_h16 && splits == 4 && kb >= 32 && kb < 48) return launch<128, 3, true, true>(mp, mq, p, grid, stream);
     return launch<128, 3, true>(mp, mq, p, grid, stream);
 }
 

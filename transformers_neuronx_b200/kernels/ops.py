@@ -440,7 +440,7 @@ def raise_if_error_code(code: int, where: str = "") -> None:
 # ---------------------------------------------------------------------------------------------
 # Tensor-core kernels (bfloat16).
 _attention_impls = {}
-_gemm_plans = {}          # (M, N, K, type of the result, SMs) -> (splits, scratch bytes, counters) as the library plans them
+_gemm_plans = {}          # (M, N, K, kind of the result, a bias, SMs) -> (splits, scratch bytes, counters) as the library plans them
 _dev_state = {}          # per device: error word, split-K scratch and counters, SM count
 
 
@@ -608,14 +608,16 @@ def gemm_tc(a, w, out, bias=None, residual=None, activation=None, splits=None, f
                                _stream()), "gemv")
             return
     st = _state(a.device)
-    plan = _gemm_plans.get((M, N, K, out.dtype, st["sms"]))
+    kind = 0 if _is_h16(out) else 2 if residual is not None else 1
+    key = (M, N, K, kind, bias is not None, st["sms"])
+    plan = _gemm_plans.get(key)
     if plan is None:
         n_splits, nbytes, ncnt = c_int(1), ctypes.c_longlong(0), c_int(0)
-        lib.tnx_gemm_tc_plan(c_int(M), c_int(N), c_int(K), c_int(_is_h16(out)), c_int(st["sms"]), ctypes.byref(n_splits),
-                             ctypes.byref(nbytes), ctypes.byref(ncnt))
+        lib.tnx_gemm_tc_plan(c_int(M), c_int(N), c_int(K), c_int(kind), c_int(bias is not None), c_int(st["sms"]),
+                             ctypes.byref(n_splits), ctypes.byref(nbytes), ctypes.byref(ncnt))
         if len(_gemm_plans) > 4096:
             _gemm_plans.clear()
-        plan = _gemm_plans[(M, N, K, out.dtype, st["sms"])] = (n_splits.value, nbytes.value, ncnt.value)
+        plan = _gemm_plans[key] = (n_splits.value, nbytes.value, ncnt.value)
     n_splits, nbytes, ncnt = c_int(plan[0]), ctypes.c_longlong(plan[1]), c_int(plan[2])
     if splits is not None and M <= lib.tnx_gemm_tc_few_tokens():
         kb = -(-K // 64)
