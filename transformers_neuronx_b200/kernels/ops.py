@@ -809,8 +809,7 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
             warps, n_splits = grouped_decode_plan(R * tiles, st["sms"], heads_per_block, max_pages, d)
         most_warps = 12 if heads_per_block == 8 else 8     # a forced plan's warps: 4, or all that an SM holds
         warps = 4 if warps in (None, 4) else most_warps
-        n_splits = max(1, min(int(n_splits), max_pages, 8))
-        pps = -(-max_pages // n_splits)
+        n_splits, pps = max(1, min(int(n_splits), max_pages, 8)), 0            # (a row's own pages are cut, whatever max_pages is)
     elif n_splits is None:
         warps, n_splits = decode_attention_plan(R * n_heads, st["sms"], d, max_pages)
         pps = -(-max_pages // n_splits)
@@ -819,7 +818,8 @@ def attention_decode(q, cache, block_tables, token_request, positions, out, n_he
         warps = int(warps or 4)
         n_splits = max(1, min(int(n_splits), max_pages))
         pps = -(-max_pages // n_splits)
-    n_splits = -(-max_pages // pps)
+    if not heads_per_block:
+        n_splits = -(-max_pages // pps)
     scratch = None
     if n_splits > 1 and not heads_per_block:
         need = R * n_heads * n_splits * (d + 2)
