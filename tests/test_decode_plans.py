@@ -47,3 +47,11 @@ def test_grouped_decode_runs_the_planned_splits(recorded, rows, heads, kv, d, pa
 def test_grouped_decode_runs_the_splits_asked_for(recorded):
     assert [_grouped_call(recorded, 2, 8, 2, 64, 44, n_splits=n, warps=4) for n in (1, 3, 7, 8, 20)] == [1, 3, 7, 8, 8]
     assert _grouped_call(recorded, 2, 8, 2, 64, 3, n_splits=7, warps=4) == 3
+
+
+@pytest.mark.parametrize("heads,rows,pages,grouped", [(12, 32, 2, False), (12, 32, 4, False), (32, 64, 4, False), (32, 16, 2, False),
+                                                      (32, 8, 2, True), (12, 32, 12, True), (32, 64, 12, True), (32, 64, 128, True)])
+def test_many_short_contexts_of_112_dims_go_a_head_a_block(heads, rows, pages, grouped):
+    assert ops.grouped_decode_takes(rows, heads, heads, 112, 148, pages) == grouped
+    assert ops.grouped_decode_takes(rows, heads, heads, 96, 148, pages)
+    assert ops.grouped_decode_takes(rows, heads, heads // 4, 112, 148, pages)

@@ -709,8 +709,9 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
     """Whether decode attention runs the tensor-core kernel (csrc/attention_decode_grouped.cu) where that takes the sizes.
 
     With shared key/value heads always, but for the shortest steps (16 heads on one, 100 tokens: 4.6 us with a block a head,
-    6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1), and always at head sizes that are no power of two, where the other
-    kernel's lanes idle (80 dims, 8 rows of 32 heads over up to 1,400 tokens 33 and 25 us, 64 rows over 1,500 180 and 120).
+    6.0 grouped; 32 on 8, one row of 120 tokens 4.4 and 5.1).  Equal heads of 80, 96 and 112 dims too (1 to 64 rows of 12 and 32
+    heads over 2 to 128 pages, a block a head and grouped: 80 dims, 64 rows over 96 221 and 133 us; 96 dims, 8 rows over 2 pages 8.0
+    and 4.6, 64 over 64 192 and 110; 112 dims, 64 rows over 128 288 and 219; from 16 pages on at most 3 % slower), but for many blocks of up to four pages at 112 dims (384 blocks 6.2 and 7.1, 2,048 23.2 and 26.0).
     With equal heads of 64 or 128 dims where the other kernel's blocks do not happen to fill the SMs: it holds two blocks of
     eight or four of four warps an SM, and up to 128 pages three quarters of those places and more in one round are its best
     (512 blocks of 128 dims over 700 tokens 30.8 us and 31.3, 256 of 64 over 800 13.3 and 14.1; but 64 rows of 40 heads over
@@ -721,7 +722,7 @@ def grouped_decode_takes(rows: int, n_heads: int, n_kv: int, head_dim: int, sms:
     if max_pages <= 12 and blocks <= sms or max_pages <= 16 and n_heads > 8 * n_kv and blocks <= 2 * sms:
         return False
     if n_heads != n_kv or head_dim not in (64, 128):
-        return True
+        return n_heads != n_kv or head_dim != 112 or max_pages > 4 or blocks <= 2 * sms
     if max_pages <= 16:
         return head_dim == 128 and not 3 * sms < blocks <= 4 * sms and blocks < 6 * sms
     fills = 32 * sms < 10 * blocks <= 40 * sms
