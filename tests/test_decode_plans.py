@@ -1,4 +1,4 @@
-"""How decode attention is planned (kernels/ops.py): which kernel runs and in how many splits, on the CPU with a library that records."""
+"""How attention is planned (kernels/ops.py): which kernel runs, in how many splits, for how many SMs, on the CPU with a library that records."""
 import pytest
 import torch
 
@@ -55,3 +55,10 @@ def test_many_short_contexts_of_112_dims_go_a_head_a_block(heads, rows, pages, g
     assert ops.grouped_decode_takes(rows, heads, heads, 112, 148, pages) == grouped
     assert ops.grouped_decode_takes(rows, heads, heads, 96, 148, pages)
     assert ops.grouped_decode_takes(rows, heads, heads // 4, 112, 148, pages)
+
+
+def test_32_bit_attention_lays_its_blocks_out_for_the_devices_sms(recorded, monkeypatch):
+    monkeypatch.setattr(ops, "_sm_count", lambda device: 132)
+    q, i32 = torch.zeros(70, 32 * 64), torch.zeros(70, dtype=torch.int32)
+    ops.attention_simt(q, torch.zeros(1, 2, 32, 16, 64), torch.zeros(1, 8, dtype=torch.int32), i32, i32, q.clone(), 32, 0.1)
+    assert recorded.calls[-1][1][-2].value == 132        # before the stream

@@ -621,14 +621,14 @@ int launch_rows(const SimtParams<T>& p, cudaStream_t stream) {
 }
 
 template <typename T, int DIMS, int THREADS>
-int launch_tiles(const SimtParams<T>& p, cudaStream_t stream) {
+int launch_tiles(const SimtParams<T>& p, int sms, cudaStream_t stream) {
     constexpr int KEYS = STAGE_KEYS, PLACES = DIMS == 64 ? 4 : 2;      // blocks an SM
     const int d = p.head_dim, keys_pitch = (d > KEYS ? d : KEYS) + 4;
     const size_t staged = KEYS * keys_pitch + KEYS * d;
     const size_t smem = sizeof(float) * (TILE_ROWS * (d + 4) + staged), others_smem = sizeof(float) * (32 * (d + 4) + staged);
     if (const int rc = allow_smem(attention_simt_tiles_kernel<T, DIMS, THREADS>, smem)) return rc;
     if (const int rc = allow_smem(attention_simt_others_kernel<T, DIMS, THREADS>, others_smem)) return rc;
-    const int tiles = (p.n_tokens + TILE_ROWS - 1) / TILE_ROWS, sms = 148;
+    const int tiles = (p.n_tokens + TILE_ROWS - 1) / TILE_ROWS;
     int others = PLACES * sms / p.n_heads;
     others = others < 1 ? 1 : others > p.n_tokens ? p.n_tokens : others;
     const int round = (sms + p.n_heads - 1) / p.n_heads, first_tiles = round < tiles ? round : tiles;
@@ -640,26 +640,26 @@ int launch_tiles(const SimtParams<T>& p, cudaStream_t stream) {
 // portions: some request may have several rows.  The tiles take them where no mask shifts the 32-key steps of neighbouring
 // rows against one another and the rows are enough to give the SMs tiles.
 template <typename T>
-int launch_all(SimtParams<T> p, int portions, cudaStream_t stream) {
-    const bool staged = p.head_dim % 4 == 0 && p.head_dim <= 128 && (uintptr_t)p.cache % (4 * sizeof(T)) == 0 && p.n_heads <= 65535 && p.n_tokens <= 2000000;
+int launch_all(SimtParams<T> p, int portions, int sms, cudaStream_t stream) {
+    const bool staged = p.head_dim % 4 == 0 && p.head_dim <= 128 && (uintptr_t)p.cache % (4 * sizeof(T)) == 0 && p.n_heads <= 65535;
     if (!staged) return launch_wide<T>(p, stream);
-    if (portions && p.window == 0 && (long long)p.n_tokens * p.n_heads >= 2048)
-        return p.head_dim <= 64 ? launch_tiles<T, 64, 128>(p, stream) : launch_tiles<T, 128, 256>(p, stream);
+    if (portions && p.window == 0 && (long long)p.n_tokens * p.n_heads >= 2048 && p.n_tokens <= 2000000)      // (a grid's second axis)
+        return p.head_dim <= 64 ? launch_tiles<T, 64, 128>(p, sms, stream) : launch_tiles<T, 128, 256>(p, sms, stream);
     return p.head_dim <= 64 ? launch_rows<T, 128>(p, stream) : launch_rows<T, 64>(p, stream);
 }
 }  // namespace
 
-// portions: 0 where every request of the batch has one row (the rows kernel alone), else 1.
+// portions: 0 where every request of the batch has one row (the rows kernel alone), else 1; sms: how many the device has.
 TNX_EXPORT int tnx_attention_simt(const void* q, int q_stride, const void* cache, const int* block_tables,
                                   int bt_stride, const int* token_request, const int* positions, void* out,
                                   int out_stride, int n_tokens, int n_heads, int n_kv_heads, int head_dim,
                                   int page_size, int window, float scale, int keep_first, const float* bias_mul,
-                                  const float* bias_rate, int has_sink, float sink_score, int is_h16, int portions,
+                                  const float* bias_rate, int has_sink, float sink_score, int is_h16, int portions, int sms,
                                   cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (head_dim <= 0 || head_dim > 32 * WIDE_DIMS_PER_LANE || n_kv_heads <= 0 || n_heads % n_kv_heads)
         return TNX_ERR_UNSUPPORTED;
-    if (keep_first < 0 || (bias_mul && !bias_rate)) return TNX_ERR_BAD_ARG;
+    if (keep_first < 0 || (bias_mul && !bias_rate) || sms <= 0) return TNX_ERR_BAD_ARG;
     const DistanceBias bias{bias_mul, bias_rate};
     const SoftmaxSink sink{has_sink, sink_score};
     int page_shift = -1;
@@ -667,7 +667,7 @@ TNX_EXPORT int tnx_attention_simt(const void* q, int q_stride, const void* cache
 #define ASIMT(T)                                                                                                        \
     return launch_all<T>(SimtParams<T>{(const T*)q, q_stride, (const T*)cache, block_tables, bt_stride, token_request,  \
                                        positions, (T*)out, out_stride, n_tokens, n_heads, n_kv_heads, head_dim,         \
-                                       page_size, window, scale, keep_first, bias, sink, page_shift}, portions, stream)
+                                       page_size, window, scale, keep_first, bias, sink, page_shift}, portions, sms, stream)
     if (is_h16) ASIMT(h16);
     ASIMT(float);
 #undef ASIMT

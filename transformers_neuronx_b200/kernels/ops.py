@@ -372,7 +372,7 @@ def attention_simt(q, cache, block_tables, token_request, positions, out, n_head
                                   _p(token_request), _p(positions), _p(out), c_int(out_stride), c_int(N),
                                   c_int(n_heads), c_int(n_kv), c_int(d), c_int(ps), c_int(mask),
                                   c_float(scale), *_score_options(keep_first, bias, sink, n_heads, window),
-                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), _stream()), "attention_simt", 2 if tiled else 1)
+                                  c_int(_is_h16(cache)), c_int(1 if portions else 0), c_int(_sm_count(q.device)), _stream()), "attention_simt", 2 if tiled else 1)
 
 
 def sample(logits, out, temperature=None, top_k=None, top_p=None, seeds=None, counters=None, suppress_id=-1,
@@ -444,13 +444,17 @@ _gemm_plans = {}          # (M, N, K, kind of the result, a bias, SMs) -> (split
 _dev_state = {}          # per device: error word, split-K scratch and counters, SM count
 
 
+def _sm_count(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def _state(device):
     key = device.index if device.index is not None else torch.cuda.current_device()
     st = _dev_state.get(key)
     if st is None:
         st = {"err": torch.zeros(1, dtype=torch.int32, device=device),
               "scratch": None, "counters": torch.zeros(1024, dtype=torch.int32, device=device),
-              "sms": torch.cuda.get_device_properties(device).multi_processor_count}
+              "sms": _sm_count(device)}
         _dev_state[key] = st
     return st
 
