@@ -576,10 +576,8 @@ template <int D, int NT, int WARPS, bool BIAS, bool RING>
 int launch_as(dim3 grid, cudaStream_t stream, const GroupedParams& p) {
     constexpr size_t smem = (size_t)WARPS * warp_bytes<D, NT, BIAS, RING>();
     auto kernel = attention_decode_grouped_kernel<D, NT, WARPS, BIAS, RING>;
-    if (smem > 40 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-    }
+    static TnxSmemLimit limit;
+    if (const int rc = limit.allow(kernel, smem)) return rc;
     if (p.n_splits == 1) return tnx_launch_in_order(kernel, grid, dim3(WARPS * 32), smem, stream, p);
     return tnx_launch_cluster(0, dim3(1, 1, p.n_splits), kernel, grid, dim3(WARPS * 32), smem, stream, p);
 }

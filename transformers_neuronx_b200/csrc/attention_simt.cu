@@ -603,31 +603,23 @@ int launch_wide(const SimtParams<T>& p, cudaStream_t stream) {
 #undef WIDE
 }
 
-// More than 48 KB of shared memory have to be asked for, and a kernel's static arrays count as well (the tiles' and the others' take up
-// to 5.2 KB: heads of 56 and 60 dims stay below with a tile's dynamic part alone).
-template <typename K>
-int allow_smem(K kernel, size_t smem) {
-    if (smem + 6 * 1024 <= 48 * 1024) return 0;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) cudaGetLastError();
-    return (int)e;
-}
-
 template <typename T, int KEYS>
 int launch_rows(const SimtParams<T>& p, cudaStream_t stream) {
-    const size_t smem = sizeof(float) * (KEYS * (2 * p.head_dim + 4) + p.head_dim + KEYS);
-    if (const int rc = allow_smem(attention_simt_rows_kernel<T, KEYS>, smem)) return rc;
+    auto smem_of = [](int d) { return sizeof(float) * (KEYS * (2 * d + 4) + d + KEYS); };
+    static TnxSmemLimit limit;
+    if (const int rc = limit.allow(attention_simt_rows_kernel<T, KEYS>, smem_of(KEYS == 128 ? 64 : 128))) return rc;
+    const size_t smem = smem_of(p.head_dim);
     return tnx_launch_in_order(attention_simt_rows_kernel<T, KEYS>, dim3(p.n_tokens, p.n_heads), dim3(128), smem, stream, p);
 }
 
 template <typename T, int DIMS, int THREADS>
 int launch_tiles(const SimtParams<T>& p, int sms, cudaStream_t stream) {
     constexpr int KEYS = STAGE_KEYS, PLACES = DIMS == 64 ? 4 : 2;      // blocks an SM
-    const int d = p.head_dim, keys_pitch = (d > KEYS ? d : KEYS) + 4;
-    const size_t staged = KEYS * keys_pitch + KEYS * d;
-    const size_t smem = sizeof(float) * (TILE_ROWS * (d + 4) + staged), others_smem = sizeof(float) * (32 * (d + 4) + staged);
-    if (const int rc = allow_smem(attention_simt_tiles_kernel<T, DIMS, THREADS>, smem)) return rc;
-    if (const int rc = allow_smem(attention_simt_others_kernel<T, DIMS, THREADS>, others_smem)) return rc;
+    auto smem_of = [](int rows, int d) { return sizeof(float) * (rows * (d + 4) + KEYS * ((d > KEYS ? d : KEYS) + 4) + KEYS * d); };
+    static TnxSmemLimit limit, others_limit;
+    if (const int rc = limit.allow(attention_simt_tiles_kernel<T, DIMS, THREADS>, smem_of(TILE_ROWS, DIMS))) return rc;
+    if (const int rc = others_limit.allow(attention_simt_others_kernel<T, DIMS, THREADS>, smem_of(32, DIMS))) return rc;
+    const size_t smem = smem_of(TILE_ROWS, p.head_dim), others_smem = smem_of(32, p.head_dim);
     const int tiles = (p.n_tokens + TILE_ROWS - 1) / TILE_ROWS;
     int others = PLACES * sms / p.n_heads;
     others = others < 1 ? 1 : others > p.n_tokens ? p.n_tokens : others;

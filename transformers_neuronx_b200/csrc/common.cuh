@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #define TNX_EXPORT extern "C" __attribute__((visibility("default")))
 
 // Entry points return 0 on success, a CUDA error code (>0) if a launch failed, or a negative
@@ -98,6 +100,21 @@ static inline int tnx_launch_in_order(void (*kernel)(KArgs...), dim3 grid, dim3 
                                  Args... args) {
     return tnx_launch_ex(0, kernel, grid, block, smem, stream, args...);
 }
+
+// Shared memory beyond 48 KB, a kernel's static arrays among it, has to be allowed on every device.  One of these, static, beside the
+// launch of a kernel asks once a device for the most that it may need (0, or an error).
+struct TnxSmemLimit {
+    std::once_flag once[64];
+    cudaError_t result[64];
+    template <typename K> int allow(K kernel, size_t most) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev < 0 || dev >= 64) return TNX_ERR_UNSUPPORTED;
+        std::call_once(once[dev], [&] { result[dev] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most); });
+        if (result[dev] != cudaSuccess) cudaGetLastError();
+        return (int)result[dev];
+    }
+};
 
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(h16 v) { return h16_to_float(v); }

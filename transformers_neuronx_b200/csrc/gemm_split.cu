@@ -485,15 +485,8 @@ split_terms_kernel(const float* __restrict__ A, h16* __restrict__ planes, float*
 template <int BN, int NT>
 int launch_product(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int sms, cudaStream_t stream) {
     using S = Shape<BN, NT>;
-    static std::once_flag once[64];
-    static cudaError_t set[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return TNX_ERR_UNSUPPORTED;
-    std::call_once(once[dev], [&] {
-        set[dev] = cudaFuncSetAttribute(gemm_split_kernel<BN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
-    });
-    if (set[dev] != cudaSuccess) return (int)set[dev];
+    static TnxSmemLimit limit;
+    if (const int rc = limit.allow(gemm_split_kernel<BN, NT>, S::SMEM)) return rc;
     const int grid = p.items < sms ? p.items : sms;
     return tnx_launch_ex(1, gemm_split_kernel<BN, NT>, dim3(grid), dim3(S::THREADS), S::SMEM, stream, mw, mx, p);
 }
