@@ -18,9 +18,9 @@
 //   tiles   for portions of prompts without a mask: a block takes 64 neighbouring rows and one head, 64 staged keys and
 //           values serve all of them; what a tile holds beside its largest portion goes to a kernel that runs beside it (others)
 // Measured, 32 heads of 64, 32-bit: a portion of 499 tokens behind 256 beside three single rows of 500 to 700 keys, 2,417 us
-// with `wide` for all rows, 1,200 with `rows`, 160 with `tiles` (in tiles of 32 rows with the single rows in a kernel
+// with `wide` for all rows, 1,200 with `rows`, 147 with `tiles` (in tiles of 32 rows with the single rows in a kernel
 // after them 279); four single rows of 100 to 900 keys 382 us with `wide`, 53 with `rows`; 64 of 100 to 1,360 keys 1,106 and 434;
-// a portion of 2,048 tokens, 16 heads of 128, 0.60 ms (tiles of 32 rows 1.66).
+// a portion of 2,048 tokens, 16 heads of 128, 0.58 ms (tiles of 32 rows 1.66).
 #include "common.cuh"
 
 namespace {
@@ -130,16 +130,20 @@ __device__ __forceinline__ float4 load4(const h16* p) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// One row and one head by THREADS threads (no fewer than KEYS and the head's dims): a block, or part `part` of one.
-template <typename T, int KEYS, int THREADS>
-__device__ __forceinline__ void attend_row(const SimtParams<T>& p, float* sm, int n, int h, int part) {
-    auto meet = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + part), "n"(THREADS) : "memory"); };
+// One row and one head by THREADS threads (no fewer than KEYS and the head's dims): a block (part < 0), or part 0 or 1 of one.  (A named
+// barrier where the block's own would do cost the rows kernel 4 %.)
+template <typename T, int KEYS, int THREADS, bool WHOLE = true>
+__device__ __forceinline__ void attend_row(const SimtParams<T>& p, float* sm, int n, int h, int part = -1) {
+    auto meet = [&] {
+        if (WHOLE) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + part), "n"(THREADS) : "memory");
+    };
     const int d = p.head_dim, d4 = d / 4;
     float* ks = sm;                                 // [KEYS][d + 4]: a warp's 16-byte reads down the rows meet all banks evenly
     float* vs = ks + KEYS * (d + 4);                // [KEYS][d]
     float* qs = vs + KEYS * d;                      // [d]
     float* ss = qs + d;                             // [KEYS] the staged keys' scores
-    const int tid = threadIdx.x % THREADS, lane = tid & 31;
+    const int tid = WHOLE ? threadIdx.x : threadIdx.x % THREADS, lane = tid & 31;
     const int kvh = h / (p.n_heads / p.n_kv_heads);
     const size_t head_block = (size_t)p.page_size * d;
     const float mul = p.bias.mul ? p.bias.mul[h] : 0.f, rate = p.bias.mul ? p.bias.rate[h] : 0.f;
@@ -215,7 +219,7 @@ attention_simt_rows_kernel(const SimtParams<T> p) {
     extern __shared__ __align__(16) float sm[];
     pdl_launch_dependents();
     pdl_wait();
-    attend_row<T, KEYS, 128>(p, sm, blockIdx.x, blockIdx.y, 0);
+    attend_row<T, KEYS, 128>(p, sm, blockIdx.x, blockIdx.y);
 }
 
 // A tile's portions: in 64 neighbouring rows, a request's rows.
@@ -578,9 +582,9 @@ attention_simt_others_kernel(const SimtParams<T> p) {
         auto row = [&](int i) { return base + mine[AT_ONCE * TILE_ROWS - 1 - i]; };
         if (pairs) {                                 // two rows at a time (100 dims 0.89 of the time of one; 128 dims 1.2)
             const int part = tid / 128;
-            for (int i = part; i < n_rows; i += 2) attend_row<T, 32, 128>(p, sm + part * (32 * (2 * p.head_dim + 4) + p.head_dim + 32), row(i), h, part);
+            for (int i = part; i < n_rows; i += 2) attend_row<T, 32, 128, false>(p, sm + part * (32 * (2 * p.head_dim + 4) + p.head_dim + 32), row(i), h, part);
         } else {
-            for (int i = 0; i < n_rows; ++i) attend_row<T, 64, THREADS>(p, sm, row(i), h, 0);
+            for (int i = 0; i < n_rows; ++i) attend_row<T, 64, THREADS>(p, sm, row(i), h);
         }
         __syncthreads();
     }

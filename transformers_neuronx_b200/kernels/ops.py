@@ -444,8 +444,14 @@ _gemm_plans = {}          # (M, N, K, kind of the result, a bias, SMs) -> (split
 _dev_state = {}          # per device: error word, split-K scratch and counters, SM count
 
 
+_sm_counts = {}          # per device: asking torch takes 3 us
+
+
 def _sm_count(device) -> int:
-    return torch.cuda.get_device_properties(device).multi_processor_count
+    n = _sm_counts.get(device)
+    if n is None:
+        n = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return n
 
 
 def _state(device):
